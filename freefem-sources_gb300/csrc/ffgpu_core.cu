@@ -2,7 +2,7 @@
 #include <stdarg.h>
 #include <string.h>
 
-#include "ffgpu_internal.cuh"
+#include "ffgpu_gridsync.cuh"
 
 namespace ffgpu {
 
@@ -280,12 +280,17 @@ int ffgpu_ctx_create(int device, ffgpu_ctx **out) {
         cudaMalloc((void **)&c->d_part, sizeof(double) * 8192) != cudaSuccess ||
         cudaMalloc((void **)&c->d_status, sizeof(int) * 4) != cudaSuccess ||
         cudaMalloc((void **)&c->d_ticket, sizeof(unsigned int) * 16) != cudaSuccess ||
-        cudaMalloc((void **)&c->d_iscratch, sizeof(int) * 16) != cudaSuccess) {
+        cudaMalloc((void **)&c->d_iscratch, sizeof(int) * 16) != cudaSuccess ||
+        cudaMalloc(&c->d_sync, kGsBytes) != cudaSuccess) {
         set_error("ffgpu_ctx_create: CUDA setup failed: %s", cudaGetErrorString(cudaGetLastError()));
         if (c->pool) cudaMemPoolDestroy(c->pool);
         delete c;
         return FFGPU_ECUDA;
     }
+    int coop = 0, sms = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    c->coop = coop && sms >= kNumSM;
     cudaMemset(c->d_status, 0, sizeof(int) * 4);
     cudaMemset(c->d_ticket, 0, sizeof(unsigned int) * 16);
     cudaDeviceSynchronize();
@@ -300,6 +305,7 @@ int ffgpu_ctx_destroy(ffgpu_ctx *c) {
     cudaFree(c->d_status);
     cudaFree(c->d_ticket);
     cudaFree(c->d_iscratch);
+    cudaFree(c->d_sync);
     cudaStreamDestroy(c->stream);
     // blocks of objects still alive are released when those objects free them
     cudaMemPoolDestroy(c->pool);

@@ -82,6 +82,8 @@ struct ffgpu_ctx {
     int *d_status;              // DevStatus word
     unsigned int *d_ticket;     // last-block counters
     int *d_iscratch;            // small integer scratch (max reductions)
+    void *d_sync;               // slots of the in-kernel exchanges (ffgpu_gridsync.cuh)
+    int coop;                   // the device runs cooperative launches of one block on each of kNumSM SMs
     // SpMV layout chosen by timing, per matrix shape (nb, nnzb, bs) and mode, kept for the
     // context's lifetime: every later matrix of a shape gets the same layout, however many
     // shapes the context has seen
@@ -161,6 +163,9 @@ struct ffgpu_matrix {
     // per-grid partitions of the chunks over warps, balanced by slot count (nw+1 starts)
     int spart_nw[4];
     int32_t *spart[4];
+    // in-kernel CG loop (ffgpu_persist.cu): widest column range and most row-group slots of a
+    // block (0: not measured yet, -1: could not be)
+    int band_range, band_slots;
     int sell32_kind;      // chunk assignment of the FP32 SELL SpMV (tuned): 64 ranges, 65 rotated
 };
 
@@ -322,6 +327,11 @@ int spmv(ffgpu_matrix *A, const double *x, double *y, int trans, cudaStream_t s)
 // whether it takes the matrix (a rule on sizes and the device, never on timings), and the run
 // from the state cg_init leaves (x, g, h, Krylov scalars; x receives the solution).
 bool cluster_cg_fits(ffgpu_matrix *A, int trans);
+// the CG loop of a scalar system with a narrow column range in one cooperative kernel
+// (ffgpu_persist.cu), under the same contract
+constexpr int kLoopRefused = 1;      // the launch was refused, nothing ran
+bool band_cg_fits(ffgpu_matrix *A);
+int band_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, double *h2, double *cg, cudaStream_t s);
 constexpr int kClusterRefused = 1;   // cluster_cg_run: the launch was refused, nothing ran
 int cluster_cg_run(ffgpu_matrix *A, int trans, double *x, const double *g, const double *h, cudaStream_t s);
 // the direct solver's factorisation: stale after a numeric change (the ordering and the

@@ -1,0 +1,282 @@
+// ffgpu_persist.cu -- the CG loop of ffgpu_solve_cg inside one cooperative kernel.
+//
+// FreeFEM's ConjugueGradient (src/femlib/CG.cpp:196-265) as ffgpu_solve.cu describes it, for
+// scalar systems whose block rows touch a narrow range of columns (2D meshes, small 3D ones).
+// One block per SM owns consecutive rows for the whole solve:
+//   * its rows of the matrix in shared memory (values FP64, columns as 16-bit numbers relative
+//     to the first column the block touches), x, g and 1/A_ii in registers;
+//   * per iteration it forms the direction h' = gamma h - C g once for every column it touches
+//     (its own rows and the halo), from the h and C g the owners left in L2, multiplies from
+//     shared memory, and takes part in two exchanges (ffgpu_gridsync.cuh): (g,h'), (h',A h')
+//     and (g, C g).
+// So nothing of the matrix moves after the start, and an iteration is two trips through L2.
+// The launches of the two-kernel loop spend an iteration on kernel boundaries, a chain of
+// dependent L2 reads and FP64 reductions over many more warps than the sums need.
+#include <stdlib.h>
+#include <string.h>
+
+#include <algorithm>
+
+#include "ffgpu_gridsync.cuh"
+
+namespace ffgpu {
+
+struct BandArgs {
+    int n, rows;                 // rows per block
+    const int32_t *rp, *col;
+    const double *val, *dinv;
+    double *x, *g, *h0, *h1, *cg;
+    KrylovScalars *ks;
+    GridSync gs;
+    int range_cap;               // doubles of the staged direction
+};
+
+// What a block needs: the column range of its rows and the slots of its row groups (32 rows
+// padded to the longest).  need[0]: widest range, need[1]: most slots (both over the blocks).
+__global__ void __launch_bounds__(128) band_need_kernel(int n, int rows, const int32_t *__restrict__ rp,
+                                                        const int32_t *__restrict__ col, int *need) {
+    __shared__ int lo, hi, slots;
+    if (threadIdx.x == 0) { lo = 0x7fffffff; hi = -1; slots = 0; }
+    __syncthreads();
+    const int r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
+    for (int base = r0; base < r1; base += blockDim.x) {
+        const int r = base + threadIdx.x;
+        int L = 0;
+        if (r < r1) {
+            const int b = rp[r], e = rp[r + 1];
+            L = e - b;
+            int cl = r, ch = r;   // the row itself is staged too
+            for (int k = b; k < e; ++k) { cl = min(cl, col[k]); ch = max(ch, col[k]); }
+            atomicMin(&lo, cl);
+            atomicMax(&hi, ch);
+        }
+        L = __reduce_max_sync(0xffffffffu, L);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&slots, L);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicMax(need, hi - lo + 1);
+        atomicMax(need + 1, slots);
+    }
+}
+
+// RPT rows per thread, NT threads.  Row r0 + u * NT + t belongs to thread t.
+// FP64 instructions set the floor (one per 64 cycles and sub-partition): about 16 per group of
+// 32 rows and iteration on a 2D P1 mesh.
+template <int NT, int RPT>
+__global__ void __launch_bounds__(NT, 1) cg_band(BandArgs A) {
+    constexpr int NW = NT / 32;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ double red[kGsRed<NW>];
+    __shared__ int s_lo, s_hi, s_base[RPT * NW + 1];
+    if (A.ks->done) return;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int r0 = blockIdx.x * A.rows, r1 = min(A.n, r0 + A.rows);
+    double *hs = reinterpret_cast<double *>(smraw);
+    if (t == 0) { s_lo = 0x7fffffff; s_hi = -1; }
+    __syncthreads();
+    double x[RPT], g[RPT], z[RPT], d[RPT];
+    int len[RPT];
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+        const int r = r0 + u * NT + t;
+        const bool own = r < r1;
+        int L = 0;
+        x[u] = g[u] = z[u] = d[u] = 0.0;
+        if (own) {
+            const int b = A.rp[r], e = A.rp[r + 1];
+            L = e - b;
+            int cl = r, ch = r;
+            for (int k = b; k < e; ++k) { cl = min(cl, A.col[k]); ch = max(ch, A.col[k]); }
+            atomicMin(&s_lo, cl);
+            atomicMax(&s_hi, ch);
+            x[u] = A.x[r]; g[u] = A.g[r]; d[u] = A.dinv[r];
+        }
+        len[u] = __reduce_max_sync(0xffffffffu, L);
+        if (lane == 0) s_base[u * NW + w] = len[u];
+    }
+    __syncthreads();
+    if (t == 0) {
+        int s = 0;
+        for (int i = 0; i < RPT * NW; ++i) { const int L = s_base[i]; s_base[i] = s; s += L; }
+        s_base[RPT * NW] = s;
+    }
+    __syncthreads();
+    const int lo = s_lo, nc = s_hi - lo + 1;
+    double *mv = hs + A.range_cap;
+    uint16_t *mc = reinterpret_cast<uint16_t *>(mv + (size_t)s_base[RPT * NW] * 32);
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+        const int r = r0 + u * NT + t;
+        const int b = r < r1 ? A.rp[r] : 0, L = r < r1 ? A.rp[r + 1] - b : 0;
+        const int base = s_base[u * NW + w] * 32 + lane;
+        for (int j = 0; j < len[u]; ++j) {
+            mv[base + 32 * j] = j < L ? A.val[b + j] : 0.0;
+            mc[base + 32 * j] = (uint16_t)(j < L ? A.col[b + j] - lo : 0);
+        }
+    }
+    const double eps2 = A.ks->eps2;
+    const int itmax = A.ks->itmax;
+    double gcg = A.ks->gcg, gcgp = gcg, gamma = 1.0, rho = 0.0, sgh = 0.0, shq = 0.0;
+    int iter = 0, conv = 0, k = 0;
+    bool good = true;
+    const double *hold = A.h0;
+    double *hnew = A.h1;
+    for (;;) {
+        // ---- the direction on every column the block touches (the loads of four in flight)
+        for (int c0 = t; c0 < nc; c0 += 4 * NT) {
+            double hv[4], cv[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int c = c0 + q * NT;
+                hv[q] = c < nc ? __ldcg(hold + lo + c) : 0.0;
+                cv[q] = c < nc && iter ? __ldcg(A.cg + lo + c) : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int c = c0 + q * NT;
+                if (c < nc) hs[c] = fma(gamma, hv[q], -cv[q]);
+            }
+        }
+        __syncthreads();
+        // ---- q = A h' from shared memory, the rows' products side by side
+        double y[RPT], ho[RPT];
+        double pa = 0.0, pb = 0.0;
+#pragma unroll
+        for (int u = 0; u < RPT; ++u) {
+            const int r = r0 + u * NT + t;
+            const int base = s_base[u * NW + w] * 32 + lane;
+            double s = 0.0;
+#pragma unroll 4
+            for (int j = 0; j < len[u]; ++j) s = fma(mv[base + 32 * j], hs[mc[base + 32 * j]], s);
+            y[u] = s;
+            ho[u] = 0.0;
+            if (u * NT < A.rows) {               // uniform: groups past the rows do no FP64 work
+                ho[u] = r < r1 ? hs[r - lo] : 0.0;
+                if (r < r1) __stcg(hnew + r, ho[u]);
+                pa = fma(g[u], ho[u], pa);
+                pb = fma(ho[u], y[u], pb);
+            }
+        }
+        if (!gs_sum2<NW, false>(A.gs, k++, pa, pb, red)) { good = false; break; }
+        sgh = pa;
+        shq = pb;
+        rho = -pa / pb;
+        // ---- x += rho h', g += rho q, C g
+        double pc = 0.0, none = 0.0;
+#pragma unroll
+        for (int u = 0; u < RPT; ++u) {
+            if (u * NT < A.rows) {
+                const int r = r0 + u * NT + t;
+                x[u] = fma(rho, ho[u], x[u]);
+                g[u] = fma(rho, y[u], g[u]);
+                z[u] = __dmul_rn(d[u], g[u]);
+                if (r < r1) __stcg(A.cg + r, z[u]);
+                pc = fma(g[u], z[u], pc);
+            }
+        }
+        if (!gs_sum2<NW, true>(A.gs, k++, pc, none, red)) { good = false; break; }
+        gcgp = gcg;
+        gcg = pc;
+        gamma = gcg / gcgp;
+        ++iter;
+        conv = gcg < eps2;
+        if (conv || iter >= itmax) break;
+        double *const swap = const_cast<double *>(hold);
+        hold = hnew;
+        hnew = swap;
+    }
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+        const int r = r0 + u * NT + t;
+        if (r < r1) A.x[r] = x[u];
+    }
+    if (blockIdx.x == 0 && t == 0) {
+        KrylovScalars *ks = A.ks;
+        ks->gcg = gcg; ks->gcgp = gcgp; ks->gamma = gamma; ks->rho = rho; ks->s_gh = sgh; ks->s_hq = shq;
+        ks->iter = iter;
+        ks->converged = conv;
+        ks->done = good ? 1 : 2;
+    }
+}
+
+// ------------------------------------------------------------------ host side
+// Rows per block: a multiple of 32, all SMs, at least 64 (a shorter block costs more exchange than
+// it saves FP64 time).
+static int band_rows(int n) {
+    const int per = (n + kNumSM - 1) / kNumSM;
+    return std::max(64, (per + 31) / 32 * 32);
+}
+// threads and rows per thread by the rows of a block: 128 threads (one warp per sub-partition)
+// keep the block sums short; 256 from 512 rows on, where registers run out
+static void *band_fn(int rows, int *nt) {
+    *nt = rows <= 512 ? 128 : 256;
+    if (rows <= 128) return (void *)cg_band<128, 1>;
+    if (rows <= 256) return (void *)cg_band<128, 2>;
+    if (rows <= 512) return (void *)cg_band<128, 4>;
+    if (rows <= 1024) return (void *)cg_band<256, 4>;
+    return (void *)cg_band<256, 8>;
+}
+constexpr int kBandMaxRows = 2048;
+constexpr size_t kBandSmem = 224 * 1024;   // of the 227 KB a block may have: the static arrays too
+
+static size_t band_smem(const ffgpu_matrix *A) {
+    return sizeof(double) * (((size_t)A->band_range + 1) & ~(size_t)1) + (size_t)A->band_slots * 32 * (sizeof(double) + sizeof(uint16_t));
+}
+
+// Whether the in-kernel loop takes this matrix: a rule on the pattern and the device, never on
+// timings.  The pattern's needs are measured once (band_need_kernel).
+bool band_cg_fits(ffgpu_matrix *A) {
+    ffgpu_ctx *ctx = A->ctx;
+    if (!ctx->coop || !ctx->d_sync || A->bs != 1) return false;
+    const int rows = band_rows(A->n);
+    if (rows > kBandMaxRows) return false;
+    if (A->band_range == 0) {
+        cudaStream_t s = ctx->stream;
+        int need[2] = {0, 0};
+        A->band_range = -1;
+        if (cudaMemsetAsync(ctx->d_iscratch, 0, sizeof(need), s) != cudaSuccess) return false;
+        band_need_kernel<<<(A->n + rows - 1) / rows, 128, 0, s>>>(A->n, rows, A->browptr, A->bcol, ctx->d_iscratch);
+        if (launch_check(ctx, "band_need") != FFGPU_OK) return false;
+        if (cudaMemcpyAsync(need, ctx->d_iscratch, sizeof(need), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess)
+            return false;
+        A->band_range = need[0];
+        A->band_slots = need[1];
+    }
+    return A->band_range > 0 && A->band_range < 65536 && band_smem(A) <= kBandSmem;
+}
+
+// The loop from the state cg_init leaves (x, g, h, Krylov scalars); h2, cg: two more work
+// vectors.  x receives the solution.
+int band_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, double *h2, double *cg, cudaStream_t s) {
+    ffgpu_ctx *ctx = A->ctx;
+    const int rows = band_rows(A->n);
+    int nt = 0;
+    void *fn = band_fn(rows, &nt);
+    const size_t smem = band_smem(A);
+    BandArgs a;
+    memset(&a, 0, sizeof(a));
+    a.n = A->n; a.rows = rows;
+    a.rp = A->browptr; a.col = A->bcol;
+    a.val = trans ? A->val_t : A->val;
+    a.dinv = A->diag_inv;
+    a.x = x; a.g = g; a.h0 = h; a.h1 = h2; a.cg = cg;
+    a.ks = A->ks;
+    a.gs.slots = (ulonglong2 *)ctx->d_sync;
+    a.range_cap = (A->band_range + 1) & ~1;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        cudaGetLastError();
+        return kLoopRefused;
+    }
+    FFGPU_CUDA(cudaMemsetAsync(ctx->d_sync, 0xff, kGsBytes, s));
+    void *args[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3((A->n + rows - 1) / rows), dim3(nt), args, smem, s);
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // nothing ran: the caller takes the launches per iteration
+        return kLoopRefused;
+    }
+    return launch_check(ctx, "cg_band");
+}
+
+}  // namespace ffgpu

@@ -1185,6 +1185,13 @@ struct KcaCall {
     }
 };
 
+// The loops that stay inside one kernel (ffgpu_persist.cu) are the default; FFGPU_CG_FUSE=0 or
+// FFGPU_CLUSTER_CG=0 selects launches per iteration.
+static bool in_kernel_loops() {
+    const char *f = getenv("FFGPU_CG_FUSE"), *c = getenv("FFGPU_CLUSTER_CG");
+    return !(f && f[0] == '0') && !(c && c[0] == '0');
+}
+
 static bool cg_fused_fits(const ffgpu_matrix *A, int mode) {
     const char *e = getenv("FFGPU_CG_FUSE");
     if (e && e[0] == '0') return false;
@@ -1338,9 +1345,11 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     // (ffgpu_cluster.cu), unless a layout is fixed by the caller
     const bool cluster = mode == 0 && !A->layout_pinned && cluster_cg_fits(A, trans);
     A->last_cluster = cluster;
-    const bool fused = !cluster && cg_fused_fits(A, mode);
+    bool fused = !cluster && cg_fused_fits(A, mode);
     if (fused) unroll += unroll & 1;   // the H buffers alternate: an even number of iterations per body
-    if (!cluster) FFGPU_TRY(cg_graph(A, trans, unroll, mode, x, g, h, q, fused, h2, cgv));
+    // the whole loop in one cooperative kernel where a block's rows and columns fit its SM
+    bool loop = mode == 0 && !cluster && !A->layout_pinned && in_kernel_loops() && band_cg_fits(A);
+    if (!cluster && !loop) FFGPU_TRY(cg_graph(A, trans, unroll, mode, x, g, h, q, fused, h2, cgv));
     FFGPU_CUDA(cudaMemcpyAsync(x, xu, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -1357,14 +1366,26 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
         split_vec_kernel<<<kVecBlocks, kVecThreads, 0, s>>>(n, h, A->hx);
         FFGPU_TRY(launch_check(ctx, "split_vec"));
     }
-    if (fused) {
+    if (fused && !loop) {
         FFGPU_CUDA(cudaMemsetAsync(cgv, 0, sizeof(double) * n, s));
         cg_fuse_start<<<1, 32, 0, s>>>(A->ks);
         FFGPU_TRY(launch_check(ctx, "cg_fuse_start"));
     }
     const char *ge = getenv("FFGPU_CG_GRAPH");
     int bodies_host = -1;
-    bool use_graph = !cluster;
+    bool use_graph = !cluster && !loop;
+    if (loop) {
+        const int rc = band_cg_run(A, trans, x, g, h, h2, cgv, s);
+        if (rc == kLoopRefused) {
+            // the launches per iteration from the same state
+            FFGPU_TRY(cg_graph(A, trans, unroll, mode, x, g, h, q, false, h2, cgv));
+            loop = fused = false;
+            use_graph = true;
+        } else {
+            FFGPU_TRY(rc);
+            bodies_host = 0;
+        }
+    }
     if (cluster) {
         const int rc = cluster_cg_run(A, trans, x, g, h, s);
         if (rc == kClusterRefused) {
@@ -1420,6 +1441,7 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     int bodies = bodies_host >= 0 ? bodies_host
                                   : (fused ? hk.iter / unroll + 1 : (hk.iter == 0 ? 1 : (hk.iter + unroll - 1) / unroll));
     if (use_graph) ctx->launches += (int64_t)bodies * A->cg_kernels_body;
+    FFGPU_CHECK(!loop || hk.done != 2, FFGPU_ECUDA, "CG loop: a wait between blocks ran out after %d iterations", hk.iter);
     if (st) {
         st->iterations = hk.iter;
         st->converged = hk.converged != 0;
