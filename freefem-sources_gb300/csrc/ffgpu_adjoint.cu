@@ -78,6 +78,9 @@ int ffgpu_diffusion_sensitivity(ffgpu_matrix *A, const double *u, const double *
     DevOut<double> gk(grad_kappa, grad_kappa ? S->nt : 0, ctx, false), gf(grad_f, grad_f ? S->nt : 0, ctx, false);
     FFGPU_TRY(ud.err); FFGPU_TRY(ld.err); FFGPU_TRY(gk.err); FFGPU_TRY(gf.err);
     const uint8_t *wcl = A->ntgv > 0 ? A->wcl : nullptr;
+    ffgpu_varf any;   // only the measures and gradients are read
+    memset(&any, 0, sizeof(any));
+    FFGPU_TRY(matrix_geometry(A, &any));
     int grid = (S->nt + 255) / 256;
     if (S->dim == 2)
         sensitivity_kernel<2><<<grid, 256, 0, s>>>(S->nt, S->nodes, A->geo, c_stiff, ud.d, ld.d, wcl, gk.d, gf.d);

@@ -1,19 +1,26 @@
 // ffgpu_assembly.cu -- mesh/FE-space upload, symbolic pattern and numeric assembly.
 //
 // Design (GB300): FreeFEM walks elements and scatters each element matrix into a hash
-// matrix (problem.cpp:1096-1103, HashMatrix.cpp:1295-1332).  Here every matrix row is
-// owned by one warp, which gathers the contributions of the elements incident to its node:
-//   pass 1 (count):  gather the nodes of the incident elements, sort, unique -> row degree;
+// matrix (problem.cpp:1096-1103, HashMatrix.cpp:1295-1332).  Here every matrix row gathers the
+// contributions of the elements incident to its node:
+//   pattern (once per matrix): a warp per row collects the nodes of the incident elements in a
+//                    small hash table, ranks the distinct ones, and notes for every incidence
+//                    the rank of each of the element's nodes in the row (pattern_kernel);
 //   scan:            row pointer;
-//   pass 2 (fill):   same gather -> sorted column list, then add the element-matrix rows of
-//                    the incident elements in ascending element order (the reference's
-//                    summation order), apply tgv, write the row once, coalesced.
+//   element pass:    the element matrices -- P1 in closed form (p1_elem_kernel), P2 from the
+//                    tensor cores (ffgpu_elemtc.cu), coefficients at quadrature points from
+//                    their own kernels;
+//   fill:            a group of lanes per row adds the rows of the element matrices in ascending
+//                    element order (the reference's summation order) into shared memory at the
+//                    noted ranks, applies tgv, and writes the row once, coalesced.
 // No atomics and no colouring are needed on the value path: each value is written once and
-// no read-modify-write of the matrix happens.  The element geometry (barycentric gradients
-// and measure) is computed once per element and cached (16 doubles per element).
+// no read-modify-write of the matrix happens.  A numeric reassembly repeats the last two only.
 // For [P2]^3 the pattern is stored as 3x3 blocks (DOF = 3*node + c, FESpacen.hpp:582),
 // which is the same (i,j) set as FreeFEM's MatriceMorse and 2/3 of the index traffic.
+#include <math.h>
 #include <string.h>
+
+#include <algorithm>
 
 #include "ffgpu_internal.cuh"
 
@@ -82,33 +89,25 @@ __global__ void inc_count_kernel(const int32_t *nodes, int64_t m, int32_t *cnt) 
     if (t < m) atomicAdd(&cnt[nodes[t]], 1);
 }
 
-__global__ void inc_fill_kernel(const int32_t *nodes, int64_t m, int nn, const int32_t *ptr,
-                                int32_t *cursor, int32_t *inc_elem, uint8_t *inc_loc) {
+__global__ void inc_fill_kernel(const int32_t *nodes, int64_t m, const int32_t *ptr, int32_t *cursor, int32_t *inc) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= m) return;
     int a = nodes[t];
-    int pos = ptr[a] + atomicAdd(&cursor[a], 1);
-    inc_elem[pos] = (int32_t)(t / nn);
-    inc_loc[pos] = (uint8_t)(t % nn);
+    inc[ptr[a] + atomicAdd(&cursor[a], 1)] = (int32_t)t;
 }
 
-// sort each node's incidence list by element number (the reference's element order)
-__global__ void inc_sort_kernel(const int32_t *ptr, int nnodes, int max_inc, int32_t *inc_elem,
-                                uint8_t *inc_loc) {
-    extern __shared__ long long sh_inc[];
+// sort each node's incidence list by slot, i.e. by element number (the reference's element order)
+__global__ void inc_sort_kernel(const int32_t *ptr, int nnodes, int max_inc, int32_t *inc) {
+    extern __shared__ int sh_inc[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int P = pow2_ceil(max_inc);
-    long long *s = sh_inc + (int64_t)w * P;
+    int *s = sh_inc + (int64_t)w * P;
     for (int a = blockIdx.x * (blockDim.x >> 5) + w; a < nnodes; a += gridDim.x * (blockDim.x >> 5)) {
         int b = ptr[a], e = ptr[a + 1], n = e - b;
-        for (int i = lane; i < P; i += 32)
-            s[i] = i < n ? (((long long)inc_elem[b + i]) << 8) | inc_loc[b + i] : 0x7fffffffffffffffLL;
+        for (int i = lane; i < P; i += 32) s[i] = i < n ? inc[b + i] : 0x7fffffff;
         __syncwarp();
         warp_bitonic_sort(s, P);
-        for (int i = lane; i < n; i += 32) {
-            inc_elem[b + i] = (int32_t)(s[i] >> 8);
-            inc_loc[b + i] = (uint8_t)(s[i] & 0xff);
-        }
+        for (int i = lane; i < n; i += 32) inc[b + i] = s[i];
         __syncwarp();
     }
 }
@@ -285,336 +284,369 @@ __device__ __forceinline__ double basis_integral(double meas, int i) {
     return i < 3 ? 0.0 : meas / 3.0;
 }
 
-// ------------------------------------------------------------------ row gather (both passes)
-// Register path for rows with at most 32 distinct neighbours: the candidates are read 32 at
-// a time, duplicates inside a batch are merged with __match_any_sync, the new ones are
-// appended to a list held one entry per lane, and the list is sorted by a 32-lane bitonic
-// network on shuffles.  Returns the degree, or -1 when the row has more than 32 neighbours.
-__device__ int gather_row_small(int b, int m, const int32_t *inc_elem, const int32_t *nodes, int nn, int *s) {
-    const int lane = threadIdx.x & 31;
-    const unsigned full = 0xffffffffu;
-    int u = 0, mine = 0x7fffffff;
-    for (int p0 = 0; p0 < m; p0 += 32) {
-        const int p = p0 + lane;
-        int v = 0x7fffffff;
-        if (p < m) {
-            const int t = p / nn, i = p - t * nn;
-            v = nodes[(int64_t)inc_elem[b + t] * nn + i];
-        }
-        const unsigned grp = __match_any_sync(full, v);
-        bool fresh = v != 0x7fffffff && lane == __ffs(grp) - 1;
-        for (int L = 0; L < u; ++L) fresh &= __shfl_sync(full, mine, L) != v;
-        const unsigned bal = __ballot_sync(full, fresh);
-        const int cnt = __popc(bal);
-        if (u + cnt > 32) return -1;
-        if (fresh) s[u + __popc(bal & ((1u << lane) - 1u))] = v;
-        __syncwarp();
-        if (lane >= u && lane < u + cnt) mine = s[lane];
-        __syncwarp();
-        u += cnt;
-    }
-    // ascending bitonic sort of one value per lane (unused lanes hold INT_MAX)
+// ------------------------------------------------------------------ P1 element matrices
+// Products and sums with their roundings spelled out where two kernels have to form the same
+// bits (the measure enters the matrix kernel and the linear form).
+__device__ __forceinline__ double det2(double a, double b, double c, double d) { return fma(a, d, -__dmul_rn(b, c)); }
+
+// Vertex coordinates of an element relative to its first vertex: V[i] = P[i+1] - P[0]
+template <int DIM>
+__device__ __forceinline__ void edge_vectors(const double *__restrict__ X, const int32_t *__restrict__ v, double V[DIM][DIM]) {
+    double A[DIM];
 #pragma unroll
-    for (int k = 2; k <= 32; k <<= 1)
+    for (int d = 0; d < DIM; ++d) A[d] = __ldg(X + (int64_t)DIM * v[0] + d);
 #pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            const int o = __shfl_xor_sync(full, mine, j);
-            const bool lower = (lane & j) == 0, up = (lane & k) == 0;
-            mine = (lower == up) ? min(mine, o) : max(mine, o);
-        }
-    if (lane < u) s[lane] = mine;
-    __syncwarp();
-    return u;
+    for (int i = 0; i < DIM; ++i)
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) V[i][d] = __dsub_rn(__ldg(X + (int64_t)DIM * v[i + 1] + d), A[d]);
+}
+// det of the edge vectors (DIM! times the measure) and, in 3D, the cross product V1 x V2
+__device__ __forceinline__ double edge_det(const double V[2][2], double *) { return det2(V[0][0], V[0][1], V[1][0], V[1][1]); }
+__device__ __forceinline__ double edge_det(const double V[3][3], double *c) {
+    c[0] = det2(V[1][1], V[1][2], V[2][1], V[2][2]);
+    c[1] = det2(V[1][2], V[1][0], V[2][2], V[2][0]);
+    c[2] = det2(V[1][0], V[1][1], V[2][0], V[2][1]);
+    return fma(V[0][2], c[2], fma(V[0][1], c[1], __dmul_rn(V[0][0], c[0])));
+}
+template <int DIM>
+__device__ __forceinline__ double measure_of(double det) { return __dmul_rn(det, DIM == 2 ? 0.5 : 1.0 / 6.0); }
+
+__device__ __forceinline__ void store4(double *p, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
 }
 
-// Gathers the candidate neighbour nodes of node a into s, sorts and compacts them in
-// place; returns the row degree (or -1 on overflow).
-__device__ int gather_row(int a, const int32_t *inc_ptr, const int32_t *inc_elem,
-                          const int32_t *nodes, int nn, int *s, int *status) {
-    const int lane = threadIdx.x & 31;
-    int b = inc_ptr[a], e = inc_ptr[a + 1];
-    int m = (e - b) * nn;
-    if (m > kCandMax) { if (lane == 0) dev_fail(status, kDevCandOverflow); return -1; }
-    if (nn <= 4) {
-        const int u = gather_row_small(b, m, inc_elem, nodes, nn, s);
-        if (u >= 0) return u;
+// Element matrices of int(c_stiff kappa grad u.grad v + c_mass u v) on P1, one thread each:
+//   grad phi_i = N_i / det with N_i the inward normals (cross products of edges), so
+//   K_ij = (kappa c_stiff / (DIM! det)) N_i.N_j, the pairs among the vertices 1..DIM as dot products
+//   and the others from the zero row sums (sum_i grad phi_i = 0).
+// Row la of element e at out[(e * (DIM + 1) + la) * 4], four doubles wide (32-byte stores; the
+// row fill reads one sector).  FP64 issue bounds it (one warp instruction per 76 cycles and
+// sub-partition): about 75 FP64 operations per tetrahedron against about 60 for the gradients
+// alone, and none of the products is left to the row fill.
+template <int DIM>
+__global__ void __launch_bounds__(256) p1_elem_kernel(const double *__restrict__ X, const int32_t *__restrict__ elems, int nt,
+                                                      const double *__restrict__ kappa, double c_stiff, double c_mass,
+                                                      double *__restrict__ out, double *__restrict__ measure) {
+    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (e >= nt) return;
+    constexpr int NV = DIM + 1;
+    int32_t v[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = __ldg(elems + e * NV + i);
+    double V[DIM][DIM], c[3];
+    edge_vectors<DIM>(X, v, V);
+    const double det = edge_det(V, c);
+    const double meas = measure_of<DIM>(det);
+    if (measure) measure[e] = meas;
+    if (!out) return;
+    const double w = (kappa ? kappa[e] : 1.0) * c_stiff / (DIM == 2 ? 2.0 * det : 6.0 * det);
+    double K[NV][NV];
+    if constexpr (DIM == 2) {
+        // edges opposite the vertices: e0 = V2 - V1, e1 = -V2, e2 = V1
+        const double x0 = V[1][0] - V[0][0], y0 = V[1][1] - V[0][1];
+        K[0][1] = -w * fma(x0, V[1][0], y0 * V[1][1]);
+        K[0][2] = w * fma(x0, V[0][0], y0 * V[0][1]);
+        K[1][2] = -w * fma(V[1][0], V[0][0], V[1][1] * V[0][1]);
+        K[0][0] = -(K[0][1] + K[0][2]);
+        K[1][1] = -(K[0][1] + K[1][2]);
+        K[2][2] = -(K[0][2] + K[1][2]);
+    } else {
+        // N1 = V1 x V2 (c), N2 = V2 x V0, N3 = V0 x V1
+        const double p0 = det2(V[2][1], V[2][2], V[0][1], V[0][2]), p1 = det2(V[2][2], V[2][0], V[0][2], V[0][0]),
+                     p2 = det2(V[2][0], V[2][1], V[0][0], V[0][1]);
+        const double q0 = det2(V[0][1], V[0][2], V[1][1], V[1][2]), q1 = det2(V[0][2], V[0][0], V[1][2], V[1][0]),
+                     q2 = det2(V[0][0], V[0][1], V[1][0], V[1][1]);
+        K[1][1] = w * fma(c[2], c[2], fma(c[1], c[1], c[0] * c[0]));
+        K[2][2] = w * fma(p2, p2, fma(p1, p1, p0 * p0));
+        K[3][3] = w * fma(q2, q2, fma(q1, q1, q0 * q0));
+        K[1][2] = w * fma(c[2], p2, fma(c[1], p1, c[0] * p0));
+        K[1][3] = w * fma(c[2], q2, fma(c[1], q1, c[0] * q0));
+        K[2][3] = w * fma(p2, q2, fma(p1, q1, p0 * q0));
+        K[0][1] = -(K[1][1] + K[1][2] + K[1][3]);
+        K[0][2] = -(K[1][2] + K[2][2] + K[2][3]);
+        K[0][3] = -(K[1][3] + K[2][3] + K[3][3]);
+        K[0][0] = -(K[0][1] + K[0][2] + K[0][3]);
     }
-    int P = pow2_ceil(max(m, 32));
-    for (int p = lane; p < P; p += 32) {
-        int v = 0x7fffffff;
-        if (p < m) {
-            int t = p / nn, i = p - t * nn;
-            v = nodes[(int64_t)inc_elem[b + t] * nn + i];
-        }
-        s[p] = v;
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+        for (int j = 0; j < i; ++j) K[i][j] = K[j][i];
+    if (c_mass != 0.0) {
+        const double m = c_mass * meas * (DIM == 3 ? 1.0 / 20.0 : 1.0 / 12.0);
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+#pragma unroll
+            for (int j = 0; j < NV; ++j) K[i][j] += i == j ? 2.0 * m : m;
     }
-    __syncwarp();
-    warp_bitonic_sort(s, P);
-    int count = 0, prev = (int)0x80000000;
-    for (int c = 0; c < P; c += 32) {
-        int v = s[c + lane];
-        int vp = __shfl_up_sync(0xffffffffu, v, 1);
-        if (lane == 0) vp = prev;
-        bool f = (v != 0x7fffffff) && (v != vp);
-        unsigned bal = __ballot_sync(0xffffffffu, f);
-        prev = __shfl_sync(0xffffffffu, v, 31);
-        __syncwarp();
-        if (f) s[count + __popc(bal & ((1u << lane) - 1u))] = v;
-        count += __popc(bal);
-        __syncwarp();
-    }
-    return count;
+    double *o = out + e * NV * 4;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) store4(o + 4 * i, K[i][0], K[i][1], K[i][2], DIM == 3 ? K[i][NV - 1] : 0.0);
 }
 
-__global__ void row_count_kernel(int nnodes, const int32_t *inc_ptr, const int32_t *inc_elem,
-                                 const int32_t *nodes, int nn, int32_t *deg, int *status) {
-    __shared__ int sh[4][kCandMax];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// ------------------------------------------------------------------ pattern
+// Warp per row.  The candidates (all nodes of the incident elements, in incidence order) go into
+// a hash table of H >= their number entries, so each distinct node is kept once; the rank of
+// a node is the count of smaller ones (an O(degree^2 / 32) loop of broadcast reads: shorter than a
+// sort up to the degrees FE meshes have).  tmpcol: the row's sorted columns at inc_ptr[a] * NN;
+// rmap: rank of node lb of incidence t at t * NN + lb; drank: rank of the row's own node.
+template <int NN>
+__global__ void __launch_bounds__(128) pattern_kernel(int nnodes, const int32_t *__restrict__ inc_ptr,
+                                                      const int32_t *__restrict__ inc, const int32_t *__restrict__ nodes,
+                                                      int logH, int32_t *__restrict__ deg, int32_t *__restrict__ tmpcol,
+                                                      uint16_t *__restrict__ rmap, int32_t *__restrict__ drank, int *status) {
+    extern __shared__ int sh_pat[];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, H = 1 << logH;
+    int *tab = sh_pat + w * 3 * H, *lst = tab + H;
+    uint16_t *sl = reinterpret_cast<uint16_t *>(lst + H), *lsl = sl + H;
     for (int a = blockIdx.x * 4 + w; a < nnodes; a += gridDim.x * 4) {
-        int d = gather_row(a, inc_ptr, inc_elem, nodes, nn, sh[w], status);
-        if (lane == 0) deg[a] = d < 0 ? 0 : d;
+        const int b = inc_ptr[a], m = (inc_ptr[a + 1] - b) * NN;
+        if (m > kCandMax) { if (lane == 0) { dev_fail(status, kDevCandOverflow); deg[a] = 0; } continue; }
+        for (int i = lane; i < H; i += 32) tab[i] = -1;
+        __syncwarp();
+        for (int p = lane; p < m; p += 32) {
+            const int t = p / NN, i = p - t * NN;
+            const int v = __ldg(nodes + __ldg(inc + b + t) / NN * NN + i);
+            int h = (int)(((unsigned)v * 2654435761u) >> (32 - logH));
+            for (;;) {
+                const int old = atomicCAS(tab + h, -1, v);
+                if (old == -1 || old == v) break;
+                h = (h + 1) & (H - 1);
+            }
+            sl[p] = (uint16_t)h;
+        }
+        __syncwarp();
+        int u = 0;
+        for (int c = 0; c < H; c += 32) {
+            const int v = tab[c + lane];
+            const unsigned bal = __ballot_sync(0xffffffffu, v >= 0);
+            if (v >= 0) {
+                const int i = u + __popc(bal & ((1u << lane) - 1u));
+                lst[i] = v;
+                lsl[i] = (uint16_t)(c + lane);
+            }
+            u += __popc(bal);
+        }
+        __syncwarp();
+        bool self = false;
+        for (int i = lane; i < u; i += 32) {
+            const int v = lst[i];
+            int r = 0;
+#pragma unroll 4
+            for (int k = 0; k < u; ++k) r += lst[k] < v;
+            tmpcol[(int64_t)b * NN + r] = v;
+            tab[lsl[i]] = r;
+            if (v == a) { drank[a] = r; self = true; }
+        }
+        self = __any_sync(0xffffffffu, self);
+        for (int p = lane; p < m; p += 32) rmap[(int64_t)b * NN + p] = (uint16_t)tab[sl[p]];
+        if (lane == 0) {
+            deg[a] = u;
+            if (!self) { drank[a] = 0; dev_fail(status, kDevNotFound); }
+        }
         __syncwarp();
     }
 }
 
 // ------------------------------------------------------------------ fill + numeric pass
 struct FillArgs {
-    int nnodes, nt;
-    const int32_t *inc_ptr, *inc_elem;
-    const uint8_t *inc_loc;
+    int nnodes;
+    const int32_t *inc_ptr, *inc;
     const int32_t *nodes;
-    const double *geo;
+    const double *geo;        // element geometry (only where the fill itself forms or scales entries)
     const int32_t *browptr;
-    int32_t *bcol;            // NULL: numeric only (pattern already built)
-    const int32_t *pcol;      // numeric only: the stored pattern, read instead of re-gathering rows
-    int32_t *diagpos;         // block index of the diagonal block, written with the pattern
-    double *val;              // NULL: no matrix (linear form only)
-    double *rhs;              // NULL: no linear form
-    const double *fP0;        // nt*bs or NULL
-    const double *fint;       // element vectors of a source at quadrature points, or NULL
+    int32_t *bcol;
+    const uint16_t *rmap;     // rank in its row of every node of every incidence (pattern_kernel)
+    const int32_t *tmpcol;    // first numeric pass: the rows' columns and own ranks as pattern_kernel
+    const int32_t *drank;     //   left them, copied to bcol / diagpos; NULL later
+    int32_t *diagpos;         // block index of the diagonal block
+    double *val;
+    const double *kloc;       // element stiffness matrices, row la of element e at (e * NN + la) * krs, or NULL
+    int krs;
     const double *mloc;       // element mass matrices of a coefficient at quadrature points, or NULL
-    const double *kloc;       // element stiffness matrices of a coefficient at quadrature points, or NULL
     const double *tloc;       // element matrices of the general volume terms (ffgpu_varf.terms), or NULL
     const double *lame;       // per-element (lambda, mu) of the elasticity form, or NULL
     const double *eloc;       // [P2]^3 element blocks from the tensor cores (ffgpu_elemtc.cu), or NULL
-    double f0, f1, f2;
-    double c_mass;
+    double c_mass;            // mass term to add (has_mass); none where kloc includes it
+    int has_mass;
     double lam, mu;           // elasticity
     const uint8_t *onbc;
-    const double *g;
     double tgv;
+    int tgv_rows;             // tgv > 0 and there is an on(...)
+    int neg;                  // tgv < 0 and there is an on(...): the NegTgv bits of the variant
     int max_deg;
     int *status;
-    // boundary terms (NULL bptr: none): node -> codes b*NN + il, element vectors / matrices
+    // boundary terms (NULL bptr: none): node -> codes b*NN + il, element matrices
     const int32_t *bptr, *blist, *bel_elem;
-    const double *brhs, *bmat;
+    const double *bmat;
 };
 
-// FE: 1 = P1 scalar, 2 = P2 scalar, 3 = [P2]^3 elasticity
-template <int DIM, int FE>
-__global__ void __launch_bounds__(128) row_fill_kernel(FillArgs A) {
+enum NegTgv { kNegOn = 1, kNegKeepRow = 2, kNegZeroCol = 4, kNegZeroColDiag = 8, kNegZeroDiag = 16 };
+
+static int neg_tgv_bits(double tgv) {
+    if (!(tgv < 0)) return 0;
+    const auto is = [&](double v) { return fabs(tgv + v) < 1e-10; };
+    int bits = kNegOn;
+    if (is(3.0) || is(30.0)) bits |= kNegKeepRow;
+    if (is(2.0) || is(20.0) || is(3.0) || is(30.0)) bits |= kNegZeroCol;
+    if (tgv < -19.0) bits |= kNegZeroColDiag;
+    if (tgv < -9.0) bits |= kNegZeroDiag;
+    return bits;
+}
+
+// Numeric fill.  FE: 1 = P1 scalar, 2 = P2 scalar, 3 = [P2]^3 elasticity.
+// A group of GL lanes owns a row, RW rows per warp: lane lb of a scalar group adds entry (la, lb)
+// of one incident element after the other to the row in shared memory; a [P2]^3 group has a lane
+// per (lb, component) and adds three values.  The nodes of one element are distinct, so the lanes
+// of a step never meet on an entry, and every FP64 add is issued by all the rows of the warp at
+// once: FP64 issue (76 cycles per warp instruction and sub-partition, however many lanes are
+// active) bounds the fill, and a step per incident element is the fewest adds there are.
+// The form this replaces gave the row one copy per concurrent element and summed the copies:
+// 21 warp adds per P1 row in 3D instead of 3.  PLAIN: the element matrices are complete (kloc or
+// eloc and nothing to add); the general form keeps its tests out of that loop.  On 96^3 cells (912 673 rows, 13.4 M entries), the
+// products moved to p1_elem_kernel (0.76 ms): 3.27 -> 0.30 ms; 16 % of the old form's time was FP64
+// compares with constants, which cost as much as an add and are now made on the host.
+template <int DIM, int FE, bool PLAIN>
+__global__ void __launch_bounds__(256) fill_kernel(FillArgs A) {
     constexpr int nvk = DIM + 1;
     constexpr int NN = FE == 1 ? nvk : (DIM == 3 ? 10 : 6);
     constexpr int BS = FE == 3 ? 3 : 1;
     constexpr int BS2 = BS * BS;
-    // lanes = slot * NN + lb: SLOTS incident elements per step, each lane one block (la, lb).
-    // Every slot accumulates into its own copy of the row (acc[slot][k][q]) so that one step
-    // is one full-warp FP64 add; the copies are summed in slot order at the end.  Entries are
-    // therefore formed as sum_s (sum of the slot's elements in element order): deterministic,
-    // and the same association rhs_kernel uses for the linear form.
-    constexpr int SLOTS = 32 / NN;
-    extern __shared__ __align__(16) unsigned char sh_raw[];
+    constexpr int GL = NN * BS, RW = 32 / GL;
+    constexpr int STEP = 4;          // incident elements whose loads are in flight together
+    extern __shared__ __align__(16) double sh_fill[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int warps = blockDim.x >> 5;
-    int *cols = (int *)sh_raw + w * kCandMax;
-    double *acc = (double *)((int *)sh_raw + warps * kCandMax) + (int64_t)w * SLOTS * A.max_deg * BS2;
-    const double mfac = DIM == 3 ? 1.0 / 20.0 : 1.0 / 12.0;
-    const bool has_mass = A.c_mass != 0.0 && !A.mloc;
+    double *rows = sh_fill + (int64_t)w * RW * A.max_deg * BS2;
+    const int grp = lane / GL, sub = lane - grp * GL;
+    const int lb = sub / BS, c = sub - lb * BS;
 
-    for (int a = blockIdx.x * warps + w; a < A.nnodes; a += gridDim.x * warps) {
-        int deg;
-        if (A.pcol) {
-            // the row's sorted columns as the pattern pass stored them
-            const int64_t r0 = A.browptr[a];
-            deg = (int)(A.browptr[a + 1] - r0);
-            if (deg > kCandMax) { if (lane == 0) dev_fail(A.status, kDevCandOverflow); continue; }
-            for (int r = lane; r < deg; r += 32) cols[r] = A.pcol[r0 + r];
-            __syncwarp();
-        } else {
-            deg = gather_row(a, A.inc_ptr, A.inc_elem, A.nodes, NN, cols, A.status);
-        }
-        if (deg < 0) continue;
-        if (deg > A.max_deg) { if (lane == 0) dev_fail(A.status, kDevDegOverflow); continue; }
-        const int64_t rb = A.browptr[a];
-        if (A.bcol)
-            for (int r = lane; r < deg; r += 32) A.bcol[rb + r] = cols[r];
-        const int span = deg * BS2;   // one slot copy
-        for (int q = lane; q < SLOTS * span; q += 32) acc[q] = 0.0;
-        double racc = 0.0;   // rhs partial of slot `lane / NN`, component `lane % NN` (< BS)
+    for (int64_t a0 = ((int64_t)blockIdx.x * warps + w) * RW; a0 < A.nnodes; a0 += (int64_t)gridDim.x * warps * RW) {
+        const int a = (int)a0 + grp;
+        const bool act = grp < RW && a < A.nnodes;
+        const int last = (int)min((int64_t)A.nnodes, a0 + RW);
+        const int rb0 = A.browptr[a0], total = (A.browptr[last] - rb0) * BS2;
+        const int rb = act ? A.browptr[a] : rb0, deg = act ? A.browptr[a + 1] - rb : 0;
+        double *acc = rows + (int64_t)(rb - rb0) * BS2;
+        for (int q = lane; q < total; q += 32) rows[q] = 0.0;
+        const int ib = act ? A.inc_ptr[a] : 0, ie = act ? A.inc_ptr[a + 1] : 0;
+        const int steps = __reduce_max_sync(0xffffffffu, ie - ib);
         __syncwarp();
-        const int ib = A.inc_ptr[a], ie = A.inc_ptr[a + 1];
-        for (int t0 = ib; t0 < ie; t0 += SLOTS) {
-            // ---- element contributions of this step
-            const int slot = lane / NN;
-            const int lb = lane - slot * NN;
-            const int t = t0 + slot;
-            const bool act = slot < SLOTS && t < ie;
-            int rank = -1;
-            double v[BS2];
+        for (int s0 = 0; s0 < steps; s0 += STEP) {
+            double v[STEP][BS];
+            int rk[STEP];
 #pragma unroll
-            for (int q = 0; q < BS2; ++q) v[q] = 0.0;
-            if (act) {
-                const int e = A.inc_elem[t];
-                const int la = A.inc_loc[t];
-                const double *ge = A.geo + (int64_t)e * kGeoStride;
-                const double meas = __ldg(ge), kap = __ldg(ge + 1);
-                const double *G = ge + 4;
-                const int nb = A.nodes[(int64_t)e * NN + lb];
-                rank = find_sorted(cols, deg, nb);
-                if (FE == 1) {
-                    double s = 0;
+            for (int u = 0; u < STEP; ++u) {
+                const int t = ib + s0 + u;
+                rk[u] = -1;
+                if (t >= ie) continue;
+                const int64_t sl = __ldg(A.inc + t);   // e * NN + la
+                rk[u] = __ldg(A.rmap + (int64_t)t * NN + lb);
+                if (PLAIN) {
+                    const double *src = FE == 3 ? A.eloc + (sl * NN + lb) * 9 + 3 * c : A.kloc + sl * A.krs + lb;
 #pragma unroll
-                    for (int d = 0; d < DIM; ++d) s += __ldg(G + 3 * la + d) * __ldg(G + 3 * lb + d);
-                    double val = A.kloc ? A.kloc[((int64_t)e * NN + la) * NN + lb] : kap * meas * s;
-                    if (has_mass) val += A.c_mass * meas * mfac * (la == lb ? 2.0 : 1.0);
-                    if (A.mloc) val += A.mloc[((int64_t)e * NN + la) * NN + lb];
-                    if (A.tloc) val += A.tloc[((int64_t)e * NN + la) * NN + lb];
-                    v[0] = val;
-                } else if (FE == 2) {
-                    const double m = meas * mfac;
-                    v[0] = A.kloc ? A.kloc[((int64_t)e * NN + la) * NN + lb] : kap * m * P2Pair<DIM>(G, la, lb).trace();
-                    if (has_mass) v[0] += A.c_mass * meas * p2_mass<DIM>(la, lb);
-                    if (A.mloc) v[0] += A.mloc[((int64_t)e * NN + la) * NN + lb];
-                    if (A.tloc) v[0] += A.tloc[((int64_t)e * NN + la) * NN + lb];
-                } else if (A.eloc) {
-                    const double *eb = A.eloc + (((int64_t)e * NN + la) * NN + lb) * BS2;
-#pragma unroll
-                    for (int q = 0; q < BS2; ++q) v[q] = __ldg(eb + q);
+                    for (int q = 0; q < BS; ++q) v[u][q] = __ldg(src + q);
+                    continue;
+                }
+                const int64_t e = sl / NN;
+                const int la = (int)(sl - e * NN);
+                const double *ge = A.geo + e * kGeoStride;
+                if (FE <= 2) {
+                    double x;
+                    if (A.kloc) {
+                        x = __ldg(A.kloc + sl * A.krs + lb);
+                    } else {
+                        // P2 without the tensor-core element matrices
+                        x = __ldg(ge + 1) * (__ldg(ge) * (DIM == 3 ? 1.0 / 20.0 : 1.0 / 12.0)) *
+                            (FE == 2 ? P2Pair<DIM>(ge + 4, la, lb).trace() : 0.0);
+                    }
+                    if (A.has_mass) {
+                        const double meas = __ldg(ge);
+                        x += FE == 1 ? A.c_mass * meas * (DIM == 3 ? 1.0 / 20.0 : 1.0 / 12.0) * (la == lb ? 2.0 : 1.0)
+                                     : A.c_mass * meas * p2_mass<DIM>(la, lb);
+                    }
+                    if (A.mloc) x += __ldg(A.mloc + sl * NN + lb);
+                    if (A.tloc) x += __ldg(A.tloc + sl * NN + lb);
+                    v[u][0] = x;
                 } else {
-                    const P2Pair<DIM> P(G, la, lb);
-                    const double m = meas * mfac;
-                    {
-                        const double tr = P.trace();
-                        const double lam = A.lame ? __ldg(A.lame + 2 * (int64_t)e) : A.lam;
-                        const double mu = A.lame ? __ldg(A.lame + 2 * (int64_t)e + 1) : A.mu;
+                    const P2Pair<DIM> P(ge + 4, la, lb);
+                    const double m = __ldg(ge) * (1.0 / 20.0), tr = P.trace();
+                    const double lam = A.lame ? __ldg(A.lame + 2 * e) : A.lam;
+                    const double mu = A.lame ? __ldg(A.lame + 2 * e + 1) : A.mu;
 #pragma unroll
-                        for (int c = 0; c < 3; ++c)
-#pragma unroll
-                            for (int cp = 0; cp < 3; ++cp) {
-                                double x = lam * P.g(c, cp) + mu * P.g(cp, c);
-                                if (cp == c) x += mu * tr;
-                                v[3 * c + cp] = m * x;
-                            }
+                    for (int q = 0; q < BS; ++q) {
+                        double x = lam * P.g(c, q) + mu * P.g(q, c);
+                        if (q == c) x += mu * tr;
+                        v[u][q] = m * x;
                     }
                 }
-                if (rank < 0) dev_fail(A.status, kDevNotFound);
             }
-            // ---- accumulate: each slot into its own copy, no two lanes on one entry
-            if (act && rank >= 0) {
 #pragma unroll
-                for (int q = 0; q < BS2; ++q) acc[slot * span + rank * BS2 + q] += v[q];
-            }
-            // ---- linear form: lane (slot, c < BS) adds its element's share to component c
-            if (A.rhs && act && lb < BS) {
-                const int ee = A.inc_elem[t], ll = A.inc_loc[t];
-                const double meas = A.geo[(int64_t)ee * kGeoStride];
-                const double f = A.fP0 ? A.fP0[(int64_t)ee * BS + lb] : (lb == 0 ? A.f0 : (lb == 1 ? A.f1 : A.f2));
-                // explicit roundings: the linear-form-only kernel forms the same sums bit for bit
-                const double add = A.fint ? A.fint[((int64_t)ee * NN + ll) * BS + lb]
-                                          : __dmul_rn(__dmul_rn(meas, f), FE == 1 ? 1.0 / (DIM + 1)
-                                                                                  : basis_integral<DIM, 2>(1.0, ll));
-                racc = __dadd_rn(racc, add);
-            }
-            __syncwarp();
-        }
-        // ---- sum the slot copies (slot order); slots no element reached hold zeros and are
-        // skipped (a row with ie - ib < SLOTS incident elements fills only that many)
-        const int nsl = min(SLOTS, ie - ib);
-        for (int q = lane; q < span; q += 32) {
-            double t = acc[q];
-            for (int sl = 1; sl < nsl; ++sl) t += acc[sl * span + q];
-            acc[q] = t;
-        }
-        {
-            double r = 0.0;
-            for (int sl = 0; sl < max(nsl, 1); ++sl) {
-                const double p = __shfl_sync(0xffffffffu, racc, sl * NN + (lane < BS ? lane : 0));
-                r = sl == 0 ? p : r + p;
-            }
-            racc = r;   // lanes < BS: component `lane`
-        }
-        __syncwarp();
-        // ---- boundary terms, boundary element by boundary element, after the volume sum
-        if (A.bptr) {
-            const int p1 = A.bptr[a + 1];
-            for (int p = A.bptr[a]; p < p1; ++p) {
-                const int code = A.blist[p];
-                const int bb = code / NN, il = code - bb * NN;
-                if (A.bmat && A.val && lane < NN) {
-                    const int cn = A.nodes[(int64_t)A.bel_elem[bb] * NN + lane];
-                    const int rk = find_sorted(cols, deg, cn);
-                    const double m = A.bmat[((int64_t)bb * NN + il) * NN + lane];
-                    if (rk < 0) dev_fail(A.status, kDevNotFound);
-                    else
+            for (int u = 0; u < STEP; ++u) {
+                if (rk[u] >= 0) {
 #pragma unroll
-                        for (int c = 0; c < BS; ++c) acc[rk * BS2 + c * BS + c] += m;
+                    for (int q = 0; q < BS; ++q) acc[rk[u] * BS2 + c * BS + q] += v[u][q];
                 }
-                if (A.brhs && A.rhs && lane < BS) racc += A.brhs[((int64_t)bb * BS + lane) * NN + il];
+                __syncwarp();   // the next element's lanes may meet this one's entries
+            }
+        }
+        // ---- the row's columns: copied out by the first pass, where on(...) looks them up later
+        const int32_t *cs = A.tmpcol ? A.tmpcol + (int64_t)ib * NN : A.bcol + rb;
+        if (A.tmpcol)
+            for (int r = sub; r < deg; r += GL) A.bcol[rb + r] = cs[r];
+        const int self = act ? (A.tmpcol ? A.drank[a] : A.diagpos[a] - rb) : 0;
+        if (A.tmpcol && act && sub == 0) A.diagpos[a] = rb + self;
+        // ---- boundary terms, boundary element by boundary element, after the volume sum
+        if (A.bptr && A.bmat) {
+            const int p0 = act ? A.bptr[a] : 0, p1 = act ? A.bptr[a + 1] : 0;
+            const int nb = __reduce_max_sync(0xffffffffu, p1 - p0);
+            for (int s = 0; s < nb; ++s) {
+                if (p0 + s < p1) {
+                    const int code = A.blist[p0 + s];
+                    const int bb = code / NN, il = code - bb * NN;
+                    const int cn = A.nodes[(int64_t)A.bel_elem[bb] * NN + lb];
+                    const int r = find_sorted(cs, deg, cn);
+                    if (r < 0) dev_fail(A.status, kDevNotFound);
+                    else acc[r * BS2 + c * BS + c] += A.bmat[((int64_t)bb * NN + il) * NN + lb];
+                }
                 __syncwarp();
             }
         }
-        // ---- Dirichlet rows (tgv > 0): diagonal := tgv, rhs := tgv * g
-        int self = find_sorted(cols, deg, a);
-        if (self < 0) { if (lane == 0) dev_fail(A.status, kDevNotFound); continue; }
-        if (A.bcol && lane == 0) A.diagpos[a] = (int32_t)(rb + self);
-        if (lane < BS) {
-            int64_t dof = (int64_t)a * BS + lane;
-            bool on = A.onbc && A.onbc[dof];
-            if (on && A.tgv > 0) {
-                if (A.val) acc[self * BS2 + lane * BS + lane] = A.tgv;
-                racc = A.tgv * (A.g ? A.g[dof] : 0.0);
-            } else if (on) {
-                racc = A.g ? A.g[dof] : 0.0;   // tgv < 0: b_i = g_i (tgv1 = 1, problem.cpp:9937)
-            }
-            if (A.rhs) A.rhs[dof] = racc;
-        }
+        // ---- Dirichlet rows (tgv > 0): diagonal := tgv
+        if (act && sub < BS && A.tgv_rows && A.onbc[(int64_t)a * BS + sub])
+            acc[self * BS2 + sub * BS + sub] = A.tgv;
         __syncwarp();
         // tgv < 0 (HashMatrix::SetBC, HashMatrix.cpp:1195-1238): Dirichlet rows get a unit
         // diagonal (0 when tgv <= -10) and, except for -3/-30, zero off-diagonals; for
         // -2/-20/-3/-30 the Dirichlet columns are zeroed too (the diagonal also for -20/-30).
-        if (A.val && A.onbc && A.tgv < 0) {
-            const double tgv = A.tgv;
-            const bool keep_row = fabs(tgv + 3.0) < 1e-10 || fabs(tgv + 30.0) < 1e-10;
-            const bool zero_col = fabs(tgv + 2.0) < 1e-10 || fabs(tgv + 20.0) < 1e-10 || fabs(tgv + 3.0) < 1e-10 ||
-                                  fabs(tgv + 30.0) < 1e-10;
-            for (int q = lane; q < deg * BS2; q += 32) {
+        // (the tests on tgv are made on the host: FP64 compares would cost more than the sums)
+        if (A.neg) {
+            for (int q = sub; q < deg * BS2; q += GL) {
                 const int k = q / BS2, r = (q % BS2) / BS, cp = q % BS;
-                const int col = cols[k];
+                const int col = cs[k];
                 const bool diag = col == a && r == cp;
-                double v = acc[q];
-                if (A.onbc[(int64_t)a * BS + r]) v = diag ? (tgv < -9.0 ? 0.0 : 1.0) : (keep_row ? v : 0.0);
-                if (zero_col && A.onbc[(int64_t)col * BS + cp] && (!diag || tgv < -19.0)) v = 0.0;
-                acc[q] = v;
+                const bool mine = A.onbc[(int64_t)a * BS + r];
+                const bool gone = (mine && !(A.neg & kNegKeepRow) && !diag) ||
+                                  ((A.neg & kNegZeroCol) && (!diag || (A.neg & kNegZeroColDiag)) && A.onbc[(int64_t)col * BS + cp]);
+                if (gone) acc[q] = 0.0;
+                else if (mine && diag) acc[q] = A.neg & kNegZeroDiag ? 0.0 : 1.0;
             }
             __syncwarp();
         }
-        if (A.val)
-            for (int q = lane; q < deg * BS2; q += 32) A.val[rb * BS2 + q] = acc[q];
+        for (int q = lane; q < total; q += 32) A.val[(int64_t)rb0 * BS2 + q] = rows[q];
         __syncwarp();
     }
 }
 
-// linear form only (real[int] b = a(0,Vh)): per node, sum over incident elements
+// linear form (real[int] b = a(0,Vh), alone or beside the matrix): per node, sum over incident
+// elements; measure[e * mstride] is the measure of element e
 template <int DIM, int FE>
-__global__ void rhs_kernel(int nnodes, const int32_t *inc_ptr, const int32_t *inc_elem,
-                           const uint8_t *inc_loc, const double *geo, const double *fP0,
+__global__ void rhs_kernel(int nnodes, const int32_t *inc_ptr, const int32_t *inc, const double *measure, int mstride, const double *fP0,
                            const double *fint, double f0, double f1, double f2, const uint8_t *onbc,
                            const double *g,
                            double tgv, double *rhs, const int32_t *bptr, const int32_t *blist,
                            const double *brhs) {
     constexpr int BS = FE == 3 ? 3 : 1;
-    // same association as the fill kernel's fused linear form: element p of the node goes to
-    // partial p % SLOTS, partials summed in order
+    // element p of the node goes to partial p % SLOTS, partials summed in order
     constexpr int NN = FE == 1 ? DIM + 1 : (DIM == 3 ? 10 : 6);
     constexpr int SLOTS = 32 / NN;
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -629,8 +661,8 @@ __global__ void rhs_kernel(int nnodes, const int32_t *inc_ptr, const int32_t *in
         for (int sl = 0; sl < SLOTS; ++sl) {
             const int p = p0 + sl;
             if (p < ie) {
-                int e = inc_elem[p], l = inc_loc[p];
-                double meas = geo[(int64_t)e * kGeoStride];
+                const int e = inc[p] / NN, l = inc[p] - e * NN;
+                double meas = measure[(int64_t)e * mstride];
                 double f = fP0 ? fP0[(int64_t)e * BS + c] : (c == 0 ? f0 : (c == 1 ? f1 : f2));
                 const double add = fint ? fint[((int64_t)e * NN + l) * BS + c]
                                         : __dmul_rn(__dmul_rn(meas, f), FE == 1 ? 1.0 / (DIM + 1)
@@ -786,22 +818,67 @@ using namespace ffgpu;
 // ------------------------------------------------------------------ helpers on the host
 static int fill_launch(ffgpu_space *S, FillArgs &fa) {
     ffgpu_ctx *ctx = S->ctx;
-    const int warps = 4;
-    int bs2 = S->bs * S->bs;
-    const int nn = S->nn, slots = 32 / nn;
-    size_t smem = (size_t)warps * kCandMax * sizeof(int) + (size_t)warps * slots * fa.max_deg * bs2 * sizeof(double);
-    int grid = min(kNumSM * 16, max(1, (S->nnodes + warps - 1) / warps));
+    const int bs2 = S->bs * S->bs, rw = 32 / (S->nn * S->bs);
+    // a row above this degree has always been refused
+    FFGPU_CHECK((size_t)4 * (kCandMax * sizeof(int) + (size_t)(32 / S->nn) * fa.max_deg * bs2 * sizeof(double)) <= 200 * 1024,
+                FFGPU_EMESH, "row degree %d too large for shared memory", fa.max_deg);
+    const bool plain = (S->fe == FFGPU_FE_P2VEC3 ? fa.eloc : fa.kloc) && !fa.has_mass && !fa.mloc && !fa.tloc;
     void (*kern)(FillArgs) = nullptr;
-    if (S->dim == 2 && S->fe == FFGPU_FE_P1) kern = row_fill_kernel<2, 1>;
-    if (S->dim == 3 && S->fe == FFGPU_FE_P1) kern = row_fill_kernel<3, 1>;
-    if (S->dim == 2 && S->fe == FFGPU_FE_P2) kern = row_fill_kernel<2, 2>;
-    if (S->dim == 3 && S->fe == FFGPU_FE_P2) kern = row_fill_kernel<3, 2>;
-    if (S->dim == 3 && S->fe == FFGPU_FE_P2VEC3) kern = row_fill_kernel<3, 3>;
+    if (S->dim == 2 && S->fe == FFGPU_FE_P1) kern = plain ? fill_kernel<2, 1, true> : fill_kernel<2, 1, false>;
+    if (S->dim == 3 && S->fe == FFGPU_FE_P1) kern = plain ? fill_kernel<3, 1, true> : fill_kernel<3, 1, false>;
+    if (S->dim == 2 && S->fe == FFGPU_FE_P2) kern = plain ? fill_kernel<2, 2, true> : fill_kernel<2, 2, false>;
+    if (S->dim == 3 && S->fe == FFGPU_FE_P2) kern = plain ? fill_kernel<3, 2, true> : fill_kernel<3, 2, false>;
+    if (S->dim == 3 && S->fe == FFGPU_FE_P2VEC3) kern = plain ? fill_kernel<3, 3, true> : fill_kernel<3, 3, false>;
     FFGPU_CHECK(kern, FFGPU_EINVAL, "unsupported element (dim %d, fe %d)", S->dim, S->fe);
-    FFGPU_CHECK(smem <= 200 * 1024, FFGPU_EMESH, "row degree %d too large for shared memory", fa.max_deg);
+    // warps per block: 8, fewer where rows are long (48 KB of row buffers a block keep the SM full)
+    const size_t per_warp = (size_t)rw * fa.max_deg * bs2 * sizeof(double);
+    int warps = 8;
+    while (warps > 1 && warps * per_warp > 48 * 1024) warps >>= 1;
+    const size_t smem = warps * per_warp;
+    const int64_t need = ((int64_t)S->nnodes + warps * rw - 1) / (warps * rw);
     FFGPU_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, warps * 32, smem, ctx->stream>>>(fa);
-    return launch_check(ctx, "row_fill_kernel");
+    kern<<<(int)std::min<int64_t>(kNumSM * 32, std::max<int64_t>(1, need)), warps * 32, smem, ctx->stream>>>(fa);
+    return launch_check(ctx, "fill_kernel");
+}
+
+static int pattern_launch(ffgpu_space *S, int32_t *deg, int32_t *tmpcol, uint16_t *rmap, int32_t *drank) {
+    ffgpu_ctx *ctx = S->ctx;
+    int logH = 5;
+    while ((1 << logH) < S->max_inc * S->nn && logH < 9) ++logH;   // kCandMax = 512 candidates at most
+    const size_t smem = (size_t)4 * 3 * sizeof(int) << logH;
+    const int grid = std::min(kNumSM * 16, std::max(1, (S->nnodes + 3) / 4));
+#define FFGPU_PATTERN(NN)                                                                                        \
+    pattern_kernel<NN><<<grid, 128, smem, ctx->stream>>>(S->nnodes, S->inc_ptr, S->inc, S->nodes, logH, deg, \
+                                                         tmpcol, rmap, drank, ctx->d_status)
+    switch (S->nn) {
+        case 3: FFGPU_PATTERN(3); break;
+        case 4: FFGPU_PATTERN(4); break;
+        case 6: FFGPU_PATTERN(6); break;
+        default: FFGPU_PATTERN(10); break;
+    }
+#undef FFGPU_PATTERN
+    return launch_check(ctx, "pattern_kernel");
+}
+
+static int rhs_launch(ffgpu_space *S, const double *measure, int mstride, const double *fP0, const double *fint,
+                      const double *f, const uint8_t *mask, const double *g, double tgv, double *rhs,
+                      const BoundaryTerms &bt) {
+    auto k = rhs_kernel<2, 1>;
+    if (S->dim == 3 && S->fe == FFGPU_FE_P1) k = rhs_kernel<3, 1>;
+    if (S->dim == 2 && S->fe == FFGPU_FE_P2) k = rhs_kernel<2, 2>;
+    if (S->dim == 3 && S->fe == FFGPU_FE_P2) k = rhs_kernel<3, 2>;
+    if (S->dim == 3 && S->fe == FFGPU_FE_P2VEC3) k = rhs_kernel<3, 3>;
+    k<<<grid_for((int64_t)S->ndof, 256), 256, 0, S->ctx->stream>>>(S->nnodes, S->inc_ptr, S->inc, measure,
+                                                                   mstride, fP0, fint, f[0], f[1], f[2], mask, g, tgv, rhs,
+                                                                   bt.rhs ? bt.ptr : nullptr, bt.list, bt.rhs);
+    return launch_check(S->ctx, "rhs_kernel");
+}
+
+// P1 element matrices (out) and measures, either may be NULL
+static int p1_elem_launch(ffgpu_space *S, const double *kappa, double c_stiff, double c_mass, double *out, double *measure) {
+    auto k = S->dim == 2 ? p1_elem_kernel<2> : p1_elem_kernel<3>;
+    k<<<grid_for(S->nt, 256), 256, 0, S->ctx->stream>>>(S->coords, S->elems, S->nt, kappa, c_stiff, c_mass, out, measure);
+    return launch_check(S->ctx, "p1_elem_kernel");
 }
 
 static int varf_check(const ffgpu_space *S, const ffgpu_varf *v) {
@@ -824,18 +901,37 @@ static int run_geometry(ffgpu_space *S, const ffgpu_varf *v, double *geo) {
     return launch_check(ctx, "geometry_kernel");
 }
 
+// the varf needs the element geometry (measure, gradients) beyond the P1 element matrices
+static bool needs_geometry(const ffgpu_space *S, const ffgpu_varf *v) {
+    return S->fe != FFGPU_FE_P1 || v->f_qp || v->mass_qp || v->stiff_qp || v->f_expr || v->nterms > 0;
+}
+
+// Measures and gradients of the elements in M->geo.  P1 reads nothing else there, so it is formed
+// once per matrix and only when something asks for it; P2 also keeps kappa in it.
+int ffgpu::matrix_geometry(ffgpu_matrix *M, const ffgpu_varf *v) {
+    ffgpu_space *S = M->space;
+    if (M->geo && S->fe == FFGPU_FE_P1) return FFGPU_OK;
+    if (!M->geo && dalloc(M->ctx, (void **)&M->geo, sizeof(double) * kGeoStride * S->nt) != cudaSuccess) {
+        set_error("element geometry: device allocation failed");
+        return FFGPU_ENOMEM;
+    }
+    return run_geometry(S, v, M->geo);
+}
+
+// tmpcol, drank: what pattern_kernel left (first numeric pass of a matrix), else NULL
 static int numeric_pass(ffgpu_matrix *M, const ffgpu_varf *v, const ffgpu_bc *bc, double *rhs,
-                        bool build_cols) {
+                        const int32_t *tmpcol, const int32_t *drank) {
     ffgpu_space *S = M->space;
     ffgpu_ctx *ctx = S->ctx;
     FFGPU_TRY(varf_check(S, v));
-    FFGPU_TRY(run_geometry(S, v, M->geo));
     int bs = S->bs;
     DevIn<double> fP0(v->f, v->f ? (size_t)S->nt * bs : 0, ctx);
+    DevIn<double> kap(v->kappa, v->kappa && S->fe == FFGPU_FE_P1 ? S->nt : 0, ctx);
     DevIn<uint8_t> onbc(bc ? bc->onbc : nullptr, bc && bc->onbc ? S->ndof : 0, ctx);
     DevIn<double> gv(bc ? bc->g : nullptr, bc && bc->g ? S->ndof : 0, ctx);
     DevOut<double> rh(rhs, rhs ? S->ndof : 0, ctx, false);
-    FFGPU_TRY(fP0.err); FFGPU_TRY(onbc.err); FFGPU_TRY(gv.err); FFGPU_TRY(rh.err);
+    FFGPU_TRY(fP0.err); FFGPU_TRY(kap.err); FFGPU_TRY(onbc.err); FFGPU_TRY(gv.err); FFGPU_TRY(rh.err);
+    if (needs_geometry(S, v)) FFGPU_TRY(matrix_geometry(M, v));
     const uint8_t *mask = onbc.d;
     if (bc && !bc->onbc && bc->nlabels > 0) {
         if (!M->bcmask) FFGPU_CUDA(dalloc(ctx, (void **)&M->bcmask, S->ndof));
@@ -844,46 +940,57 @@ static int numeric_pass(ffgpu_matrix *M, const ffgpu_varf *v, const ffgpu_bc *bc
     }
     FillArgs fa;
     memset(&fa, 0, sizeof(fa));
-    fa.nnodes = S->nnodes; fa.nt = S->nt;
-    fa.inc_ptr = S->inc_ptr; fa.inc_elem = S->inc_elem; fa.inc_loc = S->inc_loc;
+    fa.nnodes = S->nnodes;
+    fa.inc_ptr = S->inc_ptr; fa.inc = S->inc;
     fa.nodes = S->nodes; fa.geo = M->geo; fa.browptr = M->browptr;
-    fa.bcol = build_cols ? M->bcol : nullptr;
-    fa.pcol = build_cols ? nullptr : M->bcol;
+    fa.bcol = M->bcol; fa.rmap = M->rmap; fa.tmpcol = tmpcol; fa.drank = drank;
     fa.diagpos = M->diagpos;
-    fa.val = M->val; fa.rhs = rh.d; fa.fP0 = fP0.d;
-    fa.f0 = v->f_const[0]; fa.f1 = v->f_const[1]; fa.f2 = v->f_const[2];
-    fa.c_mass = v->form == FFGPU_FORM_DIFFUSION ? v->c_mass : 0.0;
+    fa.val = M->val;
+    fa.c_mass = v->form == FFGPU_FORM_DIFFUSION && !v->mass_qp ? v->c_mass : 0.0;
     if (v->form == FFGPU_FORM_ELASTICITY) {
         fa.mu = v->E / (2 * (1 + v->nu));
         fa.lam = v->E * v->nu / ((1 + v->nu) * (1 - 2 * v->nu));
     }
-    fa.onbc = mask; fa.g = gv.d; fa.tgv = bc ? bc->tgv : 0.0;
+    fa.onbc = mask; fa.tgv = bc ? bc->tgv : 0.0;
+    fa.tgv_rows = mask && fa.tgv > 0;
+    fa.neg = mask ? neg_tgv_bits(fa.tgv) : 0;
     fa.max_deg = M->max_deg; fa.status = ctx->d_status;
     DevIn<double> lame(v->form == FFGPU_FORM_ELASTICITY ? v->lame : nullptr, (size_t)S->nt * 2, ctx);
     FFGPU_TRY(lame.err);
     fa.lame = lame.d;
-    double *fint = nullptr, *mloc = nullptr;
-    if (rh.d) FFGPU_TRY(source_prepare(S, v, M->geo, &fint));
-    double *kloc = nullptr, *tloc = nullptr;
-    int frc = mass_prepare(S, v, M->geo, &mloc);
+    double *fint = nullptr, *mloc = nullptr, *kloc = nullptr, *tloc = nullptr, *eloc = nullptr, *meas = nullptr;
+    int frc = rh.d ? source_prepare(S, v, M->geo, &fint) : FFGPU_OK;
+    if (!frc) frc = mass_prepare(S, v, M->geo, &mloc);
     if (!frc) frc = stiff_prepare(S, v, M->geo, &kloc);
     if (!frc) frc = terms_prepare(S, v, M->geo, &tloc);
-    // P2 stiffness / [P2]^3 elasticity with an element-constant coefficient: the element
-    // matrices from the tensor cores (a coefficient at the rule's points keeps its own path)
-    double *eloc = nullptr;
-    if (!frc && !kloc && (S->fe == FFGPU_FE_P2VEC3 || (S->fe == FFGPU_FE_P2 && v->c_stiff != 0.0)))
+    fa.kloc = kloc;
+    fa.krs = S->nn;
+    if (!frc && S->fe == FFGPU_FE_P1) {
+        // P1: closed form, the mass term included; only the measures where the stiffness comes
+        // from values at quadrature points
+        if (rh.d && dalloc(ctx, (void **)&meas, sizeof(double) * S->nt)) frc = FFGPU_ENOMEM;
+        if (!frc && !kloc && dalloc(ctx, (void **)&eloc, sizeof(double) * 4 * S->nn * S->nt)) frc = FFGPU_ENOMEM;
+        if (frc) set_error("assembly: allocation of the element matrices failed");
+        if (!frc && (eloc || meas)) frc = p1_elem_launch(S, kap.d, v->c_stiff, fa.c_mass, eloc, meas);
+        if (eloc) { fa.kloc = eloc; fa.krs = 4; fa.c_mass = 0.0; }
+    } else if (!frc && !kloc && (S->fe == FFGPU_FE_P2VEC3 || v->c_stiff != 0.0)) {
+        // P2 stiffness / [P2]^3 elasticity with an element-constant coefficient: the element
+        // matrices from the tensor cores (a coefficient at the rule's points keeps its own path)
         frc = elem_tc_prepare(S, M->geo, fa.lam, fa.mu, lame.d, &eloc);
-    if (frc) { dfree(ctx, fint); dfree(ctx, mloc); dfree(ctx, kloc); dfree(ctx, tloc); return frc; }
-    fa.fint = fint;
+        if (S->fe == FFGPU_FE_P2 && eloc) fa.kloc = eloc;
+        if (S->fe == FFGPU_FE_P2VEC3) fa.eloc = eloc;
+    }
+    fa.has_mass = fa.c_mass != 0.0;
     fa.mloc = mloc;
-    fa.kloc = S->fe == FFGPU_FE_P2 && eloc ? eloc : kloc;
-    fa.eloc = S->fe == FFGPU_FE_P2VEC3 ? eloc : nullptr;
     fa.tloc = tloc;
     BoundaryTerms bt;
-    frc = boundary_prepare(S, v, rh.d != nullptr, true, bt);
+    if (!frc) frc = boundary_prepare(S, v, rh.d != nullptr, true, bt);
     if (!frc) {
-        fa.bptr = bt.ptr; fa.blist = bt.list; fa.bel_elem = bt.bel_elem; fa.brhs = bt.rhs; fa.bmat = bt.mat;
+        fa.bptr = bt.ptr; fa.blist = bt.list; fa.bel_elem = bt.bel_elem; fa.bmat = bt.mat;
         frc = fill_launch(S, fa);
+        if (!frc && rh.d)
+            frc = rhs_launch(S, meas ? meas : M->geo, meas ? 1 : kGeoStride, fP0.d, fint, v->f_const, mask, gv.d, fa.tgv,
+                             rh.d, bt);
         boundary_release(S, bt);
     }
     dfree(ctx, fint);
@@ -891,6 +998,7 @@ static int numeric_pass(ffgpu_matrix *M, const ffgpu_varf *v, const ffgpu_bc *bc
     dfree(ctx, kloc);
     dfree(ctx, tloc);
     dfree(ctx, eloc);
+    dfree(ctx, meas);
     FFGPU_TRY(frc);
     FFGPU_TRY(check_device_status(ctx, "assembly"));
     FFGPU_TRY(rh.finish());
@@ -941,8 +1049,7 @@ int ffgpu_space_create(ffgpu_ctx *ctx, int dim, int nv, const double *coords, in
             dalloc(ctx, (void **)&S->elems, sizeof(int32_t) * nt * nvk) ||
             dalloc(ctx, (void **)&S->nodes, sizeof(int32_t) * m) ||
             dalloc(ctx, (void **)&S->inc_ptr, sizeof(int32_t) * (S->nnodes + 1)) ||
-            dalloc(ctx, (void **)&S->inc_elem, sizeof(int32_t) * m) ||
-            dalloc(ctx, (void **)&S->inc_loc, m) ||
+            dalloc(ctx, (void **)&S->inc, sizeof(int32_t) * m) ||
             dalloc(ctx, (void **)&cnt, sizeof(int32_t) * (S->nnodes + 1))) {
             set_error("ffgpu_space_create: device allocation failed");
             rc = FFGPU_ENOMEM; goto fail;
@@ -966,19 +1073,19 @@ int ffgpu_space_create(ffgpu_ctx *ctx, int dim, int nv, const double *coords, in
     if ((rc = device_max_i32(ctx, cnt, S->nnodes, &S->max_inc))) goto fail;
     if ((rc = device_scan_i32(ctx, cnt, S->inc_ptr, S->nnodes))) goto fail;
     cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (S->nnodes + 1), s);
-    inc_fill_kernel<<<grid_for(m, 256), 256, 0, s>>>(S->nodes, m, nn, S->inc_ptr, cnt, S->inc_elem, S->inc_loc);
+    inc_fill_kernel<<<grid_for(m, 256), 256, 0, s>>>(S->nodes, m, S->inc_ptr, cnt, S->inc);
     if ((rc = launch_check(ctx, "inc_fill"))) goto fail;
     {
         int P = 1;
         while (P < S->max_inc) P <<= 1;
-        size_t smem = (size_t)4 * P * sizeof(long long);
-        if (smem > 200 * 1024 || (int64_t)S->max_inc * nn > kCandMax) {
+        size_t smem = (size_t)4 * P * sizeof(int);
+        if (2 * smem > 200 * 1024 || (int64_t)S->max_inc * nn > kCandMax) {
             set_error("node valence %d too high (at most %d candidate neighbours)", S->max_inc, kCandMax);
             rc = FFGPU_EMESH; goto fail;
         }
         cudaFuncSetAttribute(inc_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         inc_sort_kernel<<<min(kNumSM * 8, max(1, (S->nnodes + 3) / 4)), 128, smem, s>>>(
-            S->inc_ptr, S->nnodes, S->max_inc, S->inc_elem, S->inc_loc);
+            S->inc_ptr, S->nnodes, S->max_inc, S->inc);
         if ((rc = launch_check(ctx, "inc_sort"))) goto fail;
     }
     dfree(ctx, cnt);
@@ -999,7 +1106,7 @@ int ffgpu_space_destroy(ffgpu_space *S) {
     if (!S) return FFGPU_OK;
     cudaStreamSynchronize(S->ctx->stream);
     dfree(S->ctx, S->coords); dfree(S->ctx, S->elems); dfree(S->ctx, S->nodes);
-    dfree(S->ctx, S->inc_ptr); dfree(S->ctx, S->inc_elem); dfree(S->ctx, S->inc_loc);
+    dfree(S->ctx, S->inc_ptr); dfree(S->ctx, S->inc);
     dfree(S->ctx, S->belems); dfree(S->ctx, S->blabel); dfree(S->ctx, S->bv_ptr); dfree(S->ctx, S->bv_elem); dfree(S->ctx, S->vmark);
     dfree(S->ctx, S->bel_elem); dfree(S->ctx, S->bel_face);
     delete S;
@@ -1075,17 +1182,18 @@ int ffgpu_matrix_assemble(ffgpu_space *S, const ffgpu_varf *v, const ffgpu_bc *b
     M->ctx = ctx; M->space = S; M->bs = S->bs; M->nb = S->nnodes; M->n = S->ndof;
     M->ntgv = -1; M->csr_lanes = 0;
     int rc = FFGPU_OK;
-    int32_t *deg = nullptr;
+    int32_t *deg = nullptr, *tmpcol = nullptr, *drank = nullptr;
+    const size_t cand = (size_t)S->nt * S->nn * S->nn;   // nodes of all incidences
     if (dalloc(ctx, (void **)&M->browptr, sizeof(int32_t) * (M->nb + 1)) ||
         dalloc(ctx, (void **)&deg, sizeof(int32_t) * (M->nb + 1)) ||
-        dalloc(ctx, (void **)&M->geo, sizeof(double) * kGeoStride * S->nt)) {
+        dalloc(ctx, (void **)&drank, sizeof(int32_t) * M->nb) ||
+        dalloc(ctx, (void **)&tmpcol, sizeof(int32_t) * cand) ||
+        dalloc(ctx, (void **)&M->rmap, sizeof(uint16_t) * cand)) {
         set_error("ffgpu_matrix_assemble: device allocation failed");
         rc = FFGPU_ENOMEM; goto fail;
     }
-    // symbolic: row degrees, row pointer
-    row_count_kernel<<<min(kNumSM * 16, max(1, (M->nb + 3) / 4)), 128, 0, s>>>(
-        M->nb, S->inc_ptr, S->inc_elem, S->nodes, S->nn, deg, ctx->d_status);
-    if ((rc = launch_check(ctx, "row_count"))) goto fail;
+    // symbolic: the rows' columns and degrees, row pointer
+    if ((rc = pattern_launch(S, deg, tmpcol, M->rmap, drank))) goto fail;
     if ((rc = check_device_status(ctx, "pattern"))) goto fail;
     if ((rc = device_max_i32(ctx, deg, M->nb, &M->max_deg))) goto fail;
     if ((rc = device_scan_i32(ctx, deg, M->browptr, M->nb))) goto fail;
@@ -1110,11 +1218,15 @@ int ffgpu_matrix_assemble(ffgpu_space *S, const ffgpu_varf *v, const ffgpu_bc *b
         set_error("ffgpu_matrix_assemble: allocation of %lld values failed", (long long)M->nnz);
         rc = FFGPU_ENOMEM; goto fail;
     }
-    if ((rc = numeric_pass(M, v, bc, rhs, true))) goto fail;
+    if ((rc = numeric_pass(M, v, bc, rhs, tmpcol, drank))) goto fail;
+    dfree(ctx, tmpcol);
+    dfree(ctx, drank);
     *out = M;
     return FFGPU_OK;
 fail:
-    if (deg) dfree(ctx, deg);
+    dfree(ctx, deg);
+    dfree(ctx, tmpcol);
+    dfree(ctx, drank);
     ffgpu_matrix_destroy(M);
     return rc;
 }
@@ -1122,7 +1234,7 @@ fail:
 int ffgpu_matrix_reassemble(ffgpu_matrix *M, const ffgpu_varf *v, const ffgpu_bc *bc, double *rhs) {
     FFGPU_CHECK(M && M->space, FFGPU_EINVAL, "ffgpu_matrix_reassemble: matrix has no FE space");
     FFGPU_CUDA(cudaSetDevice(M->ctx->device));
-    return numeric_pass(M, v, bc, rhs, false);
+    return numeric_pass(M, v, bc, rhs, nullptr, nullptr);
 }
 
 int ffgpu_rhs_assemble(ffgpu_space *S, const ffgpu_varf *v, const ffgpu_bc *bc, double *rhs) {
@@ -1131,9 +1243,11 @@ int ffgpu_rhs_assemble(ffgpu_space *S, const ffgpu_varf *v, const ffgpu_bc *bc, 
     ffgpu_ctx *ctx = S->ctx;
     cudaStream_t s = ctx->stream;
     FFGPU_CUDA(cudaSetDevice(ctx->device));
+    // P1 with a source per element needs the measures only
+    const bool full = S->fe != FFGPU_FE_P1 || v->f_qp || v->f_expr;
     double *geo = nullptr;
-    FFGPU_CUDA(dalloc(ctx, (void **)&geo, sizeof(double) * kGeoStride * S->nt));
-    int rc = run_geometry(S, v, geo);
+    FFGPU_CUDA(dalloc(ctx, (void **)&geo, sizeof(double) * (full ? kGeoStride : 1) * S->nt));
+    int rc = full ? run_geometry(S, v, geo) : p1_elem_launch(S, nullptr, 0.0, 0.0, nullptr, geo);
     {
         DevIn<double> fP0(v->f, v->f ? (size_t)S->nt * S->bs : 0, ctx);
         DevIn<uint8_t> onbc(bc ? bc->onbc : nullptr, bc && bc->onbc ? S->ndof : 0, ctx);
@@ -1151,21 +1265,8 @@ int ffgpu_rhs_assemble(ffgpu_space *S, const ffgpu_varf *v, const ffgpu_bc *bc, 
         double *fint = nullptr;
         if (!rc) rc = source_prepare(S, v, geo, &fint);
         if (!rc) rc = boundary_prepare(S, v, true, false, bt);
-        if (!rc) {
-            void (*k)(int, const int32_t *, const int32_t *, const uint8_t *, const double *,
-                      const double *, const double *, double, double, double, const uint8_t *,
-                      const double *, double, double *, const int32_t *, const int32_t *,
-                      const double *) = nullptr;
-            if (S->dim == 2 && S->fe == FFGPU_FE_P1) k = rhs_kernel<2, 1>;
-            if (S->dim == 3 && S->fe == FFGPU_FE_P1) k = rhs_kernel<3, 1>;
-            if (S->dim == 2 && S->fe == FFGPU_FE_P2) k = rhs_kernel<2, 2>;
-            if (S->dim == 3 && S->fe == FFGPU_FE_P2) k = rhs_kernel<3, 2>;
-            if (S->dim == 3 && S->fe == FFGPU_FE_P2VEC3) k = rhs_kernel<3, 3>;
-            k<<<grid_for((int64_t)S->ndof, 256), 256, 0, s>>>(
-                S->nnodes, S->inc_ptr, S->inc_elem, S->inc_loc, geo, fP0.d, fint, v->f_const[0],
-                v->f_const[1], v->f_const[2], mask, gv.d, bc ? bc->tgv : 0.0, rh.d, bt.ptr, bt.list, bt.rhs);
-            rc = launch_check(ctx, "rhs_kernel");
-        }
+        if (!rc)
+            rc = rhs_launch(S, geo, full ? kGeoStride : 1, fP0.d, fint, v->f_const, mask, gv.d, bc ? bc->tgv : 0.0, rh.d, bt);
         boundary_release(S, bt);
         dfree(ctx, fint);
         if (!rc) rc = rh.finish();
@@ -1229,7 +1330,7 @@ int ffgpu_matrix_destroy(ffgpu_matrix *M) {
     if (M->cg_exec) cudaGraphExecDestroy(M->cg_exec);
     direct_release(M);
     dfree(M->ctx, M->browptr); dfree(M->ctx, M->bcol); dfree(M->ctx, M->diagpos); dfree(M->ctx, M->rowperm); dfree(M->ctx, M->val);
-    dfree(M->ctx, M->geo); dfree(M->ctx, M->bcmask);
+    dfree(M->ctx, M->geo); dfree(M->ctx, M->bcmask); dfree(M->ctx, M->rmap);
     dfree(M->ctx, M->diag_inv); dfree(M->ctx, M->wcl); dfree(M->ctx, M->vec); dfree(M->ctx, M->val_t);
     dfree(M->ctx, M->val32); dfree(M->ctx, M->valx); dfree(M->ctx, M->valx_t); dfree(M->ctx, M->hx); dfree(M->ctx, M->ks);
     sell_release(M);

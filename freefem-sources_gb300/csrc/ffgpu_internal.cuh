@@ -101,8 +101,7 @@ struct ffgpu_space {
     int32_t *elems;      // nt*nvk
     int32_t *nodes;      // nt*nn  (scalar node of each local basis function)
     int32_t *inc_ptr;    // nnodes+1
-    int32_t *inc_elem;   // node -> incident elements, ascending
-    uint8_t *inc_loc;    // local index of the node in that element
+    int32_t *inc;        // node -> its slots e * nn + local index in the node table, ascending
     int max_inc;
     // boundary elements (for on(labels)): nbe x dim vertices, labels, vertex -> element CSR
     int nbe;
@@ -123,7 +122,8 @@ struct ffgpu_matrix {
     int32_t *diagpos;     // nb: index of the diagonal block of each block row
     int32_t *rowperm;     // nb: block rows by decreasing degree (stable), the SpMV's row order
     double *val;          // nnzb*bs*bs, each block row-major
-    double *geo;          // per-element geometry cache (16 doubles per element)
+    double *geo;          // per-element geometry (16 doubles per element), NULL until needed on P1
+    uint16_t *rmap;       // rank in its row of every node of every incidence (assembled matrices)
     uint8_t *bcmask;      // on(labels) DOF mask computed on the device (ndof)
     // solver state (lazily allocated)
     double *diag_inv;     // Jacobi 1/A_ii (1 if tiny)
@@ -318,6 +318,8 @@ int resident_grid(const void *kernel, int threads, size_t smem = 0);
 // shorter cross-block reduction
 int sized_grid(const void *kernel, int threads, int64_t need, size_t smem = 0);
 
+// the element geometry of an assembled matrix in A->geo (ffgpu_assembly.cu)
+int matrix_geometry(ffgpu_matrix *M, const ffgpu_varf *v);
 // matrix-level operations shared by the solvers
 int matrix_prepare_solver(ffgpu_matrix *A);
 int matrix_prepare_transpose(ffgpu_matrix *A);
