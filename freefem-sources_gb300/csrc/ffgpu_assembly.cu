@@ -27,29 +27,6 @@
 namespace ffgpu {
 
 // ------------------------------------------------------------------ small device utils
-template <typename T>
-__device__ void warp_bitonic_sort(T *s, int P) {
-    const int lane = threadIdx.x & 31;
-    for (int k = 2; k <= P; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = lane; i < P; i += 32) {
-                int ixj = i ^ j;
-                if (ixj > i) {
-                    bool up = (i & k) == 0;
-                    T a = s[i], b = s[ixj];
-                    if ((a > b) == up) { s[i] = b; s[ixj] = a; }
-                }
-            }
-            __syncwarp();
-        }
-}
-
-__device__ __forceinline__ int pow2_ceil(int x) {
-    int p = 1;
-    while (p < x) p <<= 1;
-    return p;
-}
-
 // binary search of v in the sorted list s[0..n)
 __device__ __forceinline__ int find_sorted(const int *s, int n, int v) {
     int lo = 0, hi = n - 1;
@@ -79,36 +56,55 @@ __global__ void build_nodes_kernel(const int32_t *dof, int nt, int ndofK, int nn
     nodes[t] = node;
 }
 
+// four numbers per thread, in one load where the array (a caller's, maybe) is aligned for it
 __global__ void check_elems_kernel(const int32_t *elems, int64_t m, int nv, int *status) {
-    int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t < m && (elems[t] < 0 || elems[t] >= nv)) dev_fail(status, kDevBadIndex);
+    const int64_t t = 4 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
+    bool bad = false;
+    if (t + 4 <= m && (reinterpret_cast<uintptr_t>(elems) & 15) == 0) {
+        const int4 v = *reinterpret_cast<const int4 *>(elems + t);
+        bad = min(min(v.x, v.y), min(v.z, v.w)) < 0 || max(max(v.x, v.y), max(v.z, v.w)) >= nv;
+    } else {
+        for (int64_t i = t; i < m && i < t + 4; ++i) bad |= elems[i] < 0 || elems[i] >= nv;
+    }
+    if (bad) dev_fail(status, kDevBadIndex);
 }
 
-__global__ void inc_count_kernel(const int32_t *nodes, int64_t m, int32_t *cnt) {
+// incidences per node, and the arrival number of each slot at its node: the fill needs no atomics
+__global__ void inc_count_kernel(const int32_t *nodes, int64_t m, int32_t *cnt, uint16_t *at) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t < m) atomicAdd(&cnt[nodes[t]], 1);
+    if (t < m) at[t] = (uint16_t)min(atomicAdd(&cnt[nodes[t]], 1), 65535);
 }
 
-__global__ void inc_fill_kernel(const int32_t *nodes, int64_t m, const int32_t *ptr, int32_t *cursor, int32_t *inc) {
+__global__ void inc_fill_kernel(const int32_t *nodes, int64_t m, const int32_t *ptr, const uint16_t *at, int32_t *inc) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= m) return;
-    int a = nodes[t];
-    inc[ptr[a] + atomicAdd(&cursor[a], 1)] = (int32_t)t;
+    if (t < m) inc[ptr[nodes[t]] + at[t]] = (int32_t)t;
 }
 
-// sort each node's incidence list by slot, i.e. by element number (the reference's element order)
-__global__ void inc_sort_kernel(const int32_t *ptr, int nnodes, int max_inc, int32_t *inc) {
-    extern __shared__ int sh_inc[];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int P = pow2_ceil(max_inc);
-    int *s = sh_inc + (int64_t)w * P;
-    for (int a = blockIdx.x * (blockDim.x >> 5) + w; a < nnodes; a += gridDim.x * (blockDim.x >> 5)) {
-        int b = ptr[a], e = ptr[a + 1], n = e - b;
-        for (int i = lane; i < P; i += 32) s[i] = i < n ? inc[b + i] : 0x7fffffff;
-        __syncwarp();
-        warp_bitonic_sort(s, P);
-        for (int i = lane; i < n; i += 32) inc[b + i] = s[i];
-        __syncwarp();
+// Each node's incidence list by slot, i.e. by element number (the reference's element order): the
+// place of a slot is the number of smaller ones.  G lanes per node (8 up to 8 slots a node on
+// average, as 2D meshes have, else 32); lists longer than G lanes hold are counted from memory.  (A bitonic sort by
+// a warp per node of the longest list's length: 632 us for the 21 M slots of 96^3 cells; this, 158 us.)
+template <int G>
+__global__ void __launch_bounds__(256) inc_sort_kernel(const int32_t *__restrict__ ptr, int nnodes,
+                                                       const int32_t *__restrict__ in, int32_t *__restrict__ inc) {
+    const int sub = threadIdx.x & (G - 1);
+    const unsigned mask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
+    const int64_t per = (int64_t)gridDim.x * (blockDim.x / G);
+    for (int64_t a = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G; a < nnodes; a += per) {
+        const int b = ptr[a], n = ptr[a + 1] - b;
+        if (n <= G) {
+            const int key = sub < n ? in[b + sub] : 0x7fffffff;
+            int r = 0;
+            for (int k = 0; k < n; ++k) r += __shfl_sync(mask, key, k, G) < key;
+            if (sub < n) inc[b + r] = key;
+        } else {
+            for (int i = sub; i < n; i += G) {
+                const int key = in[b + i];
+                int r = 0;
+                for (int k = 0; k < n; ++k) r += in[b + k] < key;
+                inc[b + r] = key;
+            }
+        }
     }
 }
 
@@ -503,8 +499,8 @@ static int neg_tgv_bits(double tgv) {
 // The form this replaces gave the row one copy per concurrent element and summed the copies:
 // 21 warp adds per P1 row in 3D instead of 3.  PLAIN: the element matrices are complete (kloc or
 // eloc and nothing to add); the general form keeps its tests out of that loop.  On 96^3 cells (912 673 rows, 13.4 M entries), the
-// products moved to p1_elem_kernel (0.76 ms): 3.27 -> 0.30 ms; 16 % of the old form's time was FP64
-// compares with constants, which cost as much as an add and are now made on the host.
+// products moved to p1_elem_kernel (0.76 ms): 3.27 -> 0.30 ms.  (With the tests on tgv and c_mass
+// as FP64 compares in the loops it took 1.6 ms: a compare costs as much as an add.)
 template <int DIM, int FE, bool PLAIN>
 __global__ void __launch_bounds__(256) fill_kernel(FillArgs A) {
     constexpr int nvk = DIM + 1;
@@ -685,21 +681,27 @@ __global__ void rhs_kernel(int nnodes, const int32_t *inc_ptr, const int32_t *in
 }
 
 // ------------------------------------------------------------------ CSR export
-__global__ void export_csr_kernel(int nb, int bs, const int32_t *browptr, const int32_t *bcol,
-                                  const double *val, int32_t *rowptr, int32_t *col, double *out) {
-    int a = blockIdx.x * blockDim.x + threadIdx.x;
+// [P2]^3 blocks to scalar rows: a warp per block row, lanes along each scalar row (a scalar
+// matrix is stored as the CSR it exports, ffgpu_matrix_csr copies it).  A thread per block row,
+// its writes scattered over the warp's rows, took 567 us for 24.7 M entries; this, 104 us.
+__global__ void __launch_bounds__(256) export_bsr3_kernel(int nb, const int32_t *__restrict__ browptr,
+                                                          const int32_t *__restrict__ bcol, const double *__restrict__ val,
+                                                          int32_t *__restrict__ rowptr, int32_t *__restrict__ col,
+                                                          double *__restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t a = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (a >= nb) return;
-    int64_t b0 = browptr[a], deg = browptr[a + 1] - b0;
-    for (int c = 0; c < bs; ++c) {
-        int64_t r0 = b0 * bs * bs + c * bs * deg;
-        rowptr[(int64_t)a * bs + c] = (int32_t)r0;
-        for (int64_t k = 0; k < deg; ++k)
-            for (int cp = 0; cp < bs; ++cp) {
-                col[r0 + k * bs + cp] = bs * bcol[b0 + k] + cp;
-                out[r0 + k * bs + cp] = val[(b0 + k) * bs * bs + c * bs + cp];
-            }
+    const int64_t b0 = browptr[a], deg = browptr[a + 1] - b0;
+    if (lane < 3) rowptr[3 * a + lane] = (int32_t)(9 * b0 + 3 * lane * deg);
+    if (lane == 3 && a == nb - 1) rowptr[3 * (int64_t)nb] = (int32_t)(9 * (int64_t)browptr[nb]);
+    for (int c = 0; c < 3; ++c) {
+        const int64_t r0 = 9 * b0 + 3 * c * deg;
+        for (int64_t q = lane; q < 3 * deg; q += 32) {
+            const int64_t k = q / 3, cp = q - 3 * k;
+            col[r0 + q] = 3 * bcol[b0 + k] + (int)cp;
+            out[r0 + q] = val[(b0 + k) * 9 + 3 * c + cp];
+        }
     }
-    if (a == nb - 1) rowptr[(int64_t)nb * bs] = (int32_t)((int64_t)browptr[nb] * bs * bs);
 }
 
 // ------------------------------------------------------------------ on(labels): DOF marking
@@ -723,6 +725,15 @@ __global__ void bmark_vertices_kernel(int nbe, int bdim, const int32_t *belems, 
 __device__ __forceinline__ void mark_node(uint8_t *onbc, int node, int bs, int comp_mask) {
     for (int c = 0; c < bs; ++c)
         if (comp_mask == 0 || (comp_mask >> c) & 1) onbc[(int64_t)node * bs + c] = 1;
+}
+
+// P1 without a DOF table: the nodes are the vertices (the same mask from the boundary elements
+// alone; onbc is zero before)
+__global__ void bmark_p1_kernel(int nbe, int bdim, const int32_t *belems, const int32_t *blabel, int nlabels,
+                                const int32_t *labels, uint8_t *onbc) {
+    int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= nbe || !label_selected(blabel[b], nlabels, labels)) return;
+    for (int k = 0; k < bdim; ++k) onbc[belems[(int64_t)b * bdim + k]] = 1;
 }
 
 template <int DIM>
@@ -794,8 +805,12 @@ int space_bc_mask_device(ffgpu_space *S, int nlabels, const int32_t *labels, int
     cudaStream_t s = ctx->stream;
     DevIn<int32_t> lab(labels, nlabels, ctx);
     FFGPU_TRY(lab.err);
-    FFGPU_CUDA(cudaMemsetAsync(S->vmark, 0, S->nv, s));
     FFGPU_CUDA(cudaMemsetAsync(onbc, 0, S->ndof, s));
+    if (S->nodes == S->elems && !(comp_mask && !(comp_mask & 1))) {
+        bmark_p1_kernel<<<grid_for(S->nbe, 256), 256, 0, s>>>(S->nbe, S->dim, S->belems, S->blabel, nlabels, lab.d, onbc);
+        return launch_check(ctx, "bmark_p1");
+    }
+    FFGPU_CUDA(cudaMemsetAsync(S->vmark, 0, S->nv, s));
     bmark_vertices_kernel<<<grid_for(S->nbe, 256), 256, 0, s>>>(S->nbe, S->dim, S->belems, S->blabel, nlabels,
                                                                  lab.d, S->vmark);
     FFGPU_TRY(launch_check(ctx, "bmark_vertices"));
@@ -1041,53 +1056,64 @@ int ffgpu_space_create(ffgpu_ctx *ctx, int dim, int nv, const double *coords, in
     S->bs = bs; S->ndofK = ndofK; S->ndof = ndof; S->nnodes = ndof / bs;
     int64_t m = (int64_t)nt * nn;
     int rc = FFGPU_OK;
-    int32_t *cnt = nullptr;
+    int32_t *cnt = nullptr, *unsorted = nullptr;
+    uint16_t *at = nullptr;
     {
         DevIn<int32_t> D(dof, dof ? (size_t)nt * ndofK : 0, ctx);   // NULL (P1): the vertices
         if (D.err) { rc = D.err; goto fail; }
         if (dalloc(ctx, (void **)&S->coords, sizeof(double) * nv * dim) ||
             dalloc(ctx, (void **)&S->elems, sizeof(int32_t) * nt * nvk) ||
-            dalloc(ctx, (void **)&S->nodes, sizeof(int32_t) * m) ||
+            (dof && dalloc(ctx, (void **)&S->nodes, sizeof(int32_t) * m)) ||
             dalloc(ctx, (void **)&S->inc_ptr, sizeof(int32_t) * (S->nnodes + 1)) ||
             dalloc(ctx, (void **)&S->inc, sizeof(int32_t) * m) ||
-            dalloc(ctx, (void **)&cnt, sizeof(int32_t) * (S->nnodes + 1))) {
+            dalloc(ctx, (void **)&cnt, sizeof(int32_t) * (S->nnodes + 1)) ||
+            dalloc(ctx, (void **)&at, sizeof(uint16_t) * m) || dalloc(ctx, (void **)&unsorted, sizeof(int32_t) * m)) {
             set_error("ffgpu_space_create: device allocation failed");
             rc = FFGPU_ENOMEM; goto fail;
         }
+        if (!dof) S->nodes = S->elems;   // P1 without a table: the nodes are the vertices
         // host or device arrays, copied straight into the space's own buffers
         if (cudaMemcpyAsync(S->coords, coords, sizeof(double) * nv * dim, cudaMemcpyDefault, s) ||
             cudaMemcpyAsync(S->elems, elems, sizeof(int32_t) * nt * nvk, cudaMemcpyDefault, s)) {
             set_error("ffgpu_space_create: copy of the mesh failed");
             rc = FFGPU_ECUDA; goto fail;
         }
-        check_elems_kernel<<<grid_for((int64_t)nt * nvk, 256), 256, 0, s>>>(S->elems, (int64_t)nt * nvk, nv, ctx->d_status);
+        check_elems_kernel<<<grid_for(((int64_t)nt * nvk + 3) / 4, 256), 256, 0, s>>>(S->elems, (int64_t)nt * nvk, nv,
+                                                                                       ctx->d_status);
         if ((rc = launch_check(ctx, "check_elems"))) goto fail;
-        build_nodes_kernel<<<grid_for(m, 256), 256, 0, s>>>(dof ? D.d : S->elems, nt, ndofK, nn, bs, ndof,
-                                                            S->nodes, ctx->d_status);
-        if ((rc = launch_check(ctx, "build_nodes"))) goto fail;
+        if (dof) {
+            build_nodes_kernel<<<grid_for(m, 256), 256, 0, s>>>(D.d, nt, ndofK, nn, bs, ndof, S->nodes, ctx->d_status);
+            if ((rc = launch_check(ctx, "build_nodes"))) goto fail;
+        }
         if ((rc = check_device_status(ctx, "ffgpu_space_create"))) goto fail;
     }
     cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (S->nnodes + 1), s);
-    inc_count_kernel<<<grid_for(m, 256), 256, 0, s>>>(S->nodes, m, cnt);
+    inc_count_kernel<<<grid_for(m, 256), 256, 0, s>>>(S->nodes, m, cnt, at);
     if ((rc = launch_check(ctx, "inc_count"))) goto fail;
     if ((rc = device_max_i32(ctx, cnt, S->nnodes, &S->max_inc))) goto fail;
-    if ((rc = device_scan_i32(ctx, cnt, S->inc_ptr, S->nnodes))) goto fail;
-    cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (S->nnodes + 1), s);
-    inc_fill_kernel<<<grid_for(m, 256), 256, 0, s>>>(S->nodes, m, S->inc_ptr, cnt, S->inc);
-    if ((rc = launch_check(ctx, "inc_fill"))) goto fail;
     {
+        // the bounds of the pattern pass (which also keep the arrival numbers in 16 bits)
         int P = 1;
         while (P < S->max_inc) P <<= 1;
-        size_t smem = (size_t)4 * P * sizeof(int);
-        if (2 * smem > 200 * 1024 || (int64_t)S->max_inc * nn > kCandMax) {
+        if ((size_t)4 * P * sizeof(long long) > 200 * 1024 || (int64_t)S->max_inc * nn > kCandMax) {
             set_error("node valence %d too high (at most %d candidate neighbours)", S->max_inc, kCandMax);
             rc = FFGPU_EMESH; goto fail;
         }
-        cudaFuncSetAttribute(inc_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        inc_sort_kernel<<<min(kNumSM * 8, max(1, (S->nnodes + 3) / 4)), 128, smem, s>>>(
-            S->inc_ptr, S->nnodes, S->max_inc, S->inc);
-        if ((rc = launch_check(ctx, "inc_sort"))) goto fail;
     }
+    if ((rc = device_scan_i32(ctx, cnt, S->inc_ptr, S->nnodes))) goto fail;
+    inc_fill_kernel<<<grid_for(m, 256), 256, 0, s>>>(S->nodes, m, S->inc_ptr, at, unsorted);
+    if ((rc = launch_check(ctx, "inc_fill"))) goto fail;
+    if (m <= (int64_t)8 * S->nnodes)
+        inc_sort_kernel<8><<<min(kNumSM * 64, grid_for((int64_t)S->nnodes * 8, 256)), 256, 0, s>>>(S->inc_ptr, S->nnodes,
+                                                                                                    unsorted, S->inc);
+    else
+        inc_sort_kernel<32><<<min(kNumSM * 64, grid_for((int64_t)S->nnodes * 32, 256)), 256, 0, s>>>(S->inc_ptr, S->nnodes,
+                                                                                                      unsorted, S->inc);
+    if ((rc = launch_check(ctx, "inc_sort"))) goto fail;
+    dfree(ctx, at);
+    dfree(ctx, unsorted);
+    at = nullptr;
+    unsorted = nullptr;
     dfree(ctx, cnt);
     cnt = nullptr;
     if (cudaStreamSynchronize(s) != cudaSuccess) {
@@ -1097,7 +1123,9 @@ int ffgpu_space_create(ffgpu_ctx *ctx, int dim, int nv, const double *coords, in
     *out = S;
     return FFGPU_OK;
 fail:
-    if (cnt) dfree(ctx, cnt);
+    dfree(ctx, cnt);
+    dfree(ctx, at);
+    dfree(ctx, unsorted);
     ffgpu_space_destroy(S);
     return rc;
 }
@@ -1105,7 +1133,9 @@ fail:
 int ffgpu_space_destroy(ffgpu_space *S) {
     if (!S) return FFGPU_OK;
     cudaStreamSynchronize(S->ctx->stream);
-    dfree(S->ctx, S->coords); dfree(S->ctx, S->elems); dfree(S->ctx, S->nodes);
+    dfree(S->ctx, S->coords);
+    if (S->nodes != S->elems) dfree(S->ctx, S->nodes);
+    dfree(S->ctx, S->elems);
     dfree(S->ctx, S->inc_ptr); dfree(S->ctx, S->inc);
     dfree(S->ctx, S->belems); dfree(S->ctx, S->blabel); dfree(S->ctx, S->bv_ptr); dfree(S->ctx, S->bv_elem); dfree(S->ctx, S->vmark);
     dfree(S->ctx, S->bel_elem); dfree(S->ctx, S->bel_face);
@@ -1137,8 +1167,8 @@ int ffgpu_space_set_boundary(ffgpu_space *S, int nbe, const int32_t *belems, con
     }
     FFGPU_CUDA(cudaMemcpyAsync(S->belems, belems, sizeof(int32_t) * nbe * bdim, cudaMemcpyDefault, s));
     FFGPU_CUDA(cudaMemcpyAsync(S->blabel, blabel, sizeof(int32_t) * nbe, cudaMemcpyDefault, s));
-    check_elems_kernel<<<grid_for((int64_t)nbe * bdim, 256), 256, 0, s>>>(S->belems, (int64_t)nbe * bdim, S->nv,
-                                                                           ctx->d_status);
+    check_elems_kernel<<<grid_for(((int64_t)nbe * bdim + 3) / 4, 256), 256, 0, s>>>(S->belems, (int64_t)nbe * bdim, S->nv,
+                                                                                     ctx->d_status);
     FFGPU_TRY(launch_check(ctx, "check_belems"));
     int rc = check_device_status(ctx, "ffgpu_space_set_boundary");
     if (!rc) {
@@ -1351,13 +1381,21 @@ int ffgpu_matrix_csr(const ffgpu_matrix *M, int32_t *rowptr, int32_t *col, doubl
     ffgpu_ctx *ctx = M->ctx;
     cudaStream_t s = ctx->stream;
     FFGPU_CUDA(cudaSetDevice(ctx->device));
+    if (M->bs == 1) {
+        // stored as exported: copied to the caller's arrays, host or device
+        FFGPU_CUDA(cudaMemcpyAsync(rowptr, M->browptr, sizeof(int32_t) * ((size_t)M->n + 1), cudaMemcpyDefault, s));
+        FFGPU_CUDA(cudaMemcpyAsync(col, M->bcol, sizeof(int32_t) * M->nnz, cudaMemcpyDefault, s));
+        FFGPU_CUDA(cudaMemcpyAsync(val, M->val, sizeof(double) * M->nnz, cudaMemcpyDefault, s));
+        FFGPU_CUDA(cudaStreamSynchronize(s));
+        return FFGPU_OK;
+    }
     DevOut<int32_t> rp(rowptr, M->n + 1, ctx, false);
     DevOut<int32_t> cl(col, M->nnz, ctx, false);
     DevOut<double> vl(val, M->nnz, ctx, false);
     FFGPU_TRY(rp.err); FFGPU_TRY(cl.err); FFGPU_TRY(vl.err);
-    export_csr_kernel<<<grid_for(M->nb, 128), 128, 0, s>>>(M->nb, M->bs, M->browptr, M->bcol, M->val,
-                                                            rp.d, cl.d, vl.d);
-    FFGPU_TRY(launch_check(ctx, "export_csr"));
+    export_bsr3_kernel<<<grid_for((int64_t)M->nb * 32, 256), 256, 0, s>>>(M->nb, M->browptr, M->bcol, M->val, rp.d, cl.d,
+                                                                       vl.d);
+    FFGPU_TRY(launch_check(ctx, "export_bsr3"));
     FFGPU_TRY(rp.finish()); FFGPU_TRY(cl.finish()); FFGPU_TRY(vl.finish());
     FFGPU_CUDA(cudaStreamSynchronize(s));
     return FFGPU_OK;

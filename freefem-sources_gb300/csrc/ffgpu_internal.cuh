@@ -99,7 +99,7 @@ struct ffgpu_space {
     int dim, nvk, nv, nt, fe, nn, bs, ndofK, ndof, nnodes;
     double *coords;      // nv*dim
     int32_t *elems;      // nt*nvk
-    int32_t *nodes;      // nt*nn  (scalar node of each local basis function)
+    int32_t *nodes;      // nt*nn  (scalar node of each local basis function; P1 without a table: elems)
     int32_t *inc_ptr;    // nnodes+1
     int32_t *inc;        // node -> its slots e * nn + local index in the node table, ascending
     int max_inc;

@@ -281,7 +281,7 @@ int ffgpu_number_p2(ffgpu_ctx *ctx, int nv, int nt, const int32_t *elems, int32_
     }
     // element vertex indices are checked first: every incidence index below depends on them
     if (!rc) {
-        check_elems_kernel<<<grid_n(n4, 256), 256, 0, s>>>(E.d, n4, nv, ctx->d_status);
+        check_elems_kernel<<<grid_n((n4 + 3) / 4, 256), 256, 0, s>>>(E.d, n4, nv, ctx->d_status);
         rc = launch_check(ctx, "check_elems");
         if (!rc) rc = check_device_status(ctx, "ffgpu_number_p2");
     }
