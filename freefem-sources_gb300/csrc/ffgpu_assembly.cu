@@ -70,9 +70,10 @@ __global__ void check_elems_kernel(const int32_t *elems, int64_t m, int nv, int 
 }
 
 // incidences per node, and the arrival number of each slot at its node: the fill needs no atomics
-__global__ void inc_count_kernel(const int32_t *nodes, int64_t m, int32_t *cnt, uint16_t *at) {
+// (a node number out of range is skipped here: the status word, read with the counts, has it)
+__global__ void inc_count_kernel(const int32_t *nodes, int64_t m, int nnodes, int32_t *cnt, uint16_t *at) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t < m) at[t] = (uint16_t)min(atomicAdd(&cnt[nodes[t]], 1), 65535);
+    if (t < m && (unsigned)nodes[t] < (unsigned)nnodes) at[t] = (uint16_t)min(atomicAdd(&cnt[nodes[t]], 1), 65535);
 }
 
 __global__ void inc_fill_kernel(const int32_t *nodes, int64_t m, const int32_t *ptr, const uint16_t *at, int32_t *inc) {
@@ -681,6 +682,20 @@ __global__ void rhs_kernel(int nnodes, const int32_t *inc_ptr, const int32_t *in
 }
 
 // ------------------------------------------------------------------ CSR export
+// a scalar matrix is stored as the CSR it exports: one launch for the three arrays
+__global__ void __launch_bounds__(256) copy_csr_kernel(int nr, int64_t nnz, const int32_t *__restrict__ rp,
+                                                       const int32_t *__restrict__ cl, const double *__restrict__ vl,
+                                                       int32_t *__restrict__ orp, int32_t *__restrict__ ocl,
+                                                       double *__restrict__ ovl) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x, t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    for (int64_t t = t0; t < nr; t += step) orp[t] = rp[t];
+#pragma unroll 4
+    for (int64_t t = t0; t < nnz; t += step) {
+        ocl[t] = cl[t];
+        ovl[t] = __ldcs(vl + t);
+    }
+}
+
 // [P2]^3 blocks to scalar rows: a warp per block row, lanes along each scalar row (a scalar
 // matrix is stored as the CSR it exports, ffgpu_matrix_csr copies it).  A thread per block row,
 // its writes scattered over the warp's rows, took 567 us for 24.7 M entries; this, 104 us.
@@ -764,16 +779,18 @@ __global__ void bmark_nodes_kernel(int nt, int nn, const int32_t *elems, const i
     }
 }
 
-__global__ void bcount_kernel(int nbe, int bdim, const int32_t *belems, int32_t *cnt) {
+// (vertex numbers out of range are skipped; the status word has them)
+__global__ void bcount_kernel(int nbe, int bdim, int nv, const int32_t *belems, int32_t *cnt) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t < (int64_t)nbe * bdim) atomicAdd(&cnt[belems[t]], 1);
+    if (t < (int64_t)nbe * bdim && (unsigned)belems[t] < (unsigned)nv) atomicAdd(&cnt[belems[t]], 1);
 }
 
-__global__ void bfill_kernel(int nbe, int bdim, const int32_t *belems, const int32_t *ptr, int32_t *cursor,
+__global__ void bfill_kernel(int nbe, int bdim, int nv, const int32_t *belems, const int32_t *ptr, int32_t *cursor,
                              int32_t *out) {
     int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= (int64_t)nbe * bdim) return;
     int v = belems[t];
+    if ((unsigned)v >= (unsigned)nv) return;
     out[ptr[v] + atomicAdd(&cursor[v], 1)] = (int32_t)(t / bdim);
 }
 
@@ -1085,12 +1102,11 @@ int ffgpu_space_create(ffgpu_ctx *ctx, int dim, int nv, const double *coords, in
             build_nodes_kernel<<<grid_for(m, 256), 256, 0, s>>>(D.d, nt, ndofK, nn, bs, ndof, S->nodes, ctx->d_status);
             if ((rc = launch_check(ctx, "build_nodes"))) goto fail;
         }
-        if ((rc = check_device_status(ctx, "ffgpu_space_create"))) goto fail;
     }
     cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (S->nnodes + 1), s);
-    inc_count_kernel<<<grid_for(m, 256), 256, 0, s>>>(S->nodes, m, cnt, at);
+    inc_count_kernel<<<grid_for(m, 256), 256, 0, s>>>(S->nodes, m, S->nnodes, cnt, at);
     if ((rc = launch_check(ctx, "inc_count"))) goto fail;
-    if ((rc = device_max_i32(ctx, cnt, S->nnodes, &S->max_inc))) goto fail;
+    if ((rc = device_max_status(ctx, cnt, S->nnodes, nullptr, "ffgpu_space_create", &S->max_inc, nullptr))) goto fail;
     {
         // the bounds of the pattern pass (which also keep the arrival numbers in 16 bits)
         int P = 1;
@@ -1170,19 +1186,17 @@ int ffgpu_space_set_boundary(ffgpu_space *S, int nbe, const int32_t *belems, con
     check_elems_kernel<<<grid_for(((int64_t)nbe * bdim + 3) / 4, 256), 256, 0, s>>>(S->belems, (int64_t)nbe * bdim, S->nv,
                                                                                      ctx->d_status);
     FFGPU_TRY(launch_check(ctx, "check_belems"));
-    int rc = check_device_status(ctx, "ffgpu_space_set_boundary");
-    if (!rc) {
-        cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (S->nv + 1), s);
-        bcount_kernel<<<grid_for((int64_t)nbe * bdim, 256), 256, 0, s>>>(nbe, bdim, S->belems, cnt);
-        rc = launch_check(ctx, "bcount");
-    }
+    cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (S->nv + 1), s);
+    bcount_kernel<<<grid_for((int64_t)nbe * bdim, 256), 256, 0, s>>>(nbe, bdim, S->nv, S->belems, cnt);
+    int rc = launch_check(ctx, "bcount");
     if (!rc) rc = device_scan_i32(ctx, cnt, S->bv_ptr, S->nv);
     if (!rc) {
         cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (S->nv + 1), s);
-        bfill_kernel<<<grid_for((int64_t)nbe * bdim, 256), 256, 0, s>>>(nbe, bdim, S->belems, S->bv_ptr, cnt,
+        bfill_kernel<<<grid_for((int64_t)nbe * bdim, 256), 256, 0, s>>>(nbe, bdim, S->nv, S->belems, S->bv_ptr, cnt,
                                                                          S->bv_elem);
         rc = launch_check(ctx, "bfill");
     }
+    if (!rc) rc = check_device_status(ctx, "ffgpu_space_set_boundary");
     dfree(ctx, cnt);
     if (!rc && cudaStreamSynchronize(s) != cudaSuccess) { set_error("ffgpu_space_set_boundary failed"); rc = FFGPU_ECUDA; }
     return rc;
@@ -1224,22 +1238,19 @@ int ffgpu_matrix_assemble(ffgpu_space *S, const ffgpu_varf *v, const ffgpu_bc *b
     }
     // symbolic: the rows' columns and degrees, row pointer
     if ((rc = pattern_launch(S, deg, tmpcol, M->rmap, drank))) goto fail;
-    if ((rc = check_device_status(ctx, "pattern"))) goto fail;
-    if ((rc = device_max_i32(ctx, deg, M->nb, &M->max_deg))) goto fail;
     if ((rc = device_scan_i32(ctx, deg, M->browptr, M->nb))) goto fail;
+    {
+        int32_t nnzb = 0;
+        if ((rc = device_max_status(ctx, deg, M->nb, M->browptr + M->nb, "pattern", &M->max_deg, &nnzb))) goto fail;
+        M->nnzb = nnzb;
+        M->nnz = M->nnzb * M->bs * M->bs;
+    }
     // SpMV row order: block rows grouped by degree so that the lanes of a warp share trip counts
     if (dalloc(ctx, (void **)&M->rowperm, sizeof(int32_t) * M->nb)) {
         set_error("ffgpu_matrix_assemble: device allocation failed");
         rc = FFGPU_ENOMEM; goto fail;
     }
     if ((rc = device_order_by_key_desc(ctx, deg, M->nb, M->max_deg, M->rowperm))) goto fail;
-    {
-        int32_t nnzb = 0;
-        cudaMemcpyAsync(&nnzb, M->browptr + M->nb, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-        cudaStreamSynchronize(s);
-        M->nnzb = nnzb;
-        M->nnz = M->nnzb * M->bs * M->bs;
-    }
     dfree(ctx, deg);
     deg = nullptr;
     if (dalloc(ctx, (void **)&M->bcol, sizeof(int32_t) * M->nnzb) ||
@@ -1381,6 +1392,14 @@ int ffgpu_matrix_csr(const ffgpu_matrix *M, int32_t *rowptr, int32_t *col, doubl
     ffgpu_ctx *ctx = M->ctx;
     cudaStream_t s = ctx->stream;
     FFGPU_CUDA(cudaSetDevice(ctx->device));
+    if (M->bs == 1 && is_device_ptr(rowptr) && is_device_ptr(col) && is_device_ptr(val)) {
+        const int64_t per = 4 * 256;
+        copy_csr_kernel<<<(int)std::min<int64_t>((M->nnz + per - 1) / per + 1, 16 * kNumSM), 256, 0, s>>>(
+            M->n + 1, M->nnz, M->browptr, M->bcol, M->val, rowptr, col, val);
+        FFGPU_TRY(launch_check(ctx, "copy_csr"));
+        FFGPU_CUDA(cudaStreamSynchronize(s));
+        return FFGPU_OK;
+    }
     if (M->bs == 1) {
         // stored as exported: copied to the caller's arrays, host or device
         FFGPU_CUDA(cudaMemcpyAsync(rowptr, M->browptr, sizeof(int32_t) * ((size_t)M->n + 1), cudaMemcpyDefault, s));

@@ -58,6 +58,10 @@ int check_device_status(ffgpu_ctx *ctx, const char *where) {
     int st = 0;
     FFGPU_CUDA(cudaMemcpyAsync(&st, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     FFGPU_CUDA(cudaStreamSynchronize(ctx->stream));
+    return device_status_result(ctx, st, where);
+}
+
+int device_status_result(ffgpu_ctx *ctx, int st, const char *where) {
     if (st != kDevOk) {
         static const char *msg[] = {"ok", "too many candidate neighbours per row (mesh valence)",
                                     "row degree above capacity", "[P2]^3 DOF table is not 3*node+c",
@@ -151,11 +155,35 @@ __global__ void scan_tiles(const int32_t *in, int n, const int32_t *tot, int32_t
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) out[n] = tot[gridDim.x];
 }
 
+// one tile: the whole scan in one block
+__global__ void scan_one_tile(const int32_t *in, int n, int32_t *out) {
+    __shared__ int sh[32];
+    const int base = threadIdx.x * kScanItems;
+    int v[kScanItems], s = 0;
+    for (int k = 0; k < kScanItems; ++k) {
+        v[k] = base + k < n ? in[base + k] : 0;
+        s += v[k];
+    }
+    int t;
+    int pre = block_excl_scan(s, sh, &t);
+    for (int k = 0; k < kScanItems; ++k) {
+        if (base + k < n) out[base + k] = pre;
+        pre += v[k];
+    }
+    if (threadIdx.x == 0) out[n] = t;
+}
+
+// Up to one tile a single launch: small meshes spend their assembly on launches (three kernels,
+// an allocation and a free for each of four scans cost 33 us of 435 on a 33 x 47 square).
 int device_scan_i32(ffgpu_ctx *ctx, const int32_t *in, int32_t *out, int n) {
     int nb = (n + kScanTile - 1) / kScanTile;
     if (nb == 0) {
         FFGPU_CUDA(cudaMemsetAsync(out, 0, sizeof(int32_t), ctx->stream));
         return FFGPU_OK;
+    }
+    if (nb == 1) {
+        scan_one_tile<<<1, kScanThreads, 0, ctx->stream>>>(in, n, out);
+        return launch_check(ctx, "scan_one_tile");
     }
     int32_t *tot = nullptr;
     FFGPU_CUDA(dalloc(ctx, (void **)&tot, sizeof(int32_t) * (nb + 1)));
@@ -181,6 +209,30 @@ __global__ void max_i32_kernel(const int32_t *in, int n, int *out) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+}
+
+// out[0] stays, out[1] = *status, out[2] = *last
+__global__ void gather3_kernel(const int *status, const int32_t *last, int *out) {
+    if (threadIdx.x == 0) out[1] = *status;
+    if (threadIdx.x == 1) out[2] = last ? *last : 0;
+}
+
+// the status word, the largest of in[0..n) and (last != NULL) *last, in one trip to the host
+int device_max_status(ffgpu_ctx *ctx, const int32_t *in, int n, const int32_t *last, const char *where, int *host_max,
+                      int *host_last) {
+    cudaStream_t s = ctx->stream;
+    FFGPU_CUDA(cudaMemsetAsync(ctx->d_iscratch, 0, sizeof(int), s));
+    const int grid = min(kNumSM * 4, max(1, (n + 255) / 256));
+    max_i32_kernel<<<grid, 256, 0, s>>>(in, n, ctx->d_iscratch);
+    FFGPU_TRY(launch_check(ctx, "max_i32"));
+    gather3_kernel<<<1, 32, 0, s>>>(ctx->d_status, last, ctx->d_iscratch);
+    FFGPU_TRY(launch_check(ctx, "gather3"));
+    int h[3] = {0, 0, 0};
+    FFGPU_CUDA(cudaMemcpyAsync(h, ctx->d_iscratch, sizeof(h), cudaMemcpyDeviceToHost, s));
+    FFGPU_CUDA(cudaStreamSynchronize(s));
+    *host_max = h[0];
+    if (host_last) *host_last = h[2];
+    return device_status_result(ctx, h[1], where);
 }
 
 int device_max_i32(ffgpu_ctx *ctx, const int32_t *in, int n, int *host_max) {

@@ -242,6 +242,9 @@ struct DevOut {
 };
 
 int check_device_status(ffgpu_ctx *ctx, const char *where);
+int device_status_result(ffgpu_ctx *ctx, int status, const char *where);   // of a status word already read
+int device_max_status(ffgpu_ctx *ctx, const int32_t *in, int n, const int32_t *last, const char *where, int *host_max,
+                      int *host_last);
 int launch_check(ffgpu_ctx *ctx, const char *what);
 int device_scan_i32(ffgpu_ctx *ctx, const int32_t *in, int32_t *out, int n);  // exclusive, out[n]=total
 // status kBadIndex when an element lists a vertex outside [0, nv) (ffgpu_assembly.cu)
