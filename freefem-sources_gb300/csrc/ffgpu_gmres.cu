@@ -19,11 +19,13 @@
 //   SpMV       w = A vp
 //   gm_dots    s = V' w and the Gram row in one pass over V: blocks are (slab of the vectors'
 //              elements) x (group of basis vectors), w and v_it of a slab staged in shared
-//              memory, one warp reduction per vector per 2048 elements; last block: the sums
+//              memory, one warp reduction per pair of sums and sub-tile; last block: the sums
 //   gm_coef    h = s - L s (a warp per row, all SMs)
-//   gm_update  v_{it+1} = w - V h, ||v_{it+1}||^2; last block: Givens rotations of the new
-//              Hessenberg column (staged in shared memory), residual estimate |g_{it+1}|,
-//              FreeFEM's stopping tests
+//   gm_update  v_{it+1} = w - V h, ||v_{it+1}||^2, and the earlier rotations applied to h as
+//              u = Q h with their product Q (a warp per row); last block: the new rotation, Q's two
+//              changed rows, residual estimate |g_{it+1}|, FreeFEM's stopping tests
+// A rotation after the other (FreeFEM's loop) is a chain of 2 it dependent FP64 operations, 76
+// cycles each on GB300: 14 us at it = 190.  The product Q costs it^2 multiplications over all SMs.
 // and the Arnoldi loop of one restart cycle is a CUDA-graph `while` node.  The host reads the
 // scalars once per restart cycle.  All reductions sum in a fixed order (warp order inside a
 // block, block order across blocks), so results are reproducible run to run.
@@ -33,15 +35,16 @@
 #include <algorithm>
 #include <vector>
 
-#include "ffgpu_internal.cuh"
+#include "ffgpu_gridsync.cuh"
 #include "ffgpu_sell.cuh"
 
 namespace ffgpu {
 
 constexpr int kGmThreads = 256;
 constexpr int kGmWarps = kGmThreads / 32;
-constexpr int kGmSub = 2048;                 // elements of w and v_it staged per sub-tile of gm_dots
-constexpr int kGmMaxSlabs = 256;             // slabs of gm_dots (partials summed by its last block)
+constexpr int kGmSub = 512;                  // elements of w and v_it staged per sub-tile of gm_dots
+constexpr int kGmMaxSlabs = 32;              // slabs of gm_dots (partials summed by its last block)
+constexpr int kGmBack = 512;                 // threads of the back substitution
 constexpr int kGmHs = 1024;                  // Hessenberg columns up to this length stay in shared memory
 
 struct GmScal {
@@ -59,7 +62,8 @@ struct GmArgs {
     const double *b, *dinv;
     const uint8_t *wcl;
     int use_wcl;
-    double *H, *rot0, *rot1, *g, *y, *vnorm, *Gm, *h, *red, *part;
+    int rows;                                // rows of a block of gm_update / gm_xupd
+    double *R, *Q, *u, *g, *y, *vnorm, *Gm, *h, *red, *part;   // R: column it of the triangle at it * (m + 1)
     GmScal *sc;
     cudaGraphConditionalHandle cond;
     int in_graph;
@@ -143,6 +147,7 @@ __global__ void __launch_bounds__(kGmThreads) gm_resid(GmArgs a) {
         const double g0 = sqrt(a.red[0]);
         a.g[0] = g0;
         a.vnorm[0] = g0;
+        a.Q[0] = 1.0;
         if (c->normb < 1.e-20 || c->eps < 0) c->normb = 1.;
         c->it = 0;
         c->stop = 0;
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(kGmThreads) gm_prep(GmArgs a) {
 // s_i = (w, v_i), i <= it, and the Gram row (v_it, v_j), j < it, in one pass over V.
 // Block (slab, group): the elements [slab * slab_len, +slab_len) of the vectors i = group +
 // ngrp * r; per sub-tile of kGmSub elements w and v_it are staged in shared memory and each warp
-// runs its vectors over the sub-tile (64 elements per lane, then one warp reduction per sum).
+// runs its vectors over the sub-tile (16 elements per lane, then one warp reduction for both sums).
 // Partials part[k * nslab + slab], k < 2(it+1); the last block sums them in slab order.
 __global__ void __launch_bounds__(kGmThreads) gm_dots(GmArgs a) {
     extern __shared__ __align__(16) double smd[];
@@ -214,9 +219,8 @@ __global__ void __launch_bounds__(kGmThreads) gm_dots(GmArgs a) {
                 ts = fma(q, wsh[len2], ts);
                 tl = fma(q, vsh[len2], tl);
             }
-            ts = warp_sum(ts);
-            tl = warp_sum(tl);
-            if (lane == 0) { acc[i] += ts; acc[ni + i] += tl; }   // vector i belongs to this warp
+            const double p = warp_sum_pair(ts, tl);   // vector i belongs to this warp
+            if ((lane & 15) == 0) acc[lane ? ni + i : i] += p;
         }
     }
     __syncthreads();
@@ -237,6 +241,7 @@ __global__ void __launch_bounds__(kGmThreads) gm_dots(GmArgs a) {
     for (int k = threadIdx.x; k < K; k += blockDim.x) {
         const double *pk = a.part + (int64_t)k * a.nslab;
         double t = 0;
+#pragma unroll 8
         for (int b = 0; b < a.nslab; ++b) t += __ldcg(pk + b);
         if (k < ni) a.red[k] = t;                                    // s
         else if (k - ni < it) a.Gm[(int64_t)it * ld + (k - ni)] = t;   // Gram row of v_it
@@ -259,96 +264,102 @@ __global__ void __launch_bounds__(kGmThreads) gm_coef(GmArgs a) {
         if (lane == 0) {
             const double hi = __ldcg(a.red + i) - t;
             a.h[i] = hi;
-            a.H[(int64_t)i * ld + it] = hi;
         }
     }
 }
 
-// v_{it+1} = w - sum_i h_i v_i (FreeFEM's order: i = 0..it), ||v_{it+1}||^2; last block: the
-// Hessenberg column's Givens rotations and FreeFEM's stopping tests
-__global__ void __launch_bounds__(kGmThreads) gm_update(GmArgs a) {
-    __shared__ double hs[kGmHs], rc[kGmHs], rs[kGmHs];
-    __shared__ double sh[kGmWarps + 1];
-    const int it = a.sc->it;
-    const int ni = it + 1;
-    const double *hh = a.h;
-    const bool in_smem = ni <= kGmHs;
-    if (in_smem)
-        for (int i = threadIdx.x; i < ni; i += blockDim.x) hs[i] = a.h[i];
-    __syncthreads();
-    if (in_smem) hh = hs;
-    double *vn = a.V + (it + 1) * a.vs;
-    double s = 0;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n; k += (int64_t)gridDim.x * blockDim.x) {
-        double t = a.w[k];
-        // FreeFEM's order i = 0..it; the loads of 16 vectors are issued before their products,
-        // and the next 16 before the products of these (two batches in flight)
-        int i = 0;
-        if (ni >= 16) {
-            double q[16], r[16];
+// sum_i c_i V_i[k] over the vectors i = grp, grp + ngrp, ... < ni, onto t (negated coefficients where
+// SUB): the loads of 16 vectors are issued before their products, and the next 16 before the
+// products of these (two batches in flight)
+template <bool SUB>
+__device__ __forceinline__ double gm_combine(double t, const double *c, const double *V, int64_t vs, int64_t k, int grp,
+                                             int ngrp, int ni) {
+    const int m = (ni - grp + ngrp - 1) / ngrp;   // vectors of this group
+    const double *v = V + (int64_t)grp * vs + k;
+    const int64_t step = (int64_t)ngrp * vs;
+    const auto mad = [&](int j, double q) {
+        const double cj = c[grp + j * ngrp];
+        t = fma(SUB ? -cj : cj, q, t);
+    };
+    int j = 0;
+    if (m >= 16) {
+        double q[16], r[16];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) q[u] = __ldcs(a.V + (i + u) * a.vs + k);
-            for (; i + 32 <= ni; i += 16) {
+        for (int u = 0; u < 16; ++u) q[u] = __ldcs(v + u * step);
+        for (; j + 32 <= m; j += 16) {
 #pragma unroll
-                for (int u = 0; u < 16; ++u) r[u] = __ldcs(a.V + (i + 16 + u) * a.vs + k);
+            for (int u = 0; u < 16; ++u) r[u] = __ldcs(v + (j + 16 + u) * step);
 #pragma unroll
-                for (int u = 0; u < 16; ++u) t = fma(-hh[i + u], q[u], t);
+            for (int u = 0; u < 16; ++u) mad(j + u, q[u]);
 #pragma unroll
-                for (int u = 0; u < 16; ++u) q[u] = r[u];
-            }
-#pragma unroll
-            for (int u = 0; u < 16; ++u) t = fma(-hh[i + u], q[u], t);
-            i += 16;
+            for (int u = 0; u < 16; ++u) q[u] = r[u];
         }
-        for (; i < ni; ++i) t = fma(-hh[i], __ldcs(a.V + i * a.vs + k), t);
-        vn[k] = t;
-        s = fma(t, t, s);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) mad(j + u, q[u]);
+        j += 16;
+    }
+#pragma unroll 8
+    for (; j < m; ++j) mad(j, __ldcs(v + j * step));
+    return t;
+}
+
+// v_{it+1} = w - sum_i h_i v_i and ||v_{it+1}||^2; u = Q h; last block: the new rotation and
+// FreeFEM's stopping tests.  A block takes a.rows elements at a time, 256 / rows threads each on a
+// part of the vectors, so that small systems use all SMs (n = 9282, it = 190: 37 blocks of one
+// thread per element took 53.5 us with the rotations, 14.6 us now).
+__global__ void __launch_bounds__(kGmThreads) gm_update(GmArgs a) {
+    __shared__ double hs[kGmHs], pt[kGmThreads];
+    __shared__ double sh[kGmWarps + 1], rot[2];
+    const int it = a.sc->it;
+    const int ni = it + 1, ld = a.m + 1;
+    const double *hh = a.h;
+    if (ni <= kGmHs) {
+        for (int i = threadIdx.x; i < ni; i += blockDim.x) hs[i] = a.h[i];
+        hh = hs;
+    }
+    __syncthreads();
+    double *vn = a.V + (it + 1) * a.vs;
+    const int rows = a.rows, ngrp = kGmThreads / rows, grp = threadIdx.x / rows, r = threadIdx.x - grp * rows;
+    double s = 0;
+    for (int64_t k0 = (int64_t)blockIdx.x * rows; k0 < a.n; k0 += (int64_t)gridDim.x * rows) {
+        const int64_t k = k0 + r;
+        double t = 0;
+        if (k < a.n) t = gm_combine<true>(grp == 0 ? a.w[k] : 0.0, hh, a.V, a.vs, k, grp, ngrp, ni);
+        if (ngrp > 1) {
+            __syncthreads();
+            pt[threadIdx.x] = t;
+            __syncthreads();
+            if (grp == 0)
+                for (int q = 1; q < ngrp; ++q) t += pt[q * rows + r];
+        }
+        if (grp == 0 && k < a.n) {
+            vn[k] = t;
+            s = fma(t, t, s);
+        }
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = blockIdx.x * kGmWarps + warp; i < ni; i += gridDim.x * kGmWarps) {
+        const double *q = a.Q + (int64_t)i * (ld + 1);
+        double t = 0;
+        const int len = min(ni, i + 2);   // row i ends at its rotation
+        for (int j = lane; j < len; j += 32) t = fma(__ldcg(q + j), hh[j], t);
+        t = warp_sum(t);
+        if (lane == 0) a.u[i] = t;
     }
     const double tot = gm_block_sum(s, sh);
     if (!gm_last_block(&tot, 1, a.part, a.red + 2 * (a.m + 1), &a.sc->ticket)) return;
     GmScal *c = a.sc;
-    const int ld = a.m + 1;
-    double *H = a.H;
-    const double aux = sqrt(a.red[2 * (a.m + 1)]);
-    // the new column's rotations by the earlier ones: a chain through i, staged in shared memory
-    double *col = in_smem ? hs : nullptr;
-    if (in_smem) {
-        for (int i = threadIdx.x; i < it; i += blockDim.x) {
-            rc[i] = a.rot0[i];
-            rs[i] = a.rot1[i];
-        }
-        __syncthreads();
-    }
     if (threadIdx.x == 0) {
+        const double aux = sqrt(a.red[2 * (a.m + 1)]);
         a.vnorm[it + 1] = aux;
-        if (in_smem) {
-            double hi = col[0];
-            for (int i = 0; i < it; i++) {
-                const double hi1 = col[i + 1];
-                const double aa = rc[i] * hi + rs[i] * hi1;
-                const double bb = -rs[i] * hi + rc[i] * hi1;
-                col[i] = aa;
-                hi = bb;
-            }
-            col[it] = hi;
-        } else {
-            for (int i = 0; i < it; i++) {
-                const double hi = H[(int64_t)i * ld + it], hi1 = H[(int64_t)(i + 1) * ld + it];
-                const double aa = a.rot0[i] * hi + a.rot1[i] * hi1;
-                const double bb = -a.rot1[i] * hi + a.rot0[i] * hi1;
-                H[(int64_t)i * ld + it] = aa;
-                H[(int64_t)(i + 1) * ld + it] = bb;
-            }
-        }
-        const double hd = in_smem ? col[it] : H[(int64_t)it * ld + it], hs1 = aux;
+        const double hd = __ldcg(a.u + it), hs1 = aux;
         const double sq = sqrt(hd * hd + hs1 * hs1);
-        a.rot0[it] = hd / sq;
-        a.rot1[it] = hs1 / sq;
-        const double top = a.rot0[it] * hd + a.rot1[it] * hs1;
-        if (in_smem) col[it] = top; else H[(int64_t)it * ld + it] = top;
-        H[(int64_t)(it + 1) * ld + it] = 0.;
-        a.g[it + 1] = -a.rot1[it] * a.g[it];
-        a.g[it] = a.rot0[it] * a.g[it];
+        const double c0 = hd / sq, s0 = hs1 / sq;
+        rot[0] = c0;
+        rot[1] = s0;
+        a.R[(int64_t)it * ld + it] = c0 * hd + s0 * hs1;
+        a.g[it + 1] = -s0 * a.g[it];
+        a.g[it] = c0 * a.g[it];
         const double relres = fabs(a.g[it + 1]);
         c->relres = relres;
         c->steps += 1;
@@ -367,42 +378,61 @@ __global__ void __launch_bounds__(kGmThreads) gm_update(GmArgs a) {
         c->stop = stop;
         if (stop && a.in_graph) gm_set_cond(a.cond, 0);
     }
-    if (in_smem) {
-        __syncthreads();
-        for (int i = threadIdx.x; i <= it; i += blockDim.x) H[(int64_t)i * ld + it] = col[i];
+    __syncthreads();
+    // the column of the triangle, and Q with the new rotation of its rows it and it + 1
+    double *q0 = a.Q + (int64_t)it * (ld + 1), *q1 = q0 + ld + 1;
+    for (int i = threadIdx.x; i <= it + 1; i += blockDim.x) {
+        if (i < it) a.R[(int64_t)it * ld + i] = __ldcg(a.u + i);
+        const double q = i <= it ? __ldcg(q0 + i) : 0.0;
+        q0[i] = i <= it ? rot[0] * q : rot[1];
+        q1[i] = i <= it ? -rot[1] * q : rot[0];
     }
 }
 
-// y = H^-1 g on the it+1 leading rows (back substitution, one warp per row dot)
-__global__ void gm_back(GmArgs a) {
+// y = R^-1 g on the it+1 leading rows, column by column: y_i, then g_j -= R(j,i) y_i for all j < i
+// at once, with the next column's loads under way (one block; a warp per row's dot product took
+// 750 us for 381 rows; the whole solve: 31.2 -> 16.7 ms)
+__global__ void __launch_bounds__(kGmBack) gm_back(GmArgs a) {
+    extern __shared__ __align__(16) double smb[];
     const int it = a.sc->itf;
     if (it < 0) return;
-    const int ld = a.m + 1, lane = threadIdx.x;
-    for (int i = it; i >= 0; i--) {
-        double t = 0;
-        for (int j = i + 1 + lane; j < it + 1; j += 32) t = fma(a.H[(int64_t)i * ld + j], a.y[j], t);
-        t = warp_sum(t);
-        if (lane == 0) a.y[i] = (a.g[i] - t) / a.H[(int64_t)i * ld + i];
-        __syncwarp();
+    const int ld = a.m + 1, t = threadIdx.x;
+    double *gs = smb, *rinv = smb + it + 1;
+    for (int i = t; i <= it; i += kGmBack) {
+        gs[i] = a.g[i];
+        rinv[i] = 1.0 / a.R[(int64_t)i * ld + i];
+    }
+    double next = t < it ? a.R[(int64_t)it * ld + t] : 0.0;
+    __syncthreads();
+    for (int i = it; i >= 0; --i) {
+        const double *col = a.R + (int64_t)i * ld;
+        const double cur = next;
+        next = i > 0 && t < i - 1 ? a.R[(int64_t)(i - 1) * ld + t] : 0.0;
+        const double yi = gs[i] * rinv[i];
+        if (t == 0) a.y[i] = yi;
+        if (t < i) gs[t] = fma(-cur, yi, gs[t]);
+        for (int j = t + kGmBack; j < i; j += kGmBack) gs[j] = fma(-col[j], yi, gs[j]);
+        __syncthreads();
     }
 }
 
 // x = (sum_i y_i Vp_i) + x  (FreeFEM: wi = 0; wi += y_i Vpi[i]; uni = wi + x0)
 __global__ void __launch_bounds__(kGmThreads) gm_xupd(GmArgs a) {
+    __shared__ double pt[kGmThreads];
     const int it = a.sc->itf;
     if (it < 0) return;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n; k += (int64_t)gridDim.x * blockDim.x) {
-        double t = 0;
-        int i = 0;
-        for (; i + 16 <= it + 1; i += 16) {
-            double q[16];
-#pragma unroll
-            for (int u = 0; u < 16; ++u) q[u] = __ldcs(a.Vp + (i + u) * a.vs + k);
-#pragma unroll
-            for (int u = 0; u < 16; ++u) t = fma(a.y[i + u], q[u], t);
+    const int rows = a.rows, ngrp = kGmThreads / rows, grp = threadIdx.x / rows, r = threadIdx.x - grp * rows;
+    for (int64_t k0 = (int64_t)blockIdx.x * rows; k0 < a.n; k0 += (int64_t)gridDim.x * rows) {
+        const int64_t k = k0 + r;
+        double t = k < a.n ? gm_combine<false>(0.0, a.y, a.Vp, a.vs, k, grp, ngrp, it + 1) : 0.0;
+        if (ngrp > 1) {
+            __syncthreads();
+            pt[threadIdx.x] = t;
+            __syncthreads();
+            if (grp == 0)
+                for (int q = 1; q < ngrp; ++q) t += pt[q * rows + r];
         }
-        for (; i <= it; ++i) t = fma(a.y[i], __ldcs(a.Vp + i * a.vs + k), t);
-        a.x[k] = t + a.x[k];
+        if (grp == 0 && k < a.n) a.x[k] = t + a.x[k];
     }
 }
 
@@ -414,6 +444,13 @@ __global__ void gm_x0_kernel(int n, double *x, const double *b, const uint8_t *w
 // grids: vector kernels resident and capped by the work; the dot kernel by tiles
 static int gm_vec_grid(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(4 * kNumSM, (n + kGmThreads - 1) / kGmThreads));
+}
+// rows of a block of gm_update: 256 where that gives every SM a block, else fewer (at least a warp)
+// with the vectors split over the threads left
+static int gm_rows(int64_t n) {
+    int rows = kGmThreads;
+    while (rows > 32 && (n + rows - 1) / rows < kNumSM) rows >>= 1;
+    return rows;
 }
 // gm_dots: sub-tiles of kGmSub elements grouped into at most kGmMaxSlabs slabs, and enough
 // vector groups for about two blocks per SM
@@ -439,18 +476,21 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
     const int itmax = prm->itmax > 0 ? prm->itmax : n;
     const double tgv = prm->tgv > 0 ? prm->tgv : 1e30;
     const size_t dsmem = sizeof(double) * (2 * (size_t)kGmSub + 2 * (size_t)(m + 1));
-    FFGPU_CHECK(dsmem <= 200 * 1024, FFGPU_EINVAL, "gmres: dim_krylov %d above the supported 10000", m);
+    FFGPU_CHECK(sizeof(double) * (4096 + 2 * (size_t)(m + 1)) <= 200 * 1024, FFGPU_EINVAL, "gmres: dim_krylov %d above the supported 10000", m);
     const int64_t vs = vstride(n);
     int nslab = 1, ngrp = 1;
     int64_t slab_len = kGmSub;
     gm_dot_shape(n, nslab, ngrp, slab_len);
+    const int rows = gm_rows(n);
     const int Gv = gm_vec_grid(n), Gd = nslab * ngrp, Gc = gm_coef_grid(m);
+    const int Gu = (int)std::max<int64_t>(1, std::min<int64_t>(4 * kNumSM, ((int64_t)n + rows - 1) / rows));
+    const size_t bsmem = sizeof(double) * 2 * ((size_t)m + 1);
     // workspace: V (m+1 vectors), Vp (m), the SpMV input and output, the small arrays
-    // H, rot0 rot1 g y vnorm, Gram, h, red, part, then the scalars (in doubles, rounded up)
+    // R, Q, u g y vnorm, Gram, h, red, part, then the scalars (in doubles, rounded up)
     const size_t nscal = (sizeof(GmScal) + sizeof(double) - 1) / sizeof(double);
-    const size_t small = (size_t)(m + 2) * (m + 1) + 5 * (size_t)(m + 2) + (size_t)(m + 1) * (m + 1) +
-                         (size_t)(m + 2) + (2 * (size_t)(m + 1) + 2) + 2 * (size_t)(m + 1) * std::max(Gv, nslab) +
-                         nscal;
+    const size_t npart = std::max({2 * (size_t)(m + 1) * nslab, (size_t)Gv, (size_t)Gu});
+    const size_t small = (size_t)(m + 2) * (m + 1) + (size_t)(m + 2) * (m + 2) + 4 * (size_t)(m + 2) +
+                         (size_t)(m + 1) * (m + 1) + (size_t)(m + 2) + (2 * (size_t)(m + 1) + 2) + npart + nscal;
     double *ws = nullptr;
     const size_t nvec = (size_t)(2 * m + 3);
     FFGPU_CUDA(dalloc(ctx, (void **)&ws, sizeof(double) * (nvec * vs + small)));
@@ -460,16 +500,17 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
     a.nslab = nslab; a.ngrp = ngrp; a.slab_len = slab_len;
     a.V = ws; a.Vp = ws + (size_t)(m + 1) * vs; a.vpc = a.Vp + (size_t)m * vs; a.w = a.vpc + vs;
     double *sm = a.w + vs;
-    a.H = sm; sm += (size_t)(m + 2) * (m + 1);
-    a.rot0 = sm; sm += m + 2;
-    a.rot1 = sm; sm += m + 2;
+    a.rows = rows;
+    a.R = sm; sm += (size_t)(m + 2) * (m + 1);
+    a.Q = sm; sm += (size_t)(m + 2) * (m + 2);
+    a.u = sm; sm += m + 2;
     a.g = sm; sm += m + 2;
     a.y = sm; sm += m + 2;
     a.vnorm = sm; sm += m + 2;
     a.Gm = sm; sm += (size_t)(m + 1) * (m + 1);
     a.h = sm; sm += m + 2;
     a.red = sm; sm += 2 * (m + 1) + 2;
-    a.part = sm; sm += 2 * (size_t)(m + 1) * std::max(Gv, nslab);
+    a.part = sm; sm += npart;
     a.sc = reinterpret_cast<GmScal *>(sm);
     sm += nscal;
     if ((size_t)(sm - ws) != nvec * vs + small) {
@@ -479,6 +520,7 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
     a.x = x; a.b = b; a.dinv = A->diag_inv; a.wcl = A->wcl; a.use_wcl = A->ntgv > 0;
     FFGPU_CUDA(cudaMemsetAsync(a.sc, 0, sizeof(GmScal), s));
     FFGPU_CUDA(cudaFuncSetAttribute((const void *)gm_dots, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
+    FFGPU_CUDA(cudaFuncSetAttribute((const void *)gm_back, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
     int rc = FFGPU_OK;
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -544,14 +586,14 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
             int r2 = spmv(A, a.vpc, a.w, trans, s);
             gm_dots<<<Gd, kGmThreads, dsmem, s>>>(ag);
             gm_coef<<<Gc, kGmThreads, 0, s>>>(ag);
-            gm_update<<<Gv, kGmThreads, 0, s>>>(ag);
+            gm_update<<<Gu, kGmThreads, 0, s>>>(ag);
             cudaError_t ec = cudaStreamEndCapture(s, &body);
             if (r2 || ec != cudaSuccess) e = ec != cudaSuccess ? ec : cudaErrorUnknown;
         }
         if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(s, graph, &wnode, nullptr, 1, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            gm_back<<<1, 32, 0, s>>>(ag);
-            gm_xupd<<<Gv, kGmThreads, 0, s>>>(ag);
+            gm_back<<<1, kGmBack, bsmem, s>>>(ag);
+            gm_xupd<<<Gu, kGmThreads, 0, s>>>(ag);
             e = cudaStreamEndCapture(s, &graph);
         }
         if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
@@ -581,12 +623,12 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
                 if ((rc = spmv(A, a.vpc, a.w, trans, s))) break;
                 gm_dots<<<Gd, kGmThreads, dsmem, s>>>(a);
                 gm_coef<<<Gc, kGmThreads, 0, s>>>(a);
-                gm_update<<<Gv, kGmThreads, 0, s>>>(a);
+                gm_update<<<Gu, kGmThreads, 0, s>>>(a);
                 ctx->launches += 4;
             }
             if (rc) break;
-            gm_back<<<1, 32, 0, s>>>(a);
-            gm_xupd<<<Gv, kGmThreads, 0, s>>>(a);
+            gm_back<<<1, kGmBack, bsmem, s>>>(a);
+            gm_xupd<<<Gu, kGmThreads, 0, s>>>(a);
             ctx->launches += 2;
         } else {
             FFGPU_CUDA(cudaGraphLaunch(exec, s));
