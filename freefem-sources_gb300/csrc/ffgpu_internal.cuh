@@ -147,10 +147,11 @@ struct ffgpu_matrix {
     int last_cluster;     // the last FP64 CG solve ran in one thread-block cluster
     void *direct;         // factorisation state of the direct solver (ffgpu_direct.cu), or NULL
     int direct_method;    // FFGPU_DIRECT_AUTO / _CHOLESKY / _QR
-    // SELL-32 copy for the Krylov SpMVs: block rows sliced into chunks of 32 (one row per
-    // lane), rows sorted by decreasing degree inside windows of 1024 rows, each chunk padded
-    // to its longest row and stored slot-major so that a warp reads 32 consecutive entries.
-    int nchunk;           // ceil(nb/32)
+    // SELL-32 copy for the Krylov SpMVs: block rows sliced into chunks of 32 lanes (one row per
+    // lane, or four lanes per row: sell_lanes), by decreasing degree inside windows of 1024 rows
+    // (scalar) or over the whole matrix (3x3 blocks), each chunk padded to its longest row and
+    // stored slot-major so that a warp reads 32 consecutive entries.
+    int nchunk;           // ceil(nb * lanes per row / 32)
     int64_t nslot;        // slot rows (sum of the chunk lengths)
     int32_t *sperm;       // nchunk*32: block row of each lane (-1: padding lane)
     int32_t *slen;        // nchunk: slots of each chunk
@@ -166,7 +167,7 @@ struct ffgpu_matrix {
     // in-kernel CG loop (ffgpu_persist.cu): widest column range and most row-group slots of a
     // block (0: not measured yet, -1: could not be)
     int band_range, band_slots;
-    int sell32_kind;      // chunk assignment of the FP32 SELL SpMV (tuned): 64 ranges, 65 rotated
+    int sell32_kind;      // chunk assignment of the FP32 SELL SpMV (tuned): 64 ranges, 65 stride
 };
 
 namespace ffgpu {
@@ -303,7 +304,19 @@ struct SellArgs {
     const int32_t *perm, *len, *off, *col;
     const int16_t *col16;
     const int32_t *part;   // chunks [part[w], part[w+1]) belong to warp w of the launch
+    int unit;              // consecutive chunks that stay on one SM (spread assignment)
 };
+// Units of 8 keep neighbouring rows' gathers in one L1 where every SM has many of them; with fewer than
+// four rounds of such units per SM the remainder would unbalance the SMs: single chunks
+inline int sell_unit(int nchunk) { return nchunk >= 4 * 8 * kNumSM ? 8 : 1; }
+// blocks of the 3x3 stride assignment
+inline int sell_spread_grid(int nchunk) { return nchunk < kNumSM ? (nchunk > 0 ? nchunk : 1) : kNumSM; }
+// Lanes per block row: four for 3x3 blocks below kSellWideRows block rows.  A chunk is then 8 rows, a
+// quarter as long, which 608 FP64 pipes can share evenly, against 5 % of padding (rows end at
+// multiples of four) and three adds a row.  K_a, best of the candidates: 117 649 block rows 82 us with one lane (and with block
+// CSR), 74 us with four; 388 725 rows 196 and 198 us (double-float 145 and 159 us).
+constexpr int kSellWideRows = 300000;
+inline int sell_lanes(const ffgpu_matrix *A) { return A->bs == 3 && A->nb < kSellWideRows ? 4 : 1; }
 int sell_prepare(ffgpu_matrix *A);               // structure (once per pattern)
 // chunk ranges of the nw warps of a launch, equal slot counts (built once per nw)
 int sell_partition(ffgpu_matrix *A, int nw, const int32_t **part);
@@ -313,7 +326,7 @@ void sell_release_values(ffgpu_matrix *A);       // drop the value arrays (new n
 int ir_time_ka(ffgpu_matrix *A, int nrep, float *ms);
 void sell_release(ffgpu_matrix *A);              // drop everything (matrix destruction)
 inline SellArgs sell_args(const ffgpu_matrix *A) {
-    return SellArgs{A->nchunk, A->sperm, A->slen, A->soff, A->scol, A->scol16, nullptr};
+    return SellArgs{A->nchunk, A->sperm, A->slen, A->soff, A->scol, A->scol16, nullptr, sell_unit(A->nchunk)};
 }
 // Persistent grid of a kernel: resident blocks per SM (occupancy calculator) x SMs
 int resident_grid(const void *kernel, int threads, size_t smem = 0);

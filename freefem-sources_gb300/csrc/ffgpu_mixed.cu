@@ -40,8 +40,8 @@ struct InnerScalars {
 __device__ __noinline__ void ir_graph_stop(cudaGraphConditionalHandle cond) { cudaGraphSetConditional(cond, 0); }
 
 // inner K_a on the SELL-32 FP32 copy: q = A h and (h, q) -> rho
-template <int BS, bool C16, int ASSIGN, bool DEEP>
-__global__ void __launch_bounds__(kMxWarps * 32) ir_ka(SellArgs S, const float *__restrict__ val,
+template <int BS, bool C16, int ASSIGN, bool DEEP, int T = 1>
+__global__ void __launch_bounds__(sell_threads(BS, ASSIGN)) ir_ka(SellArgs S, const float *__restrict__ val,
                                                        const float *__restrict__ h, float *__restrict__ q,
                                                        InnerScalars *ks, float *part) {
     __shared__ float sh[32];
@@ -49,13 +49,13 @@ __global__ void __launch_bounds__(kMxWarps * 32) ir_ka(SellArgs S, const float *
     if (ks->done) return;
     const int lane = threadIdx.x & 31;
     float hq = 0;
-    sell_for_chunks<ASSIGN>(S, [&](int c, int a, int L, int64_t sr) {
+    sell_for_chunks<ASSIGN, BS>(S, [&](int c, int a, int L, int64_t sr) {
         float y[BS];
         sell_row32<BS, C16, DEEP>(S, val, h, L, sr, lane, a, y);
-        if (a >= 0) {
+        if (sell_reduce<BS, T>(y, a, lane)) {
 #pragma unroll
-            for (int m = 0; m < BS; ++m) {
-                const int64_t i = (int64_t)BS * a + m;
+            for (int m = 0; m < (T == 1 ? BS : 1); ++m) {
+                const int64_t i = sell_dof<BS, T>(a, lane) + m;
                 q[i] = y[m];
                 hq = fmaf(h[i], y[m], hq);
             }
@@ -255,17 +255,20 @@ constexpr int kSellCode = 64;
 
 static void *ir_ka_fn(const ffgpu_matrix *A, int kind) {
     const int code = kind >= kSellCode ? kind - kSellCode : 0;
-    void *t[3][4] = {{(void *)ir_ka<1, false, 0, false>, (void *)ir_ka<1, false, 1, false>,
-                      (void *)ir_ka<1, false, 0, true>, (void *)ir_ka<1, false, 1, true>},
-                     {(void *)ir_ka<1, true, 0, false>, (void *)ir_ka<1, true, 1, false>,
-                      (void *)ir_ka<1, true, 0, true>, (void *)ir_ka<1, true, 1, true>},
-                     {(void *)ir_ka<3, false, 0, false>, (void *)ir_ka<3, false, 1, false>,
-                      (void *)ir_ka<3, false, 0, true>, (void *)ir_ka<3, false, 1, true>}};
-    return t[A->bs == 3 ? 2 : (A->scol16 ? 1 : 0)][code];
+#define FFGPU_IR_ROW(BS, C16, T)                                                                     \
+    {(void *)ir_ka<BS, C16, 0, false, T>, (void *)ir_ka<BS, C16, 1, false, T>, (void *)ir_ka<BS, C16, 0, true, T>, \
+     (void *)ir_ka<BS, C16, 1, true, T>}
+    static void *const t[4][4] = {FFGPU_IR_ROW(1, false, 1), FFGPU_IR_ROW(1, true, 1), FFGPU_IR_ROW(3, false, 1),
+                                  FFGPU_IR_ROW(3, false, 4)};
+#undef FFGPU_IR_ROW
+    return t[A->bs == 3 ? (sell_lanes(A) == 4 ? 3 : 2) : (A->scol16 ? 1 : 0)][code];
 }
 // grids: the FP32 K_a by the chunks it has to take, the vector kernels by the n/4 float4 quads
-static int ir_ka_grid(const ffgpu_matrix *A, const void *ka) {
-    return sized_grid(ka, kMxWarps * 32, ((int64_t)A->nchunk + kMxWarps - 1) / kMxWarps);
+static int ir_ka_assign(int kind) { return kind >= kSellCode ? (kind - kSellCode) & 1 : kSellRanges; }
+static int ir_ka_grid(const ffgpu_matrix *A, const void *ka, int assign) {
+    return A->bs == 3 && assign == kSellStride
+               ? sell_spread_grid(A->nchunk)
+               : sized_grid(ka, kMxWarps * 32, ((int64_t)A->nchunk + kMxWarps - 1) / kMxWarps);
 }
 static int ir_vec_grid(const void *k, int n) {
     return min(4096, sized_grid(k, kMxThreads, ((int64_t)n / 4 + kMxThreads - 1) / kMxThreads));
@@ -281,7 +284,7 @@ static int ir_body(ffgpu_matrix *A, IRState &S, int unroll, cudaGraphConditional
     SellArgs sa = sell_args(A);
     const float *sv = A->sval32;
     void *ka = ir_ka_fn(A, A->sell32_kind);
-    const int gka = ir_ka_grid(A, ka);
+    const int assign = ir_ka_assign(A->sell32_kind), gka = ir_ka_grid(A, ka, assign);
     if (ir_ranges(A)) FFGPU_TRY(sell_partition(A, gka * kMxWarps, &sa.part));
     const int gkb = ir_vec_grid((const void *)ir_kb, A->n);
     const int gkc = ir_vec_grid((const void *)ir_kc, A->n);
@@ -291,7 +294,7 @@ static int ir_body(ffgpu_matrix *A, IRState &S, int unroll, cudaGraphConditional
         void *aa[] = {&sa, &sv, &S.h, &S.q, &S.ks, &part};
         void *ab[] = {&n, &S.d, &S.g, &S.h, &S.q, &S.dinv, &S.ks, &part, &cond, &in_graph};
         void *ac[] = {&n, &S.g, &S.h, &S.dinv, &S.ks, &part};
-        launch_ex(ka, gka, kMxWarps * 32, aa, 0, s, pdl);
+        launch_ex(ka, gka, sell_threads(A->bs, assign), aa, 0, s, pdl);
         launch_ex((const void *)ir_kb, gkb, kMxThreads, ab, 0, s, pdl);
         launch_ex((const void *)ir_kc, gkc, kMxThreads, ac, 0, s, pdl);
     }
@@ -314,18 +317,18 @@ static int ir_tune(ffgpu_matrix *A, IRState &S) {
     cudaEventCreate(&e1);
     float tms[4];
     const int kinds[4] = {kSellCode, kSellCode + 1, kSellCode + 2, kSellCode + 3};
-    const char *names[4] = {"ranges", "rotated", "ranges deep", "rotated deep"};
+    const char *names[4] = {"ranges", "stride", "ranges deep", "stride deep"};
     for (int kk = 0; kk < 4; ++kk) {
         SellArgs sa = sell_args(A);
         const float *sv = A->sval32;
         void *ka = ir_ka_fn(A, kinds[kk]);
-        const int g = ir_ka_grid(A, ka);
+        const int g = ir_ka_grid(A, ka, kk & 1);
         if ((kk & 1) == kSellRanges) FFGPU_TRY(sell_partition(A, g * kMxWarps, &sa.part));
         float *part = (float *)ctx->d_part;
         void *aa[] = {&sa, &sv, &S.h, &S.q, &S.ks, &part};
-        cudaLaunchKernel(ka, g, kMxWarps * 32, aa, 0, s);
+        cudaLaunchKernel(ka, g, sell_threads(A->bs, kk & 1), aa, 0, s);
         cudaEventRecord(e0, s);
-        for (int r = 0; r < 3; ++r) cudaLaunchKernel(ka, g, kMxWarps * 32, aa, 0, s);
+        for (int r = 0; r < 3; ++r) cudaLaunchKernel(ka, g, sell_threads(A->bs, kk & 1), aa, 0, s);
         cudaEventRecord(e1, s);
         FFGPU_CUDA(cudaEventSynchronize(e1));
         FFGPU_CUDA(cudaGetLastError());
@@ -359,7 +362,7 @@ int ir_time_ka(ffgpu_matrix *A, int nrep, float *ms) {
     SellArgs sa = sell_args(A);
     const float *sv = A->sval32;
     void *ka = ir_ka_fn(A, A->sell32_kind);
-    const int g = ir_ka_grid(A, ka);
+    const int assign = ir_ka_assign(A->sell32_kind), g = ir_ka_grid(A, ka, assign);
     int rc = FFGPU_OK;
     if (ir_ranges(A)) rc = sell_partition(A, g * kMxWarps, &sa.part);
     float t = 0;
@@ -369,9 +372,9 @@ int ir_time_ka(ffgpu_matrix *A, int nrep, float *ms) {
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
-        cudaLaunchKernel(ka, g, kMxWarps * 32, aa, 0, s);
+        cudaLaunchKernel(ka, g, sell_threads(A->bs, assign), aa, 0, s);
         cudaEventRecord(e0, s);
-        for (int r = 0; r < nrep; ++r) cudaLaunchKernel(ka, g, kMxWarps * 32, aa, 0, s);
+        for (int r = 0; r < nrep; ++r) cudaLaunchKernel(ka, g, sell_threads(A->bs, assign), aa, 0, s);
         cudaEventRecord(e1, s);
         cudaError_t e = cudaEventSynchronize(e1);
         if (e == cudaSuccess) e = cudaEventElapsedTime(&t, e0, e1);
@@ -395,7 +398,7 @@ static int ir_build_graph(ffgpu_matrix *A, IRState &S, int unroll) {
     // the warp partition is built before the capture starts (no allocation inside a capture)
     if (ir_ranges(A)) {
         const int32_t *part = nullptr;
-        FFGPU_TRY(sell_partition(A, ir_ka_grid(A, ir_ka_fn(A, A->sell32_kind)) * kMxWarps, &part));
+        FFGPU_TRY(sell_partition(A, ir_ka_grid(A, ir_ka_fn(A, A->sell32_kind), kSellRanges) * kMxWarps, &part));
     }
     // with programmatic dependent launch between the body's kernels first, else the plain graph
     cudaError_t e = cudaErrorUnknown;

@@ -2,16 +2,17 @@
 //
 // The assembled matrix stays in block CSR (FreeFEM's pattern, sorted columns); that is what
 // export, the transpose and the diagonal read.  The CG/IR SpMVs read a sliced copy instead:
-//   * block rows are sorted by decreasing degree inside windows of 1024 consecutive rows
-//     (rows stay near their neighbours, so the x gathers of a warp stay local), stable;
-//   * 32 consecutive sorted rows form a chunk, one row per lane; a chunk is padded to its
-//     longest row (the first one) with zero blocks;
+//   * rows are sorted by decreasing degree, stable: scalar rows inside windows of 1024 consecutive
+//     rows, 3x3 block rows over the whole matrix (rowperm; the rows of one degree keep their
+//     order, so the x gathers of a warp stay local);
+//   * 32 consecutive sorted rows form a chunk, one row per lane -- or 8 rows, four lanes each, entry
+//     4 j + sub of a row in slot j of lane sub (sell_lanes); a chunk is padded to its longest row
+//     (the first one) with zero blocks;
 //   * entry j of lane r of chunk c is stored at slot row soff[c] + j, lane r: a warp reads
 //     32 consecutive column indices and, for each of the bs*bs values, 32 consecutive values.
 // Every lane of a warp runs the same trip count, every load is a full 128/256-byte line, and
-// no lane-group reductions are needed.  Each warp of a launch owns a contiguous range of
-// chunks holding an equal share of the slots (sell_partition): windows start with their
-// longest rows, so a fixed stride over chunks would give some warps only long chunks.
+// no lane-group reductions are needed with one lane per row.  How the chunks go to the warps:
+// ffgpu_sell.cuh.
 // Within a row the entries keep their column order, so the row sums are formed in the same
 // order as the block-CSR kernels form them.
 // For bs == 1 the column is stored as the 16-bit difference column - row whenever the
@@ -56,12 +57,18 @@ __global__ void __launch_bounds__(kSellWin) sell_sort_kernel(int nb, const int32
         s == 0xFFFFFFFFu ? -1 : (int32_t)((int64_t)blockIdx.x * kSellWin + (s & 1023u));
 }
 
-__global__ void sell_len_kernel(int nchunk, const int32_t *__restrict__ perm, const int32_t *__restrict__ rp,
+// the row of each lane in rowperm order, T lanes per row; -1 past the last row (padding lanes)
+__global__ void sell_perm_kernel(int nb, int T, int npad, const int32_t *__restrict__ rowperm, int32_t *__restrict__ perm) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < npad) perm[t] = t / T < nb ? rowperm[t / T] : -1;
+}
+
+__global__ void sell_len_kernel(int nchunk, int T, const int32_t *__restrict__ perm, const int32_t *__restrict__ rp,
                                 int32_t *__restrict__ len) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < nchunk) {
         const int a = perm[(int64_t)c * 32];
-        len[c] = a >= 0 ? rp[a + 1] - rp[a] : 0;
+        len[c] = a >= 0 ? (rp[a + 1] - rp[a] + T - 1) / T : 0;
     }
 }
 
@@ -77,7 +84,7 @@ __global__ void sell_band_kernel(int nb, const int32_t *__restrict__ rp, const i
 
 // column slots: padding entries repeat the row's last column (a valid, cached x entry)
 template <bool C16>
-__global__ void sell_col_kernel(int nchunk, const int32_t *__restrict__ perm, const int32_t *__restrict__ len,
+__global__ void sell_col_kernel(int nchunk, int T, const int32_t *__restrict__ perm, const int32_t *__restrict__ len,
                                 const int32_t *__restrict__ off, const int32_t *__restrict__ rp,
                                 const int32_t *__restrict__ col, int32_t *__restrict__ scol,
                                 int16_t *__restrict__ scol16) {
@@ -89,7 +96,7 @@ __global__ void sell_col_kernel(int nchunk, const int32_t *__restrict__ perm, co
     const int64_t base = (int64_t)off[c] * 32 + lane;
     const int b = a >= 0 ? rp[a] : 0, deg = a >= 0 ? rp[a + 1] - b : 0;
     for (int j = 0; j < L; ++j) {
-        const int cj = deg > 0 ? col[b + min(j, deg - 1)] : (a >= 0 ? a : 0);
+        const int cj = deg > 0 ? col[b + min(j * T + lane % T, deg - 1)] : (a >= 0 ? a : 0);
         if (C16) scol16[base + (int64_t)j * 32] = (int16_t)(cj - (a >= 0 ? a : 0));
         else scol[base + (int64_t)j * 32] = cj;
     }
@@ -106,7 +113,7 @@ struct ToDF {
 
 // values: lane r, slot j, entry m at ((off[c] + j) * bs2 + m) * 32 + r; padding is zero
 template <int BS, typename Out, typename Conv>
-__global__ void sell_val_kernel(int nchunk, const int32_t *__restrict__ perm, const int32_t *__restrict__ len,
+__global__ void sell_val_kernel(int nchunk, int T, const int32_t *__restrict__ perm, const int32_t *__restrict__ len,
                                 const int32_t *__restrict__ off, const int32_t *__restrict__ rp,
                                 const double *__restrict__ val, Out *__restrict__ out) {
     constexpr int B2 = BS * BS;
@@ -119,9 +126,10 @@ __global__ void sell_val_kernel(int nchunk, const int32_t *__restrict__ perm, co
     const int b = a >= 0 ? rp[a] : 0, deg = a >= 0 ? rp[a + 1] - b : 0;
     Conv conv;
     for (int j = 0; j < L; ++j) {
-        const double *src = val + (int64_t)(b + j) * B2;
+        const int k = j * T + lane % T;
+        const double *src = val + (int64_t)(b + k) * B2;
 #pragma unroll
-        for (int m = 0; m < B2; ++m) out[base + ((int64_t)j * B2 + m) * 32] = conv(j < deg ? src[m] : 0.0);
+        for (int m = 0; m < B2; ++m) out[base + ((int64_t)j * B2 + m) * 32] = conv(k < deg ? src[m] : 0.0);
     }
 }
 
@@ -173,14 +181,19 @@ int sell_prepare(ffgpu_matrix *A) {
     FFGPU_CHECK(A->max_deg < 0x1FFFFF, FFGPU_EINVAL, "SELL layout: row degree %d too large", A->max_deg);
     const int nb = A->nb;
     const int nwin = (nb + kSellWin - 1) / kSellWin;
-    const int nchunk = (nb + 31) / 32;
+    const int T = sell_lanes(A);
+    const int nchunk = (int)(((int64_t)nb * T + 31) / 32);
+    const bool windows = A->bs == 1;
     A->nchunk = nchunk;
-    FFGPU_CUDA(dalloc(ctx, (void **)&A->sperm, sizeof(int32_t) * (size_t)nwin * kSellWin));
+    FFGPU_CUDA(dalloc(ctx, (void **)&A->sperm, sizeof(int32_t) * (windows ? (size_t)nwin * kSellWin : (size_t)nchunk * 32)));
     FFGPU_CUDA(dalloc(ctx, (void **)&A->slen, sizeof(int32_t) * ((size_t)nchunk + 1)));
     FFGPU_CUDA(dalloc(ctx, (void **)&A->soff, sizeof(int32_t) * ((size_t)nchunk + 1)));
-    sell_sort_kernel<<<nwin, kSellWin, 0, s>>>(nb, A->browptr, A->sperm);
-    FFGPU_TRY(launch_check(ctx, "sell_sort"));
-    sell_len_kernel<<<(nchunk + 255) / 256, 256, 0, s>>>(nchunk, A->sperm, A->browptr, A->slen);
+    if (windows)
+        sell_sort_kernel<<<nwin, kSellWin, 0, s>>>(nb, A->browptr, A->sperm);
+    else
+        sell_perm_kernel<<<(nchunk * 32 + 255) / 256, 256, 0, s>>>(nb, T, nchunk * 32, A->rowperm, A->sperm);
+    FFGPU_TRY(launch_check(ctx, "sell_order"));
+    sell_len_kernel<<<(nchunk + 255) / 256, 256, 0, s>>>(nchunk, T, A->sperm, A->browptr, A->slen);
     FFGPU_TRY(launch_check(ctx, "sell_len"));
     FFGPU_TRY(device_scan_i32(ctx, A->slen, A->soff, nchunk));
     int32_t nslot = 0;
@@ -204,11 +217,11 @@ int sell_prepare(ffgpu_matrix *A) {
     const int grid = (int)((thr + 255) / 256);
     if (c16) {
         FFGPU_CUDA(dalloc(ctx, (void **)&A->scol16, sizeof(int16_t) * (size_t)ent));
-        sell_col_kernel<true><<<grid, 256, 0, s>>>(nchunk, A->sperm, A->slen, A->soff, A->browptr, A->bcol,
+        sell_col_kernel<true><<<grid, 256, 0, s>>>(nchunk, T, A->sperm, A->slen, A->soff, A->browptr, A->bcol,
                                                    nullptr, A->scol16);
     } else {
         FFGPU_CUDA(dalloc(ctx, (void **)&A->scol, sizeof(int32_t) * (size_t)ent));
-        sell_col_kernel<false><<<grid, 256, 0, s>>>(nchunk, A->sperm, A->slen, A->soff, A->browptr, A->bcol,
+        sell_col_kernel<false><<<grid, 256, 0, s>>>(nchunk, T, A->sperm, A->slen, A->soff, A->browptr, A->bcol,
                                                     A->scol, nullptr);
     }
     return launch_check(ctx, "sell_col");
@@ -223,10 +236,10 @@ static int sell_fill(ffgpu_matrix *A, const double *src, Out **dst) {
     const int64_t thr = (int64_t)A->nchunk * 32;
     const int grid = (int)((thr + 255) / 256);
     if (A->bs == 3)
-        sell_val_kernel<3, Out, Conv><<<grid, 256, 0, ctx->stream>>>(A->nchunk, A->sperm, A->slen, A->soff,
+        sell_val_kernel<3, Out, Conv><<<grid, 256, 0, ctx->stream>>>(A->nchunk, sell_lanes(A), A->sperm, A->slen, A->soff,
                                                                     A->browptr, src, *dst);
     else
-        sell_val_kernel<1, Out, Conv><<<grid, 256, 0, ctx->stream>>>(A->nchunk, A->sperm, A->slen, A->soff,
+        sell_val_kernel<1, Out, Conv><<<grid, 256, 0, ctx->stream>>>(A->nchunk, sell_lanes(A), A->sperm, A->slen, A->soff,
                                                                     A->browptr, src, *dst);
     return launch_check(ctx, "sell_values");
 }

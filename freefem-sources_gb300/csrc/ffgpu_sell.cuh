@@ -75,16 +75,26 @@ __device__ __forceinline__ float2 split_f64(double v) {
 }
 
 // ------------------------------------------------------------------ SELL-32 chunk assignment
-// kSellRanges: warp w takes the contiguous chunks [part[w], part[w+1]) (equal slot shares).
-// kSellRotated: pass k of warp w takes chunk k*nw + (w + 5k) mod nw -- the chunks in flight at
-//   a time stay one contiguous band of the matrix, and the rotation by an odd step walks every
-//   warp through all 32 positions of the degree-sorted windows.
+// kSellRanges: warp w takes the contiguous chunks [part[w], part[w+1]) (equal slot shares), blocks
+//   of 8 warps, as many as are resident.
+// kSellStride, scalar rows: pass k of warp w takes chunk k*nw + (w + 5k) mod nw -- the chunks in
+//   flight at a time stay one contiguous band of the matrix, and the rotation by an odd step walks
+//   every warp through all 32 positions of the degree-sorted windows.
+// kSellStride, 3x3 blocks (chunks longest first over the whole matrix): one block of 32 warps per
+//   SM; units of S.unit consecutive chunks go round the SMs, there and back, and on each SM round the
+//   warps and so the four sub-partitions.  These kernels are bound by FP64 issue, one pipe per
+//   sub-partition, and the chunks of a [P2]^3 matrix are 19 to 65 slots long: what has to be even is
+//   the slots of each of the 608 pipes ([P2]^3 on 60^3 cells, 1.77 M block rows: 0.874 ms with the
+//   rotated stride over windows, 0.807 ms; scalar rows are nearly all of one length and lose 5 %
+//   by it).
 // The tuners time both, each with two unroll depths of the row loop (DEEP).
-enum SellAssign { kSellRanges = 0, kSellRotated = 1 };
+enum SellAssign { kSellRanges = 0, kSellStride = 1 };
+// threads of a block
+constexpr int sell_threads(int bs, int assign) { return bs == 3 && assign == kSellStride ? 1024 : 256; }
 
-template <int ASSIGN>
+template <int ASSIGN, int BS>
 struct ChunkWalk {
-    int c, ce, k, w, nw;
+    int c, ce, k, w, nw, U;
     __device__ __forceinline__ ChunkWalk(const SellArgs &S) {
         w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
         nw = (gridDim.x * blockDim.x) >> 5;
@@ -93,33 +103,47 @@ struct ChunkWalk {
             c = __ldg(S.part + w);
             ce = __ldg(S.part + w + 1);
         } else {
+            U = S.unit;
+            if constexpr (BS == 3) k = (threadIdx.x >> 5) / U;
             ce = S.nchunk;
-            c = at(0);
+            c = at(k);
         }
     }
-    __device__ __forceinline__ int at(int kk) const { return kk * nw + (w + 5 * kk) % nw; }
+    __device__ __forceinline__ int at(int kk) const {
+        if constexpr (BS == 3) {
+            const int u = kk * (int)gridDim.x + (kk & 1 ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+            return u * U + (threadIdx.x >> 5) % U;
+        }
+        return kk * nw + (w + 5 * kk) % nw;
+    }
     // next chunk of this warp (>= ce when done)
-    __device__ __forceinline__ int next() {
+    __device__ __forceinline__ int next() const {
         if constexpr (ASSIGN == kSellRanges) return c + 1;
+        if constexpr (BS == 3) return at(k + (int)(blockDim.x >> 5) / U);   // a warp's chunks ascend
         return (int64_t)(k + 1) * nw < ce ? at(k + 1) : ce;
     }
-    __device__ __forceinline__ void advance(int cn) { c = cn; ++k; }
+    __device__ __forceinline__ void advance(int cn) {
+        c = cn;
+        k += BS == 3 && ASSIGN == kSellStride ? (int)(blockDim.x >> 5) / U : 1;
+    }
 };
 
 // Calls body(c, a, L, sr) for every chunk of this warp (a: the lane's row, L: slots, sr: first
 // slot row), loading the next chunk's row, length and offset while the current one runs.
-template <int ASSIGN, typename F>
+template <int ASSIGN, int BS, typename F>
 __device__ __forceinline__ void sell_for_chunks(const SellArgs &S, F &&body) {
     const int lane = threadIdx.x & 31;
-    ChunkWalk<ASSIGN> it(S);
+    ChunkWalk<ASSIGN, BS> it(S);
     // the rotated stride can land past the last chunk on a warp's final pass
-    while (it.c < it.ce && it.c >= S.nchunk) it.advance(it.next());
+    if (BS == 1)
+        while (it.c < it.ce && it.c >= S.nchunk) it.advance(it.next());
     if (it.c >= it.ce) return;
     int a = __ldg(S.perm + (int64_t)it.c * 32 + lane), L = __ldg(S.len + it.c);
     int64_t sr = __ldg(S.off + it.c);
     for (;;) {
         int cn = it.next();
-        while (cn < it.ce && cn >= S.nchunk) { it.advance(cn); cn = it.next(); }
+        if (BS == 1)
+            while (cn < it.ce && cn >= S.nchunk) { it.advance(cn); cn = it.next(); }
         int an = 0, Ln = 0;
         int64_t srn = 0;
         if (cn < it.ce) {
@@ -133,6 +157,27 @@ __device__ __forceinline__ void sell_for_chunks(const SellArgs &S, F &&body) {
         a = an; L = Ln; sr = srn;
     }
 }
+
+// Row sums of T lanes per row.  T = 1: the lane's own row (component m in y[m]).  T = 4, 3x3 blocks:
+// lane sub of the row's four ends with the total of component sub in y[0] (sub = 3: none), in
+// three FP64 adds for the three totals.  Returns whether the lane holds a result.
+template <int BS, int T, typename V>
+__device__ __forceinline__ bool sell_reduce(V *y, int a, int lane) {
+    if constexpr (T == 4) {
+        static_assert(BS == 3, "four lanes per row: 3x3 blocks");
+        const bool hi = lane & 2, odd = lane & 1;
+        // lanes 0, 1 take components 0 and 1 of all four lanes, lanes 2, 3 component 2
+        const V s0 = __shfl_xor_sync(0xffffffffu, hi ? y[0] : y[2], 2), s1 = __shfl_xor_sync(0xffffffffu, y[1], 2);
+        const V p = (hi ? y[2] : y[0]) + s0, q = y[1] + s1;
+        const V other = __shfl_xor_sync(0xffffffffu, hi ? p : (odd ? p : q), 1);
+        y[0] = (hi ? p : (odd ? q : p)) + other;
+        return a >= 0 && (lane & 3) < 3;
+    }
+    return a >= 0;
+}
+// first DOF of a lane's result(s) and their number
+template <int BS, int T>
+__device__ __forceinline__ int64_t sell_dof(int a, int lane) { return (int64_t)BS * a + (T == 4 ? (lane & 3) : 0); }
 
 // ------------------------------------------------------------------ SELL-32 rows
 // Entries are read in column order; matrix streams use evict-first loads so that the gathered

@@ -397,13 +397,12 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) cg_ka_x(SpmvArgsX A, const fl
 }
 
 // ------------------------------------------------------------------ SELL-32 K_a
-// One block row per lane, one chunk of 32 rows per warp (resident grid, chunks strided over
-// warps).  FP64: AH = A H and (H, AH) -> rho; padding lanes (a < 0) write nothing.
+// One block row per lane, one chunk of 32 rows per warp (the assignments of ffgpu_sell.cuh).  FP64: AH = A H and (H, AH) -> rho; padding lanes (a < 0) write nothing.
 // (Six blocks per SM at 40 registers -- the unrolled loops fit without spilling -- measured
 // slower than the compiler's 64 registers at four: [P2]^3 K_a 1.110 against 1.055 ms, P1
 // cube(160) 0.185 against 0.146 ms; fewer loads in flight per thread.)
-template <int BS, bool C16, int ASSIGN, int LOOP>
-__global__ void __launch_bounds__(kSpmvWarps * 32) cg_ka_sell(SellArgs S, const double *__restrict__ val,
+template <int BS, bool C16, int ASSIGN, int LOOP, int T = 1>
+__global__ void __launch_bounds__(sell_threads(BS, ASSIGN)) cg_ka_sell(SellArgs S, const double *__restrict__ val,
                                                               const double *__restrict__ h, double *__restrict__ q,
                                                               KrylovScalars *ks, double *part) {
     __shared__ double sh[32];
@@ -411,13 +410,13 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) cg_ka_sell(SellArgs S, const 
     if (ks->done) return;
     const int lane = threadIdx.x & 31;
     double hq = 0;
-    sell_for_chunks<ASSIGN>(S, [&](int c, int a, int L, int64_t sr) {
+    sell_for_chunks<ASSIGN, BS>(S, [&](int c, int a, int L, int64_t sr) {
         double y[BS];
         sell_row64<BS, C16, LOOP>(S, val, h, L, sr, lane, a, y);
-        if (a >= 0) {
+        if (sell_reduce<BS, T>(y, a, lane)) {
 #pragma unroll
-            for (int m = 0; m < BS; ++m) {
-                const int64_t i = (int64_t)BS * a + m;
+            for (int m = 0; m < (T == 1 ? BS : 1); ++m) {
+                const int64_t i = sell_dof<BS, T>(a, lane) + m;
                 q[i] = y[m];
                 hq = fma(h[i], y[m], hq);
             }
@@ -472,7 +471,7 @@ __device__ __forceinline__ bool fused_prologue(KrylovScalars *ks, const double *
 }
 
 template <bool C16, int ASSIGN>
-__global__ void __launch_bounds__(kSpmvWarps * 32) cg_kca_sell(SellArgs S, const double *__restrict__ val,
+__global__ void __launch_bounds__(sell_threads(1, ASSIGN)) cg_kca_sell(SellArgs S, const double *__restrict__ val,
                                                                const double *__restrict__ hold,
                                                                const double *__restrict__ cgv,
                                                                const double *__restrict__ g,
@@ -488,7 +487,7 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) cg_kca_sell(SellArgs S, const
     if (!fused_prologue(ks, partb, nbb, parity, cond, in_graph, sh, &bc, &gamma)) return;
     const int lane = threadIdx.x & 31;
     double hq = 0, gh = 0;
-    sell_for_chunks<ASSIGN>(S, [&](int c, int a, int L, int64_t sr) {
+    sell_for_chunks<ASSIGN, 1>(S, [&](int c, int a, int L, int64_t sr) {
         const int ar = a < 0 ? 0 : a;
         const int64_t ce = sr * 32 + lane;
         const double *v = val + sr * 32 + lane;
@@ -577,8 +576,8 @@ __global__ void cg_fuse_start(KrylovScalars *ks) {
 }
 
 // double-float: AH = A H from the split H, (H, AH) in FP64
-template <int BS, bool C16, int ASSIGN, bool DEEP>
-__global__ void __launch_bounds__(kSpmvWarps * 32) cg_kax_sell(SellArgs S, const float2 *__restrict__ val,
+template <int BS, bool C16, int ASSIGN, bool DEEP, int T = 1>
+__global__ void __launch_bounds__(sell_threads(BS, ASSIGN)) cg_kax_sell(SellArgs S, const float2 *__restrict__ val,
                                                                const float2 *__restrict__ hx,
                                                                const double *__restrict__ h, double *__restrict__ q,
                                                                KrylovScalars *ks, double *part) {
@@ -587,13 +586,13 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) cg_kax_sell(SellArgs S, const
     if (ks->done) return;
     const int lane = threadIdx.x & 31;
     double hq = 0;
-    sell_for_chunks<ASSIGN>(S, [&](int c, int a, int L, int64_t sr) {
+    sell_for_chunks<ASSIGN, BS>(S, [&](int c, int a, int L, int64_t sr) {
         double y[BS];
         sell_rowx<BS, C16, DEEP>(S, val, hx, L, sr, lane, a, y);
-        if (a >= 0) {
+        if (sell_reduce<BS, T>(y, a, lane)) {
 #pragma unroll
-            for (int m = 0; m < BS; ++m) {
-                const int64_t i = (int64_t)BS * a + m;
+            for (int m = 0; m < (T == 1 ? BS : 1); ++m) {
+                const int64_t i = sell_dof<BS, T>(a, lane) + m;
                 q[i] = y[m];
                 hq = fma(h[i], y[m], hq);
             }
@@ -608,16 +607,16 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) cg_kax_sell(SellArgs S, const
 }
 
 // y = A x (FP64)
-template <int BS, bool C16, int ASSIGN, int LOOP>
-__global__ void __launch_bounds__(kSpmvWarps * 32) spmv_sell(SellArgs S, const double *__restrict__ val,
+template <int BS, bool C16, int ASSIGN, int LOOP, int T = 1>
+__global__ void __launch_bounds__(sell_threads(BS, ASSIGN)) spmv_sell(SellArgs S, const double *__restrict__ val,
                                                              const double *__restrict__ x, double *__restrict__ y) {
     const int lane = threadIdx.x & 31;
-    sell_for_chunks<ASSIGN>(S, [&](int c, int a, int L, int64_t sr) {
+    sell_for_chunks<ASSIGN, BS>(S, [&](int c, int a, int L, int64_t sr) {
         double r[BS];
         sell_row64<BS, C16, LOOP>(S, val, x, L, sr, lane, a, r);
-        if (a >= 0) {
+        if (sell_reduce<BS, T>(r, a, lane)) {
 #pragma unroll
-            for (int m = 0; m < BS; ++m) y[(int64_t)BS * a + m] = r[m];
+            for (int m = 0; m < (T == 1 ? BS : 1); ++m) y[sell_dof<BS, T>(a, lane) + m] = r[m];
         }
     });
 }
@@ -765,41 +764,41 @@ constexpr int kSellCode = 64;
 static bool is_sell(int T) { return T >= kSellCode && T < kSellCode + 8; }
 static int sell_assign(int T) { return (T - kSellCode) & 1; }
 static const char *sell_name(int T) {
-    static const char *names[8] = {"sell32 ranges", "sell32 rotated", "sell32 ranges deep", "sell32 rotated deep",
-                                   "sell32 ranges batch", "sell32 rotated batch", "sell32 ranges batch deep",
-                                   "sell32 rotated batch deep"};
+    static const char *names[8] = {"sell32 ranges", "sell32 stride", "sell32 ranges deep", "sell32 stride deep",
+                                   "sell32 ranges batch", "sell32 stride batch", "sell32 ranges batch deep",
+                                   "sell32 stride batch deep"};
     return names[T - kSellCode];
 }
 
-#define FFGPU_SELL_FN(K)                                                                             \
-    static void *K##_fn(int bs, bool c16, int code) {                                               \
-        void *t[3][4] = {{(void *)K<1, false, 0, false>, (void *)K<1, false, 1, false>,               \
-                          (void *)K<1, false, 0, true>, (void *)K<1, false, 1, true>},                \
-                         {(void *)K<1, true, 0, false>, (void *)K<1, true, 1, false>,                 \
-                          (void *)K<1, true, 0, true>, (void *)K<1, true, 1, true>},                  \
-                         {(void *)K<3, false, 0, false>, (void *)K<3, false, 1, false>,               \
-                          (void *)K<3, false, 0, true>, (void *)K<3, false, 1, true>}};               \
-        return t[bs == 3 ? 2 : (c16 ? 1 : 0)][code - kSellCode];                                     \
-    }
-FFGPU_SELL_FN(cg_kax_sell)
-#undef FFGPU_SELL_FN
+// kernel of a code by block format: scalar with 32- and 16-bit columns, 3x3 blocks with one and four
+// lanes per row
+static int sell_format(const ffgpu_matrix *A) {
+    return A->bs == 3 ? (sell_lanes(A) == 4 ? 3 : 2) : (A->scol16 ? 1 : 0);
+}
+#define FFGPU_SELL_ROW(K, BS, C16, T)                                                                  \
+    {(void *)K<BS, C16, 0, false, T>, (void *)K<BS, C16, 1, false, T>, (void *)K<BS, C16, 0, true, T>,  \
+     (void *)K<BS, C16, 1, true, T>}
+static void *cg_kax_sell_fn(const ffgpu_matrix *A, int code) {
+    static void *const t[4][4] = {FFGPU_SELL_ROW(cg_kax_sell, 1, false, 1), FFGPU_SELL_ROW(cg_kax_sell, 1, true, 1),
+                                  FFGPU_SELL_ROW(cg_kax_sell, 3, false, 1), FFGPU_SELL_ROW(cg_kax_sell, 3, false, 4)};
+    return t[sell_format(A)][code - kSellCode];
+}
+#undef FFGPU_SELL_ROW
 // FP64 kernels: the four row loops
-#define FFGPU_SELL64_FN(K)                                                                           \
-    static void *K##_fn(int bs, bool c16, int code) {                                               \
-        void *t[3][8] = {{(void *)K<1, false, 0, 0>, (void *)K<1, false, 1, 0>, (void *)K<1, false, 0, 1>,   \
-                          (void *)K<1, false, 1, 1>, (void *)K<1, false, 0, 2>, (void *)K<1, false, 1, 2>,   \
-                          (void *)K<1, false, 0, 3>, (void *)K<1, false, 1, 3>},                          \
-                         {(void *)K<1, true, 0, 0>, (void *)K<1, true, 1, 0>, (void *)K<1, true, 0, 1>,      \
-                          (void *)K<1, true, 1, 1>, (void *)K<1, true, 0, 2>, (void *)K<1, true, 1, 2>,      \
-                          (void *)K<1, true, 0, 3>, (void *)K<1, true, 1, 3>},                            \
-                         {(void *)K<3, false, 0, 0>, (void *)K<3, false, 1, 0>, (void *)K<3, false, 0, 1>,   \
-                          (void *)K<3, false, 1, 1>, (void *)K<3, false, 0, 2>, (void *)K<3, false, 1, 2>,   \
-                          (void *)K<3, false, 0, 3>, (void *)K<3, false, 1, 3>}};                         \
-        return t[bs == 3 ? 2 : (c16 ? 1 : 0)][code - kSellCode];                                     \
+#define FFGPU_SELL64_ROW(K, BS, C16, T)                                                               \
+    {(void *)K<BS, C16, 0, 0, T>, (void *)K<BS, C16, 1, 0, T>, (void *)K<BS, C16, 0, 1, T>,            \
+     (void *)K<BS, C16, 1, 1, T>, (void *)K<BS, C16, 0, 2, T>, (void *)K<BS, C16, 1, 2, T>,            \
+     (void *)K<BS, C16, 0, 3, T>, (void *)K<BS, C16, 1, 3, T>}
+#define FFGPU_SELL64_FN(K)                                                                            \
+    static void *K##_fn(const ffgpu_matrix *A, int code) {                                            \
+        static void *const t[4][8] = {FFGPU_SELL64_ROW(K, 1, false, 1), FFGPU_SELL64_ROW(K, 1, true, 1),   \
+                                      FFGPU_SELL64_ROW(K, 3, false, 1), FFGPU_SELL64_ROW(K, 3, false, 4)}; \
+        return t[sell_format(A)][code - kSellCode];                                                    \
     }
 FFGPU_SELL64_FN(cg_ka_sell)
 FFGPU_SELL64_FN(spmv_sell)
 #undef FFGPU_SELL64_FN
+#undef FFGPU_SELL64_ROW
 
 // lanes per block row of the block-CSR kernels
 static int pick_lanes(const ffgpu_matrix *A) {
@@ -863,7 +862,7 @@ static SpmvArgs spmv_args(const ffgpu_matrix *A, int trans) {
 // One K_a launch of the CG loop, with its argument storage.
 struct KaCall {
     void *fn = nullptr;
-    int grid = 0;
+    int grid = 0, threads = kSpmvWarps * 32;
     SpmvArgs sa;
     SpmvArgsX sx;
     SellArgs sl;
@@ -876,34 +875,41 @@ struct KaCall {
     double *part = nullptr;
     void *args[7];
     cudaError_t launch(cudaStream_t s, bool pdl = false) {
-        return launch_ex(fn, grid, kSpmvWarps * 32, args, 0, s, pdl);
+        return launch_ex(fn, grid, threads, args, 0, s, pdl);
     }
 };
+
+// grid of a SELL kernel of this assignment, and its partition for ranges
+static int sell_launch_shape(ffgpu_matrix *A, const void *fn, int assign, SellArgs &sl, int *grid, int *threads) {
+    *threads = sell_threads(A->bs, assign);
+    *grid = A->bs == 3 && assign == kSellStride
+                ? sell_spread_grid(A->nchunk)
+                : sized_grid(fn, *threads, ((int64_t)A->nchunk + kSpmvWarps - 1) / kSpmvWarps);
+    if (assign == kSellStride) return FFGPU_OK;
+    return sell_partition(A, *grid * kSpmvWarps, &sl.part);
+}
 
 // K_a for mode (0 FP64, 1 double-float) and layout choice T (SELL-32 codes or BSR lanes)
 static int ka_setup(ffgpu_matrix *A, int mode, int trans, int T, const double *h, double *q, KaCall &k) {
     k.h = h; k.q = q; k.ks = A->ks; k.part = A->ctx->d_part; k.hx = A->hx;
     if (is_sell(T)) {
         FFGPU_TRY(sell_values(A, mode == 1 ? (trans ? kSellXT : kSellX) : (trans ? kSell64T : kSell64)));
-        // the column format is known only once the layout exists
-        const bool c16 = A->scol16 != nullptr;
-        const bool range = sell_assign(T) == kSellRanges;
+        // (the column format is known only once the layout exists)
         k.sl = sell_args(A);
         if (mode == 1) {
             k.vx = trans ? A->svalx_t : A->svalx;
-            k.fn = cg_kax_sell_fn(A->bs, c16, T);
+            k.fn = cg_kax_sell_fn(A, T);
             k.args[0] = &k.sl; k.args[1] = &k.vx; k.args[2] = &k.hx; k.args[3] = &k.h; k.args[4] = &k.q;
             k.args[5] = &k.ks; k.args[6] = &k.part;
         } else {
             k.v64 = trans ? A->sval_t : A->sval;
-            k.fn = cg_ka_sell_fn(A->bs, c16, T);
+            k.fn = cg_ka_sell_fn(A, T);
             k.args[0] = &k.sl; k.args[1] = &k.v64; k.args[2] = &k.h; k.args[3] = &k.q; k.args[4] = &k.ks;
             k.args[5] = &k.part;
         }
-        k.grid = sized_grid(k.fn, kSpmvWarps * 32, ((int64_t)A->nchunk + kSpmvWarps - 1) / kSpmvWarps);
-        if (range) FFGPU_TRY(sell_partition(A, k.grid * kSpmvWarps, &k.sl.part));
-        return FFGPU_OK;
+        return sell_launch_shape(A, k.fn, sell_assign(T), k.sl, &k.grid, &k.threads);
     }
+    k.threads = kSpmvWarps * 32;
     if (mode == 1) {
         FFGPU_TRY(matrix_prepare_split(A, trans));
         k.sx = SpmvArgsX{A->nb, A->bs, A->browptr, A->bcol, trans ? A->valx_t : A->valx, A->rowperm};
@@ -1039,12 +1045,11 @@ int spmv(ffgpu_matrix *A, const double *x, double *y, int trans, cudaStream_t st
     if (sv) {
         SellArgs sl = sell_args(A);
         const int code = is_sell(A->csr_lanes) ? A->csr_lanes : kSellCode;
-        const bool range = sell_assign(code) == kSellRanges;
-        void *fn = spmv_sell_fn(A->bs, A->scol16 != nullptr, code);
-        const int grid = sized_grid(fn, kSpmvWarps * 32, ((int64_t)A->nchunk + kSpmvWarps - 1) / kSpmvWarps);
-        if (range) FFGPU_TRY(sell_partition(A, grid * kSpmvWarps, &sl.part));
+        void *fn = spmv_sell_fn(A, code);
+        int grid = 0, threads = 0;
+        FFGPU_TRY(sell_launch_shape(A, fn, sell_assign(code), sl, &grid, &threads));
         void *args[] = {&sl, &sv, &x, &y};
-        FFGPU_CUDA(cudaLaunchKernel(fn, grid, kSpmvWarps * 32, args, 0, st));
+        FFGPU_CUDA(cudaLaunchKernel(fn, grid, threads, args, 0, st));
         return launch_check(A->ctx, "spmv");
     }
     if (trans) FFGPU_TRY(matrix_prepare_transpose(A));
@@ -1168,7 +1173,7 @@ constexpr int64_t kFuseMaxEntries = 1 << 20;
 
 struct KcaCall {
     void *fn = nullptr;
-    int grid = 0;
+    int grid = 0, threads = kSpmvWarps * 32;
     SellArgs sl;
     SpmvArgs sa;
     const double *v64 = nullptr, *hold = nullptr, *cgv = nullptr, *g = nullptr;
@@ -1181,7 +1186,7 @@ struct KcaCall {
     int in_graph = 0;
     void *args[14];
     cudaError_t launch(cudaStream_t s, bool pdl = false) {
-        return launch_ex(fn, grid, kSpmvWarps * 32, args, 0, s, pdl);
+        return launch_ex(fn, grid, threads, args, 0, s, pdl);
     }
 };
 
@@ -1226,12 +1231,11 @@ static int kca_setup(ffgpu_matrix *A, int trans, const double *hold, double *hne
     k.fn = c16 ? (assign ? (void *)cg_kca_sell<true, 1> : (void *)cg_kca_sell<true, 0>)
                : (assign ? (void *)cg_kca_sell<false, 1> : (void *)cg_kca_sell<false, 0>);
     k.sl = sell_args(A);
-    k.grid = sized_grid(k.fn, kSpmvWarps * 32, ((int64_t)A->nchunk + kSpmvWarps - 1) / kSpmvWarps);
+    FFGPU_TRY(sell_launch_shape(A, k.fn, assign, k.sl, &k.grid, &k.threads));
     // two partial slots per block in the reduction buffer, then K_b's partials
     FFGPU_CHECK(2 * k.grid + k.nbb <= 4 * kRedBlocks, FFGPU_EINVAL, "fused CG: grid %d above the reduction buffer",
                 k.grid);
     k.partb = k.part + 2 * k.grid;
-    if (assign == kSellRanges) FFGPU_TRY(sell_partition(A, k.grid * kSpmvWarps, &k.sl.part));
     k.v64 = trans ? A->sval_t : A->sval;
     k.args[0] = &k.sl; k.args[1] = &k.v64; k.args[2] = &k.hold; k.args[3] = &k.cgv; k.args[4] = &k.g;
     k.args[5] = &k.hnew; k.args[6] = &k.q; k.args[7] = &k.ks; k.args[8] = &k.part; k.args[9] = &k.partb;
