@@ -50,6 +50,12 @@ struct BatchArgs {
     double eps, tgv;
     float eps_in;
     int itmax_in, max_outer;
+    // packed FP32 rows (batch_sm_kernel): chunks of 32 rows of one problem, a row per lane, padded to
+    // quads of entries and to the longest; quad s of a chunk at (coff[chunk] + s) * 32 + lane
+    const int32_t *pchunk;     // nprob+1: first chunk of each problem
+    const int32_t *coff;       // first quad row of each chunk
+    const float *pval;         // scaled to a unit diagonal
+    const uint16_t *pcol;
 };
 
 template <int NT>
@@ -276,6 +282,188 @@ __global__ void __launch_bounds__(NT) batch_ir_kernel(BatchArgs B) {
     }
 }
 
+// The same solve with the problem's vectors in shared memory -- the direction h (gathered), the
+// gradient g and the correction d -- and q = A h in registers, so that an inner iteration moves only
+// the packed matrix, coalesced, from L2 (6 bytes per entry).  The inner system is scaled to a
+// unit diagonal, S A S with S = C^(1/2): conjugate gradients on it are the Jacobi-preconditioned
+// ones (g here is S g, d is S^-1 d) without 1/A_ii.  The values are rounded to FP32 once, as the unscaled.
+// The kernel above gathers three values per entry through L1 and reads CSR rows, two lanes each.
+// Per inner iteration of the largest problems (N = 128, 16 641 rows): 37 us there, 12.7 us here,
+// and a batch ends when its largest problem does.
+// Thread t owns the rows u * NT + t, chunk u * NT / 32 + warp: the rows its lanes multiply.
+constexpr int kSmRows = 19;        // rows per thread: NT * 19 rows of 12 bytes fill the CTA's share
+template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) batch_sm_kernel(BatchArgs B) {
+    constexpr int NW = NT / 32;
+    extern __shared__ __align__(16) float smv[];
+    __shared__ double sh[33];
+    __shared__ float shf[66];
+    __shared__ int s_p, off[NW * kSmRows + 1];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (;;) {
+        if (threadIdx.x == 0) s_p = atomicAdd(B.queue, 1);
+        __syncthreads();
+        const int slot = s_p;
+        __syncthreads();
+        if (slot >= B.nprob) return;
+        const int p = B.order[slot];
+        const int r0 = B.voff[p], r1 = B.voff[p + 1], n = r1 - r0;
+        const int c0 = B.pchunk[p], nc = B.pchunk[p + 1] - c0, n32 = nc * 32;
+        float *h = smv, *g = smv + n32, *d = g + n32;
+        const float *scale = B.dinv32 + r0;      // S, the square roots
+        for (int i = threadIdx.x; i <= nc; i += NT) off[i] = B.coff[c0 + i];
+        for (int i = threadIdx.x; i < n; i += NT) B.x[r0 + i] = B.wcl[r0 + i] ? B.b[r0 + i] / B.tgv : 0.0;
+        __syncthreads();
+        double eps2 = 0, gcg = 0, gcg0 = 0;
+        int outer = 0, inner = 0, conv = 0;
+        for (outer = 0; outer <= B.max_outer; ++outer) {
+            cta_spmv64<NT, 2, true>(B, r0, r1, B.x, B.r);
+            __syncthreads();
+            double s64 = 0;
+            float sa = 0;
+            for (int i = threadIdx.x; i < n32; i += NT) {
+                float gi = 0.f;
+                if (i < n) {
+                    const double ri = B.b[r0 + i] - B.r[r0 + i];
+                    s64 = fma(ri, B.dinv[r0 + i] * ri, s64);
+                    gi = -(float)ri * scale[i];
+                    sa = fmaf(gi, gi, sa);
+                }
+                g[i] = gi;
+                d[i] = 0.0f;
+                h[i] = 0.0f;    // first direction -g: gamma 0
+            }
+            gcg = cta_sum<NT>(s64, sh);
+            if (outer == 0) {
+                gcg0 = gcg;
+                eps2 = B.eps > 0 ? B.eps * B.eps * gcg : B.eps * B.eps;
+                if (gcg < 1e-30) { conv = 1; break; }
+            }
+            if (gcg < eps2) { conv = 1; break; }
+            if (outer == B.max_outer) break;
+            float ig = cta_sum_f<NT>(sa, shf);
+            float s_gh = -ig, gamma = 0.0f;
+            const float ieps2 = B.eps_in * B.eps_in * ig;
+            for (int it = 0; it < B.itmax_in && ig >= 1e-30f && ig >= ieps2; ++it) {
+                for (int i = threadIdx.x; i < n32; i += NT) h[i] = fmaf(gamma, h[i], -g[i]);
+                __syncthreads();
+                // q = A h, (h, q); two quads (eight slots) in flight per warp and chunk
+                float q[kSmRows];
+                float hq = 0;
+#pragma unroll
+                for (int u = 0; u < kSmRows; ++u) {
+                    const int c = u * NW + w;
+                    if (c >= nc) break;
+                    const int s0 = off[c], L = off[c + 1] - s0;
+                    const float4 *v = reinterpret_cast<const float4 *>(B.pval) + (int64_t)s0 * 32 + lane;
+                    const uint2 *k = reinterpret_cast<const uint2 *>(B.pcol) + (int64_t)s0 * 32 + lane;
+                    float y = 0.f;
+                    for (int j = 0; j < L; j += 2) {
+                        const bool two = j + 1 < L;
+                        const float4 a0 = __ldg(v + j * 32);
+                        const uint2 k0 = __ldg(k + j * 32);
+                        float4 a1 = make_float4(0.f, 0.f, 0.f, 0.f);
+                        uint2 k1 = make_uint2(0u, 0u);
+                        if (two) { a1 = __ldg(v + j * 32 + 32); k1 = __ldg(k + j * 32 + 32); }
+                        y = fmaf(a0.x, h[k0.x & 0xffffu], y);
+                        y = fmaf(a0.y, h[k0.x >> 16], y);
+                        y = fmaf(a0.z, h[k0.y & 0xffffu], y);
+                        y = fmaf(a0.w, h[k0.y >> 16], y);
+                        if (two) {
+                            y = fmaf(a1.x, h[k1.x & 0xffffu], y);
+                            y = fmaf(a1.y, h[k1.x >> 16], y);
+                            y = fmaf(a1.z, h[k1.y & 0xffffu], y);
+                            y = fmaf(a1.w, h[k1.y >> 16], y);
+                        }
+                    }
+                    q[u] = y;
+                    hq = fmaf(h[c * 32 + lane], y, hq);
+                }
+                hq = cta_sum_f<NT>(hq, shf);
+                const float rho = -s_gh / hq;
+                float sg = 0, sgh = 0;
+#pragma unroll
+                for (int u = 0; u < kSmRows; ++u) {
+                    if (u * NW + w >= nc) break;
+                    const int i = u * NT + threadIdx.x;
+                    const float hv = h[i], gi = fmaf(rho, q[u], g[i]);
+                    d[i] = fmaf(rho, hv, d[i]);
+                    g[i] = gi;
+                    sg = fmaf(gi, gi, sg);
+                    sgh = fmaf(gi, hv, sgh);
+                }
+                // (g, Cg) and (g, h): the next direction's (g, gamma h - Cg) follows from them
+                const float2 t = cta_sum2_f<NT>(sg, sgh, shf);
+                gamma = t.x / ig;
+                ig = t.x;
+                s_gh = fmaf(gamma, t.y, -t.x);
+                ++inner;
+                if (!(ig == ig)) break;
+            }
+            for (int i = threadIdx.x; i < n; i += NT) B.x[r0 + i] += (double)(d[i] * scale[i]);
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+            B.iters[p] = inner;
+            B.outers[p] = outer;
+            B.conv[p] = conv;
+            B.resid[p] = gcg0 > 0 ? sqrt(gcg / gcg0) : 0.0;
+        }
+        __syncthreads();
+    }
+}
+
+// quads of each chunk: those of the longest of its (up to) 32 rows
+__global__ void batch_len_kernel(int nchunk, int nprob, const int32_t *__restrict__ pchunk, const int32_t *__restrict__ voff,
+                                 const int32_t *__restrict__ rp, int32_t *__restrict__ len) {
+    const int lane = threadIdx.x & 31;
+    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nchunk; c += (gridDim.x * blockDim.x) >> 5) {
+        int lo = 0, hi = nprob;   // pchunk[lo] <= c < pchunk[hi]
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (pchunk[mid] <= c) lo = mid; else hi = mid;
+        }
+        const int r = voff[lo] + (c - pchunk[lo]) * 32 + lane;
+        const int L = __reduce_max_sync(0xffffffffu, r < voff[lo + 1] ? rp[r + 1] - rp[r] : 0);
+        if (lane == 0) len[c] = (L + 3) / 4;
+    }
+}
+
+// packed rows: the scaled values S A S (the products and square roots in FP64, one rounding to FP32) and, with
+// the pattern's first assembly, columns within the problem
+__global__ void batch_pack_kernel(int nchunk, int nprob, const int32_t *__restrict__ pchunk,
+                                  const int32_t *__restrict__ voff, const int32_t *__restrict__ rp,
+                                  const int32_t *__restrict__ col, const double *__restrict__ val,
+                                  const double *__restrict__ root, const int32_t *__restrict__ coff, float *__restrict__ pval, uint16_t *__restrict__ pcol) {
+    const int lane = threadIdx.x & 31;
+    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nchunk; c += (gridDim.x * blockDim.x) >> 5) {
+        int lo = 0, hi = nprob;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (pchunk[mid] <= c) lo = mid; else hi = mid;
+        }
+        const int r0 = voff[lo], r = r0 + (c - pchunk[lo]) * 32 + lane;
+        const int b = r < voff[lo + 1] ? rp[r] : 0, deg = r < voff[lo + 1] ? rp[r + 1] - b : 0;
+        const int s0 = coff[c], L = coff[c + 1] - s0;
+        const double si = deg ? root[r] : 0.0;
+        for (int j = 0; j < 4 * L; ++j) {
+            const int64_t at = ((int64_t)(s0 + (j >> 2)) * 32 + lane) * 4 + (j & 3);
+            const int k = j < deg ? col[b + j] : r0;
+            pval[at] = j < deg ? (float)(si * val[b + j] * root[k]) : 0.0f;
+            if (pcol) pcol[at] = (uint16_t)(k - r0);
+        }
+    }
+}
+
+// S = C^(1/2) in FP64 for the packed values and in FP32 for the solver's vectors
+__global__ void root_kernel(int64_t n, const double *dinv, double *root, float *root32) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double s = sqrt(dinv[i]);
+        root[i] = s;
+        root32[i] = (float)s;
+    }
+}
+
 __global__ void f32_copy_kernel(int64_t n, const double *a, float *b) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         b[i] = (float)a[i];
@@ -343,6 +531,12 @@ struct ffgpu_batch {
     int *queue, *iters, *outers, *conv;
     double *resid;
     uint16_t *col16;    // problem-local columns (null when a problem has 65 536 DOFs or more)
+    int nchunk;         // chunks of the packed rows (0: a problem is too large for shared memory)
+    int max_rows32;     // rows of the largest problem, padded to chunks
+    int32_t *pchunk, *coff;
+    float *pval;
+    uint16_t *pcol;
+    int64_t nslot;
     bool local16;       // every problem below 65 536 DOFs: the 16-bit column kernels
     int tuned;          // index of the chosen candidate, -1 before tuning
     cudaGraphExec_t exec;
@@ -351,16 +545,37 @@ struct ffgpu_batch {
 };
 
 // tuner candidates: the first kBatchSet with 32-bit global columns, the next kBatchSet with
-// 16-bit problem-local columns (the same shapes)
+// 16-bit problem-local columns (the same shapes); then the shared-memory kernels, of which those
+// whose share of an SM's shared memory holds the largest problem are timed.  Where one does, the
+// others are not: 1024 jittered squares 100 against 32 ms, 200 of them 37.4 against 12.7 ms.
 #define FFGPU_BATCH_SET(C16)                                                                          \
     {batch_ir_kernel<256, 2, C16>, 256, 2, 4}, {batch_ir_kernel<256, 4, C16>, 256, 4, 4},             \
         {batch_ir_kernel<512, 2, C16>, 512, 2, 2}, {batch_ir_kernel<512, 4, C16>, 512, 4, 2},         \
         {batch_ir_kernel<1024, 2, C16>, 1024, 2, 1}, {batch_ir_kernel<1024, 4, C16>, 1024, 4, 1},     \
         {batch_ir_kernel<128, 2, C16>, 128, 2, 8}
-static Candidate g_cands[] = {FFGPU_BATCH_SET(false), FFGPU_BATCH_SET(true)};
+static Candidate g_cands[] = {FFGPU_BATCH_SET(false), FFGPU_BATCH_SET(true), {batch_sm_kernel<1024>, 1024, 2, 1},
+                              {batch_sm_kernel<512>, 512, 2, 2}, {batch_sm_kernel<256>, 256, 2, 4}};   // (lanes: the FP64 residual's)
 #undef FFGPU_BATCH_SET
-constexpr int kBatchSet = 7;
-static_assert(sizeof(g_cands) / sizeof(g_cands[0]) == 2 * kBatchSet, "batched tuner: candidate sets");
+constexpr int kBatchSet = 7, kBatchSm = 3;
+static_assert(sizeof(g_cands) / sizeof(g_cands[0]) == 2 * kBatchSet + kBatchSm, "batched tuner: candidate sets");
+// dynamic shared memory of a CTA when per_sm of them share an SM's 228 KB (1 KB a CTA taken by the
+// system, up to 3 KB by the static arrays)
+static size_t batch_smem_cap(int per_sm) { return (size_t)(228 / per_sm - 4) * 1024; }
+// whether a problem of `rows` padded rows fits a candidate: h, g, d in shared memory, q in registers
+static bool batch_sm_fits(int rows, int nt, int per_sm) {
+    return (size_t)rows * 12 <= batch_smem_cap(per_sm) && rows <= nt * kSmRows;
+}
+// the candidates of a batch: [first, last)
+static void batch_cands(bool local16, int nchunk, int max_rows32, int *first, int *last) {
+    if (nchunk > 0) {
+        *first = 2 * kBatchSet;
+        *last = *first + 1;
+        while (*last < 2 * kBatchSet + kBatchSm && batch_sm_fits(max_rows32, g_cands[*last].nt, g_cands[*last].per_sm)) ++*last;
+        return;
+    }
+    *first = local16 ? kBatchSet : 0;
+    *last = *first + kBatchSet;
+}
 
 static int batch_graph(ffgpu_batch *B, int cand) {
     ffgpu_ctx *ctx = B->ctx;
@@ -368,11 +583,16 @@ static int batch_graph(ffgpu_batch *B, int cand) {
     if (B->exec) { cudaGraphExecDestroy(B->exec); B->exec = nullptr; }
     const Candidate &c = g_cands[cand];
     int grid = kNumSM * c.per_sm;
+    size_t smem = 0;
+    if (cand >= 2 * kBatchSet) {
+        smem = (size_t)B->max_rows32 * 12;
+        FFGPU_CUDA(cudaFuncSetAttribute((const void *)c.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    }
     cudaGraph_t g;
     FFGPU_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     reset_queue_kernel<<<1, 1, 0, s>>>(B->queue);
     void *args[] = {&B->args};
-    cudaLaunchKernel((void *)c.k, grid, c.nt, args, 0, s);
+    cudaLaunchKernel((void *)c.k, grid, c.nt, args, smem, s);
     cudaError_t e = cudaStreamEndCapture(s, &g);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&B->exec, g, 0);
     if (e == cudaSuccess) cudaGraphDestroy(g);
@@ -449,8 +669,10 @@ static int batch_create(ffgpu_ctx *ctx, int nprob, const int32_t *nv, const int3
     }
     ffgpu_batch *B = new ffgpu_batch();
     B->ctx = ctx; B->nprob = nprob; B->voff_h = voff; B->space = nullptr; B->A = nullptr; B->tuned = -1;
-    B->exec = nullptr; B->b = nullptr; B->work32 = nullptr; B->r = nullptr; B->dinv32 = nullptr;
+    B->tuned_ms = 0; B->exec = nullptr; B->b = nullptr; B->work32 = nullptr; B->r = nullptr; B->dinv32 = nullptr;
     B->col16 = nullptr;
+    B->pchunk = B->coff = nullptr; B->pval = nullptr; B->pcol = nullptr; B->nchunk = 0; B->nslot = 0;
+    B->max_rows32 = (*std::max_element(nv, nv + nprob) + 31) / 32 * 32;
     B->local16 = *std::max_element(nv, nv + nprob) < 65536;
     // P1: the DOFs are the vertices (no DOF table)
     int rc = ffgpu_space_create(ctx, 2, NV, coords, NT, d_el, FFGPU_FE_P1, 3, nullptr, NV, &B->space);
@@ -473,6 +695,18 @@ static int batch_create(ffgpu_ctx *ctx, int nprob, const int32_t *nv, const int3
     }
     B->dinv32 = B->work32 + (size_t)4 * NV;
     cudaMemcpy(B->voff, voff.data(), sizeof(int32_t) * (nprob + 1), cudaMemcpyHostToDevice);
+    if (B->local16 && batch_sm_fits(B->max_rows32, 1024, 1)) {
+        std::vector<int32_t> pchunk(nprob + 1, 0);
+        for (int p = 0; p < nprob; ++p) pchunk[p + 1] = pchunk[p] + (nv[p] + 31) / 32;
+        B->nchunk = pchunk[nprob];
+        if (dalloc(ctx, (void **)&B->pchunk, sizeof(int32_t) * (nprob + 1)) ||
+            dalloc(ctx, (void **)&B->coff, sizeof(int32_t) * ((size_t)B->nchunk + 1))) {
+            set_error("ffgpu_batch_create: device allocation failed");
+            ffgpu_batch_destroy(B);
+            return FFGPU_ENOMEM;
+        }
+        FFGPU_CUDA(cudaMemcpyAsync(B->pchunk, pchunk.data(), sizeof(int32_t) * (nprob + 1), cudaMemcpyHostToDevice, s));
+    }
     cudaMemcpy(B->order, order.data(), sizeof(int32_t) * nprob, cudaMemcpyHostToDevice);
     *out = B;
     return FFGPU_OK;
@@ -494,21 +728,50 @@ int ffgpu_batch_assemble(ffgpu_batch *B, const double *kappa, double f, const ui
     }
     ffgpu_matrix *A = B->A;
     FFGPU_TRY(matrix_prepare_solver(A));
-    FFGPU_TRY(ffgpu_matrix_to_f32(A));
     cudaStream_t s = B->ctx->stream;
+    if (B->nchunk > 0) {
+        const int grid = std::min(16 * kNumSM, (B->nchunk + 7) / 8);
+        const bool first = !B->pval;
+        if (first) {
+            // the pattern is fixed by the first assembly: chunk lengths, offsets, columns
+            int32_t *len = nullptr;
+            FFGPU_CUDA(dalloc(B->ctx, (void **)&len, sizeof(int32_t) * (size_t)B->nchunk));
+            batch_len_kernel<<<grid, 256, 0, s>>>(B->nchunk, B->nprob, B->pchunk, B->voff, A->browptr, len);
+            int rc = launch_check(B->ctx, "batch_len");
+            if (!rc) rc = device_scan_i32(B->ctx, len, B->coff, B->nchunk);
+            int32_t nslot = 0;
+            cudaMemcpyAsync(&nslot, B->coff + B->nchunk, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+            dfree(B->ctx, len);
+            FFGPU_TRY(rc);
+            FFGPU_CUDA(cudaStreamSynchronize(s));
+            B->nslot = nslot;
+            FFGPU_CUDA(dalloc(B->ctx, (void **)&B->pcol, sizeof(uint16_t) * 128 * (size_t)nslot));
+            FFGPU_CUDA(dalloc(B->ctx, (void **)&B->pval, sizeof(float) * 128 * (size_t)nslot));
+        }
+        root_kernel<<<4 * kNumSM, 256, 0, s>>>(A->n, A->diag_inv, B->r, B->dinv32);   // r: free until the solve
+        FFGPU_TRY(launch_check(B->ctx, "batch_root"));
+        batch_pack_kernel<<<grid, 256, 0, s>>>(B->nchunk, B->nprob, B->pchunk, B->voff, A->browptr, A->bcol, A->val, B->r,
+                                               B->coff, B->pval, first ? B->pcol : nullptr);
+        FFGPU_TRY(launch_check(B->ctx, "batch_pack"));
+    } else {
+        FFGPU_TRY(ffgpu_matrix_to_f32(A));
+    }
     if (B->local16 && !B->col16) {
         // the pattern is fixed by the first assembly: number its columns within their problems
         FFGPU_CUDA(dalloc(B->ctx, (void **)&B->col16, sizeof(uint16_t) * std::max<int64_t>(A->nnz, 1)));
         local_col_kernel<<<4 * kNumSM, 256, 0, s>>>(A->n, B->nprob, B->voff, A->browptr, A->bcol, B->col16);
         FFGPU_TRY(launch_check(B->ctx, "local_col"));
     }
-    f32_copy_kernel<<<4 * kNumSM, 256, 0, s>>>(A->n, A->diag_inv, B->dinv32);
-    FFGPU_TRY(launch_check(B->ctx, "f32_copy"));
+    if (B->nchunk == 0) {
+        f32_copy_kernel<<<4 * kNumSM, 256, 0, s>>>(A->n, A->diag_inv, B->dinv32);
+        FFGPU_TRY(launch_check(B->ctx, "f32_copy"));
+    }
     float *w = B->work32;
     size_t NV = A->n;
     B->args = BatchArgs{B->nprob, B->order, B->voff, A->browptr, A->bcol, B->col16, A->val, A->val32, A->diag_inv,
                         B->dinv32, A->wcl, B->b, nullptr, w, w + NV, w + 2 * NV, w + 3 * NV, w + 5 * NV, B->r, B->queue,
-                        B->iters, B->outers, B->conv, B->resid, 1e-8, tgv > 0 ? tgv : 1e30, 1e-4f, 0, 30};
+                        B->iters, B->outers, B->conv, B->resid, 1e-8, tgv > 0 ? tgv : 1e30, 1e-4f, 0, 30,
+                        B->pchunk, B->coff, B->pval, B->pcol};
     FFGPU_CUDA(cudaStreamSynchronize(s));
     return FFGPU_OK;
 }
@@ -535,17 +798,20 @@ int ffgpu_batch_solve(ffgpu_batch *B, double *x, const ffgpu_ir_params *prm, int
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
+    int first = 0, last = 0;
+    batch_cands(B->local16, B->nchunk, B->max_rows32, &first, &last);
     if (B->tuned < 0)
         for (const ffgpu_ctx::BatchTuned &t : ctx->btuned)
-            if (t.nprob == B->nprob && t.n == NV && t.nnz == B->A->nnz && (t.cand >= kBatchSet) == B->local16)
+            if (t.nprob == B->nprob && t.n == NV && t.nnz == B->A->nnz && t.cand >= first && t.cand < last)
                 B->tuned = t.cand;
+    if (B->tuned < 0 && last == first + 1) B->tuned = first;
     if (B->tuned < 0) {
         // autotune: time every candidate (CTA size x lanes per row) on this batch and keep the
         // first one within the tuner margin of the fastest; the choice is kept in the context
         // for later batches of the same shape
-        const int base = B->local16 ? kBatchSet : 0;
+        const int base = first, count = last - first;
         float tms[kBatchSet];
-        for (int c = 0; c < kBatchSet; ++c) {
+        for (int c = 0; c < count; ++c) {
             FFGPU_TRY(batch_graph(B, base + c));
             cudaGraphLaunch(B->exec, s);   // warm
             cudaEventRecord(e0, s);
@@ -560,7 +826,7 @@ int ffgpu_batch_solve(ffgpu_batch *B, double *x, const ffgpu_ir_params *prm, int
                 fprintf(stderr, "ffgpu: batch tuner <%d threads, %d lanes, %d CTAs>: %.3f ms\n", g_cands[base + c].nt,
                         g_cands[base + c].lanes, kNumSM * g_cands[base + c].per_sm, ms);
         }
-        const int bi = base + tuned_pick(tms, kBatchSet);
+        const int bi = base + tuned_pick(tms, count);
         B->tuned = bi;
         B->tuned_ms = tms[bi - base];
         changed = true;
@@ -575,6 +841,7 @@ int ffgpu_batch_solve(ffgpu_batch *B, double *x, const ffgpu_ir_params *prm, int
     FFGPU_CUDA(cudaEventSynchronize(e1));
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
+    if (!(B->tuned_ms > 0)) B->tuned_ms = ms;   // nothing was timed: one candidate, or known from the context
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     std::vector<int> it(B->nprob), ou(B->nprob), cv(B->nprob);
@@ -626,6 +893,7 @@ int ffgpu_batch_destroy(ffgpu_batch *B) {
     cudaFree(B->voff); cudaFree(B->order); cudaFree(B->queue); cudaFree(B->iters); cudaFree(B->outers);
     cudaFree(B->conv); cudaFree(B->resid); cudaFree(B->b); cudaFree(B->r); cudaFree(B->work32);
     dfree(B->ctx, B->col16);
+    dfree(B->ctx, B->pchunk); dfree(B->ctx, B->coff); dfree(B->ctx, B->pval); dfree(B->ctx, B->pcol);
     delete B;
     return FFGPU_OK;
 }
