@@ -22,12 +22,17 @@
 // matrices are therefore the exact contraction of the rounded features (relative error below
 // 2^-53 of the element's largest feature), and exactly symmetric.
 //
-// Tile: the A operand is M (128 rows: the (I <= J) pairs, 55 on tetrahedra, 21 on triangles,
-// the rest zero; K = 16), the B operand the digit tiles (N = 48 feature rows per digit: 3
-// elasticity elements x 16 rows (9 used) or 48 scalar elements), the accumulators D[pair][row]
-// five 48-column blocks of TMEM (256 columns allocated, two CTAs per SM).  Persistent CTAs of
+// Tile: the A operand is M (128 rows: the (I <= J) pairs, 55 on tetrahedra and 21 on triangles, in
+// two or four copies, the rest zero; K = 16), the B operand the digit tiles (N = 48 feature rows
+// per digit: 3 elasticity elements x 16 rows (9 used) or 48 scalar elements), the accumulators
+// D[pair][row] five 48-column blocks of TMEM (256 columns allocated, two CTAs per SM).  Persistent CTAs of
 // 128 threads take tiles from a counter; thread 0 issues the five MMAs and commits them to an
 // mbarrier; every wait is bounded in time and a timeout is reported through the status word.
+// The epilogue's conversions and scalings bound it (about 30 FP64 instructions per warp and
+// elasticity element, one per 64 cycles and sub-partition), and a warp may read only its own
+// quarter of the TMEM lanes: with one copy of the pairs two of the four sub-partitions did all of
+// it.  The copies give every warp pairs of its own to finish, for different elements (63 888
+// elasticity elements: 552 -> 508 us).
 #include <cuda_fp16.h>
 
 #include "ffgpu_internal.cuh"
@@ -191,13 +196,15 @@ __global__ void __launch_bounds__(kTcThreads) elem_tc_kernel(int nt, const doubl
     __shared__ int tile_sh, fail_sh;
     const int tid = threadIdx.x, warp = tid >> 5;
 
-    // A operand: row t = pair (I, J), column k = b * NV + b'
+    // A operand: row = copy * SPAN + pair (I, J), column k = b * NV + b'
+    constexpr int SPAN = NP <= 32 ? 32 : 64, COPIES = 128 / SPAN;
+    const int copy = tid / SPAN, pair = tid - copy * SPAN;
     {
         int I = 0, J = 0;
-        if (tid < NP) pair_of(tid, NN, I, J);
+        if (pair < NP) pair_of(pair, NN, I, J);
         for (int k = 0; k < 16; ++k) {
             const int b = k / NV, bp = k % NV;
-            const int v = (tid < NP && k < NV * NV) ? p2m<DIM>(I, J, b, bp) : 0;
+            const int v = (pair < NP && k < NV * NV) ? p2m<DIM>(I, J, b, bp) : 0;
             *reinterpret_cast<__half *>(sa + tile_off(tid, k)) = __int2half_rn(v);
         }
     }
@@ -221,7 +228,7 @@ __global__ void __launch_bounds__(kTcThreads) elem_tc_kernel(int nt, const doubl
     for (;;) {
         if (tid == 0) tile_sh = atomicAdd(tile_counter, 1);
         __syncthreads();
-        const int e0 = tile_sh * EPT;
+        const int tile = tile_sh, e0 = tile * EPT;
         if (e0 >= nt) break;
         // ---- features of the tile's elements, as digits
         if (FE == 3) {
@@ -306,15 +313,16 @@ __global__ void __launch_bounds__(kTcThreads) elem_tc_kernel(int nt, const doubl
             break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // ---- epilogue: lane t of TMEM = pair t; warps without pairs skip it
-        if (warp * 32 < NP) {
+        // ---- epilogue: TMEM lane = copy and pair; warps without pairs skip it, the elements (or
+        // groups of 16 scalar ones) of a tile go round the copies
+        if (warp * 32 % SPAN < NP) {
             const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
             int I = 0, J = 0;
-            const bool act = tid < NP;
-            if (act) pair_of(tid, NN, I, J);
+            const bool act = pair < NP;
+            if (act) pair_of(pair, NN, I, J);
             float r[kTcDigits][16];
             if (FE == 3) {
-                for (int el = 0; el < EPT; ++el) {
+                for (int el = (copy + tile) % COPIES; el < EPT; el += COPIES) {
 #pragma unroll
                     for (int s = 0; s < kTcDigits; ++s) tmem_ld16(lane_addr + s * kTcN + el * 16, r[s]);
                     const int e = e0 + el;
@@ -348,7 +356,7 @@ __global__ void __launch_bounds__(kTcThreads) elem_tc_kernel(int nt, const doubl
                     }
                 }
             } else {
-                for (int ch = 0; ch < EPT / 16; ++ch) {
+                for (int ch = (copy + tile) % COPIES; ch < EPT / 16; ch += COPIES) {
 #pragma unroll
                     for (int s = 0; s < kTcDigits; ++s) tmem_ld16(lane_addr + s * kTcN + ch * 16, r[s]);
                     if (!act) continue;
