@@ -24,6 +24,11 @@ namespace ffgpu {
 
 constexpr unsigned long long kGsEmpty = 0xffffffffffffffffull;
 constexpr int kGsPolls = 1 << 22;      // about 2 s of polling
+// many blocks wait before they poll: the polling slows the partials that are still on their way
+// (CG on 130^2 and 256^2 cells, per iteration with two exchanges: 7.14 -> 6.4 and 9.42 -> 8.8 us; seven
+// blocks lose 0.3 us by it)
+constexpr int kGsPatient = 32;
+constexpr unsigned kGsWaitNs = 500;
 constexpr int kGsMaxBlocks = 160;      // four warps send and read, at most two slots per lane
 constexpr size_t kGsBytes = (size_t)4 * kGsMaxBlocks * kGsMaxBlocks * 16;
 
@@ -98,6 +103,7 @@ __device__ __forceinline__ bool gs_sum2(const GridSync &G, int k, double &a, dou
             ulonglong2 s0 = make_ulonglong2(0, 0), s1 = make_ulonglong2(0, 0);
             bool m0 = h0, m1 = h1;
             int left = kGsPolls;
+            if (nb >= kGsPatient) __nanosleep(kGsWaitNs);
             while (m0 || m1) {
                 if (m0) s0 = gs_load<PUBLISH>(box + i0);
                 if (m1) s1 = gs_load<PUBLISH>(box + i1);
@@ -126,6 +132,66 @@ __device__ __forceinline__ bool gs_sum2(const GridSync &G, int k, double &a, dou
     for (int i = 1; i < cnt; ++i) t += mine[i];
     a = __shfl_sync(full, t, 0);
     b = __shfl_sync(full, t, 16);
+    return true;
+}
+
+// Total of one value per thread over all threads of all blocks of 32 warps, as gs_sum2.  The block's
+// 1024 values are summed by four warps, eight per lane, through shared memory: 15 FP64
+// instructions on each sub-partition where a shuffle tree in every warp takes 40.
+// buf: 1024 + 16 doubles.
+template <bool PUBLISH>
+__device__ __forceinline__ bool gs_sum_wide(const GridSync &G, int k, double &a, double *buf) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double *part = buf + 1024, *tot = part + 8;   // part: two halves used in turn, tot likewise
+    part += (k & 1) * 4;
+    tot += (k & 1) * 4;
+    buf[threadIdx.x] = a;
+    __syncthreads();
+    const int nb = gridDim.x;
+    bool ok = true;
+    if (w < 4) {
+        double v = buf[w * 256 + lane];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) v += buf[w * 256 + 32 * i + lane];
+        v = warp_sum(v);
+        if (lane == 0) part[w] = v;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const double mine = (part[0] + part[1]) + (part[2] + part[3]);
+        double t = mine;
+        if (nb > 1) {
+            ulonglong2 *const all = G.slots + (size_t)(k & 3) * kGsMaxBlocks * kGsMaxBlocks;
+            const ulonglong2 out = make_ulonglong2(gs_bits(mine), 0);
+            if (PUBLISH) __threadfence();
+            for (int d = w * 32 + lane; d < nb; d += 128) gs_store(all + (size_t)d * kGsMaxBlocks + blockIdx.x, out);
+            ulonglong2 *const box = all + (size_t)blockIdx.x * kGsMaxBlocks;
+            const int per = (nb + 3) >> 2;
+            const int i0 = w * per + lane, i1 = i0 + 32;
+            const bool h0 = lane < per && i0 < nb, h1 = lane + 32 < per && i1 < nb;
+            ulonglong2 s0 = make_ulonglong2(0, 0), s1 = make_ulonglong2(0, 0);
+            bool m0 = h0, m1 = h1;
+            int left = kGsPolls;
+            if (nb >= kGsPatient) __nanosleep(kGsWaitNs);
+            while (m0 || m1) {
+                if (m0) s0 = gs_load<PUBLISH>(box + i0);
+                if (m1) s1 = gs_load<PUBLISH>(box + i1);
+                m0 = m0 && s0.x == kGsEmpty;
+                m1 = m1 && s1.x == kGsEmpty;
+                if (--left == 0) break;
+            }
+            ok = !(m0 || m1);
+            if (h0) gs_store(box + i0, make_ulonglong2(kGsEmpty, kGsEmpty));
+            if (h1) gs_store(box + i1, make_ulonglong2(kGsEmpty, kGsEmpty));
+            __syncwarp();
+            t = __longlong_as_double((long long)s0.x);
+            if (per > 32) t += __longlong_as_double((long long)s1.x);
+            t = warp_sum(t);
+        } else if (w) {
+            t = 0.0;
+        }
+        if (lane == 0) tot[w] = t;
+    }
+    if (__syncthreads_or(!ok)) return false;
+    a = (tot[0] + tot[1]) + (tot[2] + tot[3]);
     return true;
 }
 

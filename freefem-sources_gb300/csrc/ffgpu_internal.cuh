@@ -350,6 +350,9 @@ bool cluster_cg_fits(ffgpu_matrix *A, int trans);
 constexpr int kLoopRefused = 1;      // the launch was refused, nothing ran
 bool band_cg_fits(ffgpu_matrix *A);
 int band_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, double *h2, double *cg, cudaStream_t s);
+// the same for larger scalar systems, which stream from L2 or HBM
+bool loop_cg_fits(const ffgpu_matrix *A);
+int loop_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, double *q, double *z, cudaStream_t s);
 constexpr int kClusterRefused = 1;   // cluster_cg_run: the launch was refused, nothing ran
 int cluster_cg_run(ffgpu_matrix *A, int trans, double *x, const double *g, const double *h, cudaStream_t s);
 // the direct solver's factorisation: stale after a numeric change (the ordering and the

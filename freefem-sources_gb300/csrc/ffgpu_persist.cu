@@ -1,8 +1,9 @@
 // ffgpu_persist.cu -- the CG loop of ffgpu_solve_cg inside one cooperative kernel.
 //
-// FreeFEM's ConjugueGradient (src/femlib/CG.cpp:196-265) as ffgpu_solve.cu describes it, for
-// scalar systems whose block rows touch a narrow range of columns (2D meshes, small 3D ones).
-// One block per SM owns consecutive rows for the whole solve:
+// FreeFEM's ConjugueGradient (src/femlib/CG.cpp:196-265) as ffgpu_solve.cu describes it, in two
+// forms.  cg_loop, further down, streams the matrix.  cg_band is for scalar systems whose rows
+// touch a narrow range of columns (2D meshes, small 3D ones).  One block per SM owns
+// consecutive rows for the whole solve:
 //   * its rows of the matrix in shared memory (values FP64, columns as 16-bit numbers relative
 //     to the first column the block touches), x, g and 1/A_ii in registers;
 //   * per iteration it forms the direction h' = gamma h - C g once for every column it touches
@@ -18,6 +19,7 @@
 #include <algorithm>
 
 #include "ffgpu_gridsync.cuh"
+#include "ffgpu_sell.cuh"
 
 namespace ffgpu {
 
@@ -200,10 +202,126 @@ __global__ void __launch_bounds__(NT, 1) cg_band(BandArgs A) {
     }
 }
 
+// ------------------------------------------------------------------ larger scalar systems
+// The same loop for matrices that stream from L2 or HBM: one block of 32 warps per SM, the SELL-32
+// copy in its stride assignment with the batched row loop, three exchanges per iteration --
+//   q = A h, (h,q)              [q visible]      rho
+//   x += rho h, g += rho q, z = C g, (g,z)       gamma, FreeFEM's stopping test
+//   h = gamma h - z, (g,h)      [h visible]
+// -- on vectors each block owns a contiguous piece of; the pieces of g and z stay in shared memory.
+// Against the three launches per iteration it saves their starts, tails and last-block sums.
+// Per iteration, launches and loop: P1 on 60^3 cells 31.2 and 29.2 us, 90^3 60.2 and 50.2, 120^3 105.9
+// and 98.4 (102 with g and z in L2); on 140^3, where two pieces no longer fit, 152 and 153; P2 on 24 x
+// 23 x 22 40.9 and 33.9; P1 on 700^2 39.3 and 34.3.  3x3 blocks (24^3 cells: 90.3 and 91.4) and
+// double-float products (17 x 16 x 15: 39.3 and 49.9) are no faster and keep the launches.
+struct LoopArgs {
+    int n, per;                  // elements of a block, even
+    SellArgs S;
+    const double *val, *dinv;
+    double *x, *g, *h, *q, *z;
+    KrylovScalars *ks;
+    GridSync gs;
+};
+
+template <bool C16>
+__global__ void __launch_bounds__(1024, 1) cg_loop(LoopArgs A) {
+    extern __shared__ __align__(16) double smd[];
+    __shared__ double buf[1024 + 16];
+    if (A.ks->done) return;
+    const int t = threadIdx.x, lane = t & 31;
+    const int e0 = blockIdx.x * A.per, ne = max(0, min(A.per, A.n - e0)), np = ne >> 1;
+    double *const xs = A.x + e0, *const hs = A.h + e0, *const gs = smd, *const zs = smd + A.per;
+    const double *const ds = A.dinv + e0;
+    for (int i = t; i < ne; i += 1024) gs[i] = A.g[e0 + i];
+    __syncthreads();
+    const double eps2 = A.ks->eps2;
+    const int itmax = A.ks->itmax;
+    double gcg = A.ks->gcg, gcgp = gcg, gamma = 1.0, rho = 0.0, sgh = A.ks->s_gh, shq = 0.0;
+    int iter = 0, conv = 0, k = 0;
+    bool good = true;
+    const double *const hg = A.h;
+    for (;;) {
+        // ---- q = A h, (h, q)
+        double part = 0.0;
+        sell_for_chunks<kSellStride, 1>(A.S, [&](int c, int a, int L, int64_t sr) {
+            double y[1];
+            sell_row64<1, C16, 2, true>(A.S, A.val, hg, L, sr, lane, a, y);
+            if (a >= 0) {
+                __stcg(A.q + a, y[0]);
+                part = fma(__ldca(hg + a), y[0], part);
+            }
+        });
+        if (!gs_sum_wide<true>(A.gs, k++, part, buf)) { good = false; break; }
+        shq = part;
+        rho = -sgh / shq;
+        // ---- x += rho h, g += rho q, z = C g, (g, z)
+        part = 0.0;
+#pragma unroll 2
+        for (int j = t; j < np; j += 1024) {
+            const double2 qv = __ldcg(reinterpret_cast<const double2 *>(A.q + e0) + j);
+            const double2 hv = __ldcg(reinterpret_cast<const double2 *>(hs) + j), dv = reinterpret_cast<const double2 *>(ds)[j];
+            double2 xv = reinterpret_cast<double2 *>(xs)[j], gv = reinterpret_cast<double2 *>(gs)[j];
+            xv.x = fma(rho, hv.x, xv.x); xv.y = fma(rho, hv.y, xv.y);
+            gv.x = fma(rho, qv.x, gv.x); gv.y = fma(rho, qv.y, gv.y);
+            reinterpret_cast<double2 *>(xs)[j] = xv;
+            reinterpret_cast<double2 *>(gs)[j] = gv;
+            const double2 zv = make_double2(__dmul_rn(dv.x, gv.x), __dmul_rn(dv.y, gv.y));
+            reinterpret_cast<double2 *>(zs)[j] = zv;
+            part = fma(gv.x, zv.x, part);
+            part = fma(gv.y, zv.y, part);
+        }
+        if ((ne & 1) && t == 0) {
+            const int j = ne - 1;
+            xs[j] = fma(rho, __ldcg(hs + j), xs[j]);
+            const double gv = fma(rho, __ldcg(A.q + e0 + j), gs[j]);
+            gs[j] = gv;
+            zs[j] = __dmul_rn(ds[j], gv);
+            part = fma(gv, zs[j], part);
+        }
+        if (!gs_sum_wide<false>(A.gs, k++, part, buf)) { good = false; break; }
+        gcgp = gcg;
+        gcg = part;
+        gamma = gcg / gcgp;
+        ++iter;
+        conv = gcg < eps2;
+        if (conv || iter >= itmax) break;
+        // ---- h = gamma h - z, (g, h)
+        part = 0.0;
+#pragma unroll 2
+        for (int j = t; j < np; j += 1024) {
+            const double2 gv = reinterpret_cast<const double2 *>(gs)[j], zv = reinterpret_cast<const double2 *>(zs)[j];
+            double2 hv = __ldcg(reinterpret_cast<const double2 *>(hs) + j);
+            hv.x = fma(gamma, hv.x, -zv.x);
+            hv.y = fma(gamma, hv.y, -zv.y);
+            __stcg(reinterpret_cast<double2 *>(hs) + j, hv);
+            part = fma(gv.x, hv.x, part);
+            part = fma(gv.y, hv.y, part);
+        }
+        if ((ne & 1) && t == 0) {
+            const int j = ne - 1;
+            const double hv = fma(gamma, __ldcg(hs + j), -zs[j]);
+            __stcg(hs + j, hv);
+            part = fma(gs[j], hv, part);
+        }
+        if (!gs_sum_wide<true>(A.gs, k++, part, buf)) { good = false; break; }
+        sgh = part;
+    }
+    if (blockIdx.x == 0 && t == 0) {
+        KrylovScalars *ks = A.ks;
+        ks->gcg = gcg; ks->gcgp = gcgp; ks->gamma = gamma; ks->rho = rho; ks->s_gh = sgh; ks->s_hq = shq;
+        ks->iter = iter;
+        ks->converged = conv;
+        ks->done = good ? 1 : 2;
+    }
+}
+
 // ------------------------------------------------------------------ host side
+constexpr int kBandOneBlock = 512;
 // Rows per block: a multiple of 32, all SMs, at least 64 (a shorter block costs more exchange than
 // it saves FP64 time).
 static int band_rows(int n) {
+    // one block needs no exchange: 4.9 us per iteration for 441 rows, 5.8 with seven blocks
+    if (n <= kBandOneBlock) return (n + 31) / 32 * 32;
     const int per = (n + kNumSM - 1) / kNumSM;
     return std::max(64, (per + 31) / 32 * 32);
 }
@@ -277,6 +395,42 @@ int band_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, dou
         return kLoopRefused;
     }
     return launch_check(ctx, "cg_band");
+}
+
+constexpr size_t kLoopSmem = 190 * 1024;   // the rest of the SM's 256 KB is the L1 the gathers go through
+static int loop_piece(int n) { return ((n + kNumSM - 1) / kNumSM + 1) & ~1; }
+// Whether the streaming loop takes the system: a rule on sizes and the device.
+bool loop_cg_fits(const ffgpu_matrix *A) {
+    return A->ctx->coop && A->ctx->d_sync && A->bs == 1 && 2 * sizeof(double) * (size_t)loop_piece(A->n) <= kLoopSmem;
+}
+
+// The loop from the state cg_init leaves; z: a work vector.
+int loop_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, double *q, double *z, cudaStream_t s) {
+    ffgpu_ctx *ctx = A->ctx;
+    FFGPU_TRY(sell_values(A, trans ? kSell64T : kSell64));
+    LoopArgs a;
+    memset(&a, 0, sizeof(a));
+    a.n = A->n;
+    a.per = loop_piece(A->n);
+    a.S = sell_args(A);
+    a.val = trans ? A->sval_t : A->sval;
+    a.dinv = A->diag_inv;
+    a.x = x; a.g = g; a.h = h; a.q = q; a.z = z;
+    a.ks = A->ks;
+    a.gs.slots = (ulonglong2 *)ctx->d_sync;
+    const size_t smem = 2 * sizeof(double) * (size_t)a.per;
+    void *fn = A->scol16 ? (void *)cg_loop<true> : (void *)cg_loop<false>;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        cudaGetLastError();
+        return kLoopRefused;
+    }
+    FFGPU_CUDA(cudaMemsetAsync(ctx->d_sync, 0xff, kGsBytes, s));
+    void *args[] = {&a};
+    if (cudaLaunchCooperativeKernel(fn, dim3(kNumSM), dim3(1024), args, smem, s) != cudaSuccess) {
+        cudaGetLastError();
+        return kLoopRefused;
+    }
+    return launch_check(ctx, "cg_loop");
 }
 
 }  // namespace ffgpu

@@ -188,6 +188,14 @@ __device__ __forceinline__ int sell_col(const SellArgs &S, int64_t e, int ar) {
     return __ldcs(S.col + e);
 }
 
+// The gathered vector: read-only for the whole launch, or (COH) rewritten between phases of it, which
+// the read-only path may not be used for.
+template <bool COH, typename V>
+__device__ __forceinline__ V sell_x(const V *p) {
+    if constexpr (COH) return __ldca(p);
+    else return __ldg(p);
+}
+
 // FP32 and double-float rows process entries in batches of B slots: all column, value and vector
 // loads of a batch are issued before its first product, so a lane keeps B independent gathers
 // in flight (a runtime-length loop unrolled B deep runs its remainder one dependent load at a
@@ -210,9 +218,8 @@ template <typename V, int BS, int B>
 struct SellBatch {
     V a[B][BS * BS];
     V xv[B][BS];
-    template <bool C16, bool GUARD>
-    __device__ __forceinline__ void load(const SellArgs &S, const V *__restrict__ v, const V *__restrict__ x,
-                                         int64_t ce, int ar, int j, int rem) {
+    template <bool C16, bool GUARD, bool COH>
+    __device__ __forceinline__ void load(const SellArgs &S, const V *__restrict__ v, const V *x, int64_t ce, int ar, int j, int rem) {
 #pragma unroll
         for (int u = 0; u < B; ++u) {
             if (GUARD && u >= rem) continue;
@@ -221,7 +228,7 @@ struct SellBatch {
 #pragma unroll
             for (int k = 0; k < BS * BS; ++k) a[u][k] = __ldcs(w + 32 * k);
 #pragma unroll
-            for (int m = 0; m < BS; ++m) xv[u][m] = __ldg(x + (int64_t)BS * col + m);
+            for (int m = 0; m < BS; ++m) xv[u][m] = sell_x<COH>(x + (int64_t)BS * col + m);
         }
     }
     template <typename Acc>
@@ -254,23 +261,22 @@ struct SellTail<0> {
 
 // One block row per lane: lane `lane` of chunk c holds row a (a < 0: padding lane, its entries
 // are zero blocks on column 0), L slots starting at slot row sr.
-template <typename V, int BS, int B, bool C16, typename Acc>
-__device__ __forceinline__ void sell_row(const SellArgs &S, const V *__restrict__ val, const V *__restrict__ x,
-                                         int L, int64_t sr, int lane, int a, Acc *acc) {
+template <typename V, int BS, int B, bool C16, bool COH, typename Acc>
+__device__ __forceinline__ void sell_row(const SellArgs &S, const V *__restrict__ val, const V *x, int L, int64_t sr, int lane, int a, Acc *acc) {
     const int ar = a < 0 ? 0 : a;
     const int64_t ce = sr * 32 + lane;
     const V *v = val + sr * (BS * BS * 32) + lane;
     int j = 0;
     for (; j + B <= L; j += B) {
         SellBatch<V, BS, B> t;
-        t.template load<C16, false>(S, v, x, ce, ar, j, B);
+        t.template load<C16, false, COH>(S, v, x, ce, ar, j, B);
 #pragma unroll
         for (int u = 0; u < B; ++u) t.apply(u, acc);
     }
     const int rem = L - j;
     if (rem > 0) {
         SellBatch<V, BS, B> t;
-        t.template load<C16, true>(S, v, x, ce, ar, j, rem);
+        t.template load<C16, true, COH>(S, v, x, ce, ar, j, rem);
         SellTail<B - 1>::run(t, rem, acc);
     }
 }
@@ -292,13 +298,12 @@ struct AccF64 {
     __device__ __forceinline__ double get() const { return s; }
 };
 
-template <int BS, bool C16, int LOOP>
-__device__ __forceinline__ void sell_row64(const SellArgs &S, const double *__restrict__ val,
-                                           const double *__restrict__ x, int L, int64_t sr, int lane, int a,
+template <int BS, bool C16, int LOOP, bool COH = false>
+__device__ __forceinline__ void sell_row64(const SellArgs &S, const double *__restrict__ val, const double *x, int L, int64_t sr, int lane, int a,
                                            double *y) {
     if constexpr (LOOP >= 2) {
         AccF64 acc[BS];
-        sell_row<double, BS, SellDepth<BS, LOOP == 3>::B, C16>(S, val, x, L, sr, lane, a, acc);
+        sell_row<double, BS, SellDepth<BS, LOOP == 3>::B, C16, COH>(S, val, x, L, sr, lane, a, acc);
 #pragma unroll
         for (int m = 0; m < BS; ++m) y[m] = acc[m].get();
         return;
@@ -313,10 +318,10 @@ __device__ __forceinline__ void sell_row64(const SellArgs &S, const double *__re
         for (int j = 0; j < L; ++j) {
             const int col = sell_col<C16>(S, ce + (int64_t)j * 32, ar);
             if (BS == 1) {
-                s0 = fma(__ldcs(v + (int64_t)j * 32), __ldg(x + col), s0);
+                s0 = fma(__ldcs(v + (int64_t)j * 32), sell_x<COH>(x + col), s0);
             } else {
-                const double x0 = __ldg(x + 3 * (int64_t)col), x1 = __ldg(x + 3 * (int64_t)col + 1),
-                             x2 = __ldg(x + 3 * (int64_t)col + 2);
+                const double x0 = sell_x<COH>(x + 3 * (int64_t)col), x1 = sell_x<COH>(x + 3 * (int64_t)col + 1),
+                             x2 = sell_x<COH>(x + 3 * (int64_t)col + 2);
                 const double *w = v + (int64_t)j * 288;
                 s0 = fma(__ldcs(w), x0, s0); s0 = fma(__ldcs(w + 32), x1, s0); s0 = fma(__ldcs(w + 64), x2, s0);
                 s1 = fma(__ldcs(w + 96), x0, s1); s1 = fma(__ldcs(w + 128), x1, s1); s1 = fma(__ldcs(w + 160), x2, s1);
@@ -328,22 +333,20 @@ __device__ __forceinline__ void sell_row64(const SellArgs &S, const double *__re
     }
 }
 
-template <int BS, bool C16, bool DEEP>
-__device__ __forceinline__ void sell_rowx(const SellArgs &S, const float2 *__restrict__ val,
-                                          const float2 *__restrict__ x, int L, int64_t sr, int lane, int a,
+template <int BS, bool C16, bool DEEP, bool COH = false>
+__device__ __forceinline__ void sell_rowx(const SellArgs &S, const float2 *__restrict__ val, const float2 *x, int L, int64_t sr, int lane, int a,
                                           double *y) {
     AccDF acc[BS];
-    sell_row<float2, BS, SellDepth<BS, DEEP>::B, C16>(S, val, x, L, sr, lane, a, acc);
+    sell_row<float2, BS, SellDepth<BS, DEEP>::B, C16, COH>(S, val, x, L, sr, lane, a, acc);
 #pragma unroll
     for (int m = 0; m < BS; ++m) y[m] = acc[m].get();
 }
 
-template <int BS, bool C16, bool DEEP>
-__device__ __forceinline__ void sell_row32(const SellArgs &S, const float *__restrict__ val,
-                                           const float *__restrict__ x, int L, int64_t sr, int lane, int a,
+template <int BS, bool C16, bool DEEP, bool COH = false>
+__device__ __forceinline__ void sell_row32(const SellArgs &S, const float *__restrict__ val, const float *x, int L, int64_t sr, int lane, int a,
                                            float *y) {
     AccF32 acc[BS];
-    sell_row<float, BS, SellDepth<BS, DEEP, true>::B, C16>(S, val, x, L, sr, lane, a, acc);
+    sell_row<float, BS, SellDepth<BS, DEEP, true>::B, C16, COH>(S, val, x, L, sr, lane, a, acc);
 #pragma unroll
     for (int m = 0; m < BS; ++m) y[m] = acc[m].get();
 }

@@ -1352,7 +1352,9 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     bool fused = !cluster && cg_fused_fits(A, mode);
     if (fused) unroll += unroll & 1;   // the H buffers alternate: an even number of iterations per body
     // the whole loop in one cooperative kernel where a block's rows and columns fit its SM
-    bool loop = mode == 0 && !cluster && !A->layout_pinned && in_kernel_loops() && band_cg_fits(A);
+    const bool may_loop = mode == 0 && !cluster && !A->layout_pinned && in_kernel_loops();
+    const bool band = may_loop && band_cg_fits(A);
+    bool loop = band || (may_loop && loop_cg_fits(A));
     if (!cluster && !loop) FFGPU_TRY(cg_graph(A, trans, unroll, mode, x, g, h, q, fused, h2, cgv));
     FFGPU_CUDA(cudaMemcpyAsync(x, xu, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     cudaEvent_t e0, e1;
@@ -1379,7 +1381,7 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     int bodies_host = -1;
     bool use_graph = !cluster && !loop;
     if (loop) {
-        const int rc = band_cg_run(A, trans, x, g, h, h2, cgv, s);
+        const int rc = band ? band_cg_run(A, trans, x, g, h, h2, cgv, s) : loop_cg_run(A, trans, x, g, h, q, cgv, s);
         if (rc == kLoopRefused) {
             // the launches per iteration from the same state
             FFGPU_TRY(cg_graph(A, trans, unroll, mode, x, g, h, q, false, h2, cgv));

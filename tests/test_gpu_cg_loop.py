@@ -1,6 +1,6 @@
-"""The CG loop inside one cooperative kernel (cg_band, ffgpu_persist.cu) at the edges of its
-dispatch: one block, the row counts where the threads per block and rows per thread change, the
-last size it takes, and patterns whose column range keeps it out.
+"""The CG loops inside one cooperative kernel (cg_band and cg_loop, ffgpu_persist.cu) at the edges of
+their dispatch: one block, the row counts where the threads per block and rows per thread change, the
+last size cg_band takes, and what cg_loop takes: wide column ranges, larger systems, odd sizes.
 
 Bars: the ones of the other CG paths -- 1e-9 against the launches per iteration (FFGPU_CG_FUSE=0)
 and the oracle, iteration counts within 2, the same bits on a second solve.
@@ -108,7 +108,7 @@ def test_loop_iteration_limit_and_converged_start():
     assert np.array_equal(A.solve(z), z) and A.stats.iterations == 0
 
 
-def test_wide_patterns_and_fixed_layouts_keep_the_launches():
+def test_wide_pattern_streams_and_a_fixed_layout_keeps_the_launches():
     A, b = _matrix(mesh.square(200), eps=1e-10)
     rp, cl, vl = A.csr()
     import scipy.sparse as sp
@@ -117,9 +117,31 @@ def test_wide_patterns_and_fixed_layouts_keep_the_launches():
     S.sort_indices()
     B = ffgpu.matrix_from_csr(S.indptr, S.indices, S.data, eps=1e-10)
     u, l, it = _solve(A, b)
-    v, lw, itw = _solve(B, b[p])
-    assert l < 12 and lw >= 2 * itw                       # a block of the permuted rows touches every column
+    v, lw, itw = _solve(B, b[p])                          # a block of the permuted rows touches every column
+    assert l < 12 and lw < 12 and abs(it - itw) <= 2
     assert np.linalg.norm(v - u[p]) <= 1e-9 * np.linalg.norm(u)
+    assert np.array_equal(B.solve(b[p]), v)
+    t, lt, _ = _solve(B, b[p], trans=True)
+    assert lt < 12 and np.linalg.norm(t - v) <= 1e-9 * np.linalg.norm(v)
     w, lf, itf = _solve(A, b, spmv_layout=64)
     assert lf >= 2 * itf
     assert np.linalg.norm(w - u) <= 1e-9 * np.linalg.norm(u)
+
+
+@pytest.mark.parametrize("kind,dim,n", [("P1", 3, (59, 60, 61)), ("P1", 2, (557, 561)), ("P2", 3, (20, 21, 19)), ("P1", 3, (95, 96, 94))])
+def test_streaming_loop_against_launches(kind, dim, n):
+    import torch
+    S = ffgpu.device_space(kind, dim, *n)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    kappa = torch.exp(torch.randn(S.Vh.Th.nt, generator=g, device="cuda", dtype=torch.float64))
+    b = torch.zeros(S.Vh.ndof, device="cuda", dtype=torch.float64)
+    torch.cuda.synchronize()
+    A = ffgpu.matrix(ffgpu.varf_diffusion(kappa=kappa, on=(1, 2, 3, 4)), S, eps=1e-10, rhs_out=b)
+    bh = b.cpu().numpy()
+    u, l, it = _solve(A, bh)
+    assert l < 12, l
+    assert np.array_equal(A.solve(bh), u)
+    u3, l3, it3 = _solve(A, bh, env={"FFGPU_CG_FUSE": "0"})
+    assert l3 >= 3 * it3 and abs(it - it3) <= 2
+    assert np.linalg.norm(u - u3) <= 1e-8 * np.linalg.norm(u3)
