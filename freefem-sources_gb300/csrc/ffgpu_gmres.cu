@@ -19,16 +19,24 @@
 //   SpMV       w = A vp
 //   gm_dots    s = V' w and the Gram row in one pass over V: blocks are (slab of the vectors'
 //              elements) x (group of basis vectors), w and v_it of a slab staged in shared
-//              memory, one warp reduction per pair of sums and sub-tile; last block: the sums
+//              memory, one warp reduction per pair of sums and sub-tile, the last block of a group
+//              sums its slabs; one more block finishes step it - 1: the new rotation, Q's two
+//              changed rows, the residual estimate |g_it|, FreeFEM's stopping tests
 //   gm_coef    h = s - L s (a warp per row, all SMs)
-//   gm_update  v_{it+1} = w - V h, ||v_{it+1}||^2, and the earlier rotations applied to h as
-//              u = Q h with their product Q (a warp per row); last block: the new rotation, Q's two
-//              changed rows, residual estimate |g_{it+1}|, FreeFEM's stopping tests
-// A rotation after the other (FreeFEM's loop) is a chain of 2 it dependent FP64 operations, 76
-// cycles each on GB300: 14 us at it = 190.  The product Q costs it^2 multiplications over all SMs.
+//   gm_update  v_{it+1} = w - V h, ||v_{it+1}||^2 by blocks, and the earlier rotations applied to h
+//              as u = Q h with their product Q (a warp per row)
 // and the Arnoldi loop of one restart cycle is a CUDA-graph `while` node.  The host reads the
 // scalars once per restart cycle.  All reductions sum in a fixed order (warp order inside a
 // block, block order across blocks), so results are reproducible run to run.
+//
+// No kernel ends with one block that works alone: gm_dots ends with one per vector group, the norm
+// is summed where it is read, and the rotation (a chain of square roots and divisions) runs beside
+// the next step's dot products, at the price of that step's first three kernels once per cycle,
+// when it says stop (9282 rows, 381 steps: 16.7 ms with last blocks in gm_dots and gm_update,
+// 14.3 ms now; the FP64 products alone are 3.1 ms, the rest is latency inside the five kernels).
+// Sums of gm_dots' slabs by every block of gm_coef instead: 16.2 ms.
+// A rotation after the other (FreeFEM's loop) is a chain of 2 it dependent FP64 operations, 76
+// cycles each on GB300: 14 us at it = 190.  The product Q costs it^2 multiplications over all SMs.
 #include <math.h>
 #include <string.h>
 
@@ -50,6 +58,7 @@ constexpr int kGmHs = 1024;                  // Hessenberg columns up to this le
 struct GmScal {
     double normb, relres, eps;
     int it, iter, itmax, m, conv, stop, steps, itf;
+    int next;                                // the step of gm_prep and gm_dots (gm_coef sets it; `it` is gm_coef's and gm_update's)
     unsigned ticket;
 };
 
@@ -63,7 +72,9 @@ struct GmArgs {
     const uint8_t *wcl;
     int use_wcl;
     int rows;                                // rows of a block of gm_update / gm_xupd
-    double *R, *Q, *u, *g, *y, *vnorm, *Gm, *h, *red, *part;   // R: column it of the triangle at it * (m + 1)
+    int nupd;                                // blocks of gm_update (parts of nrm)
+    int *tick;                               // gm_dots: blocks of a vector group that are done
+    double *R, *Q, *u, *g, *y, *Gm, *h, *red, *part, *nrm;   // R: column it of the triangle at it * (m + 1)
     GmScal *sc;
     cudaGraphConditionalHandle cond;
     int in_graph;
@@ -146,10 +157,10 @@ __global__ void __launch_bounds__(kGmThreads) gm_resid(GmArgs a) {
         GmScal *c = a.sc;
         const double g0 = sqrt(a.red[0]);
         a.g[0] = g0;
-        a.vnorm[0] = g0;
         a.Q[0] = 1.0;
         if (c->normb < 1.e-20 || c->eps < 0) c->normb = 1.;
         c->it = 0;
+        c->next = 0;
         c->stop = 0;
         // an exact initial guess: FreeFEM would divide by zero here; the solve is converged
         if (g0 == 0.0) {
@@ -162,11 +173,32 @@ __global__ void __launch_bounds__(kGmThreads) gm_resid(GmArgs a) {
     }
 }
 
+// ||v_it||^2 before its scaling, in every thread of the block: the sum of gm_update's parts (at
+// most 4 * kNumSM of them)
+__device__ __forceinline__ double gm_norm2(const GmArgs &a) {
+    __shared__ double sh[kGmWarps];
+    static_assert(4 * kNumSM <= 3 * kGmThreads && kGmWarps == 8, "parts per thread");
+    double v[3];
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+        const int b = threadIdx.x + u * kGmThreads;
+        v[u] = b < a.nupd ? __ldcg(a.nrm + b) : 0.0;
+    }
+    double t = warp_sum((v[0] + v[1]) + v[2]);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+    __syncthreads();
+    t = sh[threadIdx.x & 7];
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
 // v_it *= 1/||.|| (FreeFEM: Vi[it] = (1./aux)*wi), vp = C v_it into Vp[it] and the SpMV input
 __global__ void __launch_bounds__(kGmThreads) gm_prep(GmArgs a) {
-    const int it = a.sc->it;
+    const int it = a.sc->next;
+    if (it >= a.m) return;   // the cycle is full: gm_dots finishes its last step
     double *v = a.V + it * a.vs, *vp = a.Vp + it * a.vs;
-    const double inv = 1. / a.vnorm[it];
+    const double inv = it == 0 ? 1. / a.g[0] : 1. / sqrt(gm_norm2(a));
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n; k += (int64_t)gridDim.x * blockDim.x) {
         const double vk = inv * v[k];
         v[k] = vk;
@@ -176,95 +208,162 @@ __global__ void __launch_bounds__(kGmThreads) gm_prep(GmArgs a) {
     }
 }
 
+// the end of step it: the new rotation, the triangle's column, Q, the stopping tests (one block)
+__device__ void gm_finish(const GmArgs &a, int it) {
+    __shared__ double rot[2];
+    const int ld = a.m + 1;
+    GmScal *c = a.sc;
+    const double aux = sqrt(gm_norm2(a));
+    if (threadIdx.x == 0) {
+        const double hd = a.u[it], hs1 = aux;
+        const double sq = sqrt(hd * hd + hs1 * hs1);
+        const double c0 = hd / sq, s0 = hs1 / sq;
+        rot[0] = c0;
+        rot[1] = s0;
+        a.R[(int64_t)it * ld + it] = c0 * hd + s0 * hs1;
+        const double g0 = a.g[it];
+        a.g[it + 1] = -s0 * g0;
+        a.g[it] = c0 * g0;
+        const double relres = fabs(-s0 * g0);
+        c->relres = relres;
+        c->steps += 1;
+        c->itf = it;
+        bool stop = false;
+        if (relres / c->normb < fabs(c->eps)) {
+            c->conv = 1;
+            stop = true;
+        } else if (it > c->itmax) {
+            stop = true;                       // FreeFEM: `if (it > nbitermx) break;`
+        } else {
+            c->it = it + 1;                    // the loop increment it++, iter++
+            c->iter += 1;
+            if (it + 1 >= a.m) { stop = true; c->itf = a.m - 1; }
+        }
+        c->stop = stop;
+        if (stop && a.in_graph) gm_set_cond(a.cond, 0);
+    }
+    __syncthreads();
+    // the column of the triangle, and Q with the new rotation of its rows it and it + 1
+    double *q0 = a.Q + (int64_t)it * (ld + 1), *q1 = q0 + ld + 1;
+    for (int i = threadIdx.x; i <= it + 1; i += blockDim.x) {
+        if (i < it) a.R[(int64_t)it * ld + i] = a.u[i];
+        const double q = i <= it ? q0[i] : 0.0;
+        q0[i] = i <= it ? rot[0] * q : rot[1];
+        q1[i] = i <= it ? -rot[1] * q : rot[0];
+    }
+}
+
 // s_i = (w, v_i), i <= it, and the Gram row (v_it, v_j), j < it, in one pass over V.
 // Block (slab, group): the elements [slab * slab_len, +slab_len) of the vectors i = group +
 // ngrp * r; per sub-tile of kGmSub elements w and v_it are staged in shared memory and each warp
 // runs its vectors over the sub-tile (16 elements per lane, then one warp reduction for both sums).
-// Partials part[k * nslab + slab], k < 2(it+1); the last block sums them in slab order.
+// A vector's elements are loaded before the products of the one before it (the first vector's
+// before the staging).
+// Partials part[(2 i + c) * nslab + slab]: c = 0 for s, 1 for the Gram row; the last block of a
+// vector group sums them in slab order (a half warp per sum).
 __global__ void __launch_bounds__(kGmThreads) gm_dots(GmArgs a) {
     extern __shared__ __align__(16) double smd[];
     double *wsh = smd, *vsh = smd + kGmSub, *acc = smd + 2 * kGmSub;
-    const int it = a.sc->it;
+    const int it = a.sc->next;
+    if (blockIdx.x == 0) {
+        if (it > 0) gm_finish(a, it - 1);
+        return;
+    }
+    if (it >= a.m) return;
     const int ni = it + 1, K = 2 * ni;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int slab = blockIdx.x % a.nslab, grp = blockIdx.x / a.nslab;
+    const int blk = blockIdx.x - 1;
+    const int slab = blk % a.nslab, grp = blk / a.nslab;
     for (int k = threadIdx.x; k < K; k += blockDim.x) acc[k] = 0;
     const double *vit = a.V + it * a.vs;
     const int64_t e0 = (int64_t)slab * a.slab_len;
     const int64_t e1 = e0 + a.slab_len < a.n ? e0 + a.slab_len : (int64_t)a.n;
     for (int64_t t0 = e0; t0 < e1; t0 += kGmSub) {
         const int len = e1 - t0 < kGmSub ? (int)(e1 - t0) : kGmSub;
+        const int len2 = len & ~1;   // pairs of elements as 16-byte loads; an odd last element apart
+        constexpr int NP = kGmSub / 64;
+        int i = grp + a.ngrp * warp;
+        double2 q[NP], nx[NP];
+        const auto load = [&](double2 *d, int iv) {
+            const double *vi = a.V + iv * a.vs + t0;   // 16-byte aligned: vs and t0 are even
+#pragma unroll
+            for (int u = 0; u < NP; ++u)
+                if (2 * lane + 64 * u < len2) d[u] = __ldcs(reinterpret_cast<const double2 *>(vi + 2 * lane + 64 * u));
+        };
+        if (i < ni) load(q, i);
         __syncthreads();   // the previous sub-tile's readers are done (and acc is zeroed)
         for (int e = threadIdx.x; e < len; e += blockDim.x) {
             wsh[e] = a.w[t0 + e];
             vsh[e] = vit[t0 + e];
         }
         __syncthreads();
-        const int len2 = len & ~1;   // pairs of elements as 16-byte loads; an odd last element apart
-        for (int i = grp + a.ngrp * warp; i < ni; i += a.ngrp * kGmWarps) {
-            const double *vi = a.V + i * a.vs + t0;   // 16-byte aligned: vs and t0 are even
+        while (i < ni) {
+            const int in = i + a.ngrp * kGmWarps;
+            if (in < ni) load(nx, in);
             double ts = 0, tl = 0;
-#pragma unroll 8
-            for (int e = 2 * lane; e < len2; e += 64) {
-                const double2 q = __ldcs(reinterpret_cast<const double2 *>(vi + e));
-                const double2 w2 = *reinterpret_cast<const double2 *>(wsh + e);
-                const double2 v2 = *reinterpret_cast<const double2 *>(vsh + e);
-                ts = fma(q.x, w2.x, ts);
-                tl = fma(q.x, v2.x, tl);
-                ts = fma(q.y, w2.y, ts);
-                tl = fma(q.y, v2.y, tl);
+#pragma unroll
+            for (int u = 0; u < NP; ++u) {
+                const int e = 2 * lane + 64 * u;
+                if (e < len2) {
+                    const double2 w2 = *reinterpret_cast<const double2 *>(wsh + e);
+                    const double2 v2 = *reinterpret_cast<const double2 *>(vsh + e);
+                    ts = fma(q[u].x, w2.x, ts);
+                    tl = fma(q[u].x, v2.x, tl);
+                    ts = fma(q[u].y, w2.y, ts);
+                    tl = fma(q[u].y, v2.y, tl);
+                }
             }
             if (len2 < len && lane == 0) {
-                const double q = __ldcs(vi + len2);
-                ts = fma(q, wsh[len2], ts);
-                tl = fma(q, vsh[len2], tl);
+                const double qo = __ldcs(a.V + i * a.vs + t0 + len2);
+                ts = fma(qo, wsh[len2], ts);
+                tl = fma(qo, vsh[len2], tl);
             }
             const double p = warp_sum_pair(ts, tl);   // vector i belongs to this warp
             if ((lane & 15) == 0) acc[lane ? ni + i : i] += p;
+#pragma unroll
+            for (int u = 0; u < NP; ++u) q[u] = nx[u];
+            i = in;
         }
     }
-    __syncthreads();
+    __syncwarp();   // a warp reads back its own vectors' sums
     for (int i = grp + a.ngrp * warp; i < ni; i += a.ngrp * kGmWarps)
-        if (lane == 0) {
-            a.part[(int64_t)i * a.nslab + slab] = acc[i];
-            a.part[(int64_t)(ni + i) * a.nslab + slab] = acc[ni + i];
-        }
+        if (lane < 2) a.part[(2 * (int64_t)i + lane) * a.nslab + slab] = acc[lane * ni + i];
     __shared__ bool s_last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&a.sc->ticket, 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) s_last = atomicAdd(a.tick + grp, 1) == a.nslab - 1;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    const int ld = a.m + 1;
-    // a thread per sum, slabs in order (independent loads in flight, no shuffle chain per sum)
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const double *pk = a.part + (int64_t)k * a.nslab;
-        double t = 0;
-#pragma unroll 8
-        for (int b = 0; b < a.nslab; ++b) t += __ldcg(pk + b);
-        if (k < ni) a.red[k] = t;                                    // s
-        else if (k - ni < it) a.Gm[(int64_t)it * ld + (k - ni)] = t;   // Gram row of v_it
+    static_assert(kGmMaxSlabs == 32, "two slabs per lane of a half warp");
+    const int l16 = lane & 15, c = lane >> 4;
+    for (int i = grp + a.ngrp * warp; i < ni; i += a.ngrp * kGmWarps) {
+        const double *p = a.part + (2 * (int64_t)i + c) * a.nslab;
+        double t = l16 < a.nslab ? __ldcg(p + l16) : 0.0;
+        if (l16 + 16 < a.nslab) t += __ldcg(p + l16 + 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) a.red[i] = t;                                        // s
+        if (lane == 16 && i < it) a.Gm[(int64_t)it * (a.m + 1) + i] = t;   // Gram row of v_it
     }
-    __syncthreads();
-    if (threadIdx.x == 0) a.sc->ticket = 0u;
+    if (threadIdx.x == 0) a.tick[grp] = 0;
 }
 
 // modified Gram-Schmidt's coefficients of this step to first order in the Gram entries:
 // h_i = s_i - sum_{j<i} G(i,j) s_j (a warp per row, rows over the whole grid)
 __global__ void __launch_bounds__(kGmThreads) gm_coef(GmArgs a) {
+    if (a.sc->stop) return;
     const int it = a.sc->it;
     const int ni = it + 1, ld = a.m + 1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.sc->next = ni;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = blockIdx.x * kGmWarps + warp; i < ni; i += gridDim.x * kGmWarps) {
         const double *gi = a.Gm + (int64_t)i * ld;
         double t = 0;
+#pragma unroll 8
         for (int j = lane; j < i; j += 32) t = fma(__ldcg(gi + j), __ldcg(a.red + j), t);
         t = warp_sum(t);
-        if (lane == 0) {
-            const double hi = __ldcg(a.red + i) - t;
-            a.h[i] = hi;
-        }
+        if (lane == 0) a.h[i] = __ldcg(a.red + i) - t;
     }
 }
 
@@ -303,13 +402,13 @@ __device__ __forceinline__ double gm_combine(double t, const double *c, const do
     return t;
 }
 
-// v_{it+1} = w - sum_i h_i v_i and ||v_{it+1}||^2; u = Q h; last block: the new rotation and
-// FreeFEM's stopping tests.  A block takes a.rows elements at a time, 256 / rows threads each on a
+// v_{it+1} = w - sum_i h_i v_i and ||v_{it+1}||^2 by blocks; u = Q h.  A block takes a.rows elements at a time, 256 / rows threads each on a
 // part of the vectors, so that small systems use all SMs (n = 9282, it = 190: 37 blocks of one
-// thread per element took 53.5 us with the rotations, 14.6 us now).
+// thread per element took 53.5 us with the rotations, 8.9 us now).
 __global__ void __launch_bounds__(kGmThreads) gm_update(GmArgs a) {
     __shared__ double hs[kGmHs], pt[kGmThreads];
-    __shared__ double sh[kGmWarps + 1], rot[2];
+    __shared__ double sh[kGmWarps + 1];
+    if (a.sc->stop) return;
     const int it = a.sc->it;
     const int ni = it + 1, ld = a.m + 1;
     const double *hh = a.h;
@@ -347,46 +446,7 @@ __global__ void __launch_bounds__(kGmThreads) gm_update(GmArgs a) {
         if (lane == 0) a.u[i] = t;
     }
     const double tot = gm_block_sum(s, sh);
-    if (!gm_last_block(&tot, 1, a.part, a.red + 2 * (a.m + 1), &a.sc->ticket)) return;
-    GmScal *c = a.sc;
-    if (threadIdx.x == 0) {
-        const double aux = sqrt(a.red[2 * (a.m + 1)]);
-        a.vnorm[it + 1] = aux;
-        const double hd = __ldcg(a.u + it), hs1 = aux;
-        const double sq = sqrt(hd * hd + hs1 * hs1);
-        const double c0 = hd / sq, s0 = hs1 / sq;
-        rot[0] = c0;
-        rot[1] = s0;
-        a.R[(int64_t)it * ld + it] = c0 * hd + s0 * hs1;
-        a.g[it + 1] = -s0 * a.g[it];
-        a.g[it] = c0 * a.g[it];
-        const double relres = fabs(a.g[it + 1]);
-        c->relres = relres;
-        c->steps += 1;
-        c->itf = it;
-        bool stop = false;
-        if (relres / c->normb < fabs(c->eps)) {
-            c->conv = 1;
-            stop = true;
-        } else if (it > c->itmax) {
-            stop = true;                       // FreeFEM: `if (it > nbitermx) break;`
-        } else {
-            c->it = it + 1;                    // the loop increment it++, iter++
-            c->iter += 1;
-            if (it + 1 >= a.m) { stop = true; c->itf = a.m - 1; }
-        }
-        c->stop = stop;
-        if (stop && a.in_graph) gm_set_cond(a.cond, 0);
-    }
-    __syncthreads();
-    // the column of the triangle, and Q with the new rotation of its rows it and it + 1
-    double *q0 = a.Q + (int64_t)it * (ld + 1), *q1 = q0 + ld + 1;
-    for (int i = threadIdx.x; i <= it + 1; i += blockDim.x) {
-        if (i < it) a.R[(int64_t)it * ld + i] = __ldcg(a.u + i);
-        const double q = i <= it ? __ldcg(q0 + i) : 0.0;
-        q0[i] = i <= it ? rot[0] * q : rot[1];
-        q1[i] = i <= it ? -rot[1] * q : rot[0];
-    }
+    if (threadIdx.x == 0) a.nrm[blockIdx.x] = tot;
 }
 
 // y = R^-1 g on the it+1 leading rows, column by column: y_i, then g_j -= R(j,i) y_i for all j < i
@@ -482,15 +542,16 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
     int64_t slab_len = kGmSub;
     gm_dot_shape(n, nslab, ngrp, slab_len);
     const int rows = gm_rows(n);
-    const int Gv = gm_vec_grid(n), Gd = nslab * ngrp, Gc = gm_coef_grid(m);
+    const int Gv = gm_vec_grid(n), Gd = 1 + nslab * ngrp, Gc = gm_coef_grid(m);
     const int Gu = (int)std::max<int64_t>(1, std::min<int64_t>(4 * kNumSM, ((int64_t)n + rows - 1) / rows));
     const size_t bsmem = sizeof(double) * 2 * ((size_t)m + 1);
     // workspace: V (m+1 vectors), Vp (m), the SpMV input and output, the small arrays
-    // R, Q, u g y vnorm, Gram, h, red, part, then the scalars (in doubles, rounded up)
+    // R, Q, u g y, Gram, h, red, part, nrm, tick, then the scalars (in doubles, rounded up)
     const size_t nscal = (sizeof(GmScal) + sizeof(double) - 1) / sizeof(double);
-    const size_t npart = std::max({2 * (size_t)(m + 1) * nslab, (size_t)Gv, (size_t)Gu});
-    const size_t small = (size_t)(m + 2) * (m + 1) + (size_t)(m + 2) * (m + 2) + 4 * (size_t)(m + 2) +
-                         (size_t)(m + 1) * (m + 1) + (size_t)(m + 2) + (2 * (size_t)(m + 1) + 2) + npart + nscal;
+    const size_t ntick = ((size_t)ngrp + 1) / 2;   // one counter per vector group of gm_dots
+    const size_t npart = std::max(2 * (size_t)(m + 1) * nslab, (size_t)Gv);
+    const size_t small = (size_t)(m + 2) * (m + 1) + (size_t)(m + 2) * (m + 2) + 3 * (size_t)(m + 2) +
+                         (size_t)(m + 1) * (m + 1) + (size_t)(m + 2) + 2 * (size_t)(m + 1) + npart + (size_t)Gu + ntick + nscal;
     double *ws = nullptr;
     const size_t nvec = (size_t)(2 * m + 3);
     FFGPU_CUDA(dalloc(ctx, (void **)&ws, sizeof(double) * (nvec * vs + small)));
@@ -501,16 +562,18 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
     a.V = ws; a.Vp = ws + (size_t)(m + 1) * vs; a.vpc = a.Vp + (size_t)m * vs; a.w = a.vpc + vs;
     double *sm = a.w + vs;
     a.rows = rows;
+    a.nupd = Gu;
     a.R = sm; sm += (size_t)(m + 2) * (m + 1);
     a.Q = sm; sm += (size_t)(m + 2) * (m + 2);
     a.u = sm; sm += m + 2;
     a.g = sm; sm += m + 2;
     a.y = sm; sm += m + 2;
-    a.vnorm = sm; sm += m + 2;
     a.Gm = sm; sm += (size_t)(m + 1) * (m + 1);
     a.h = sm; sm += m + 2;
-    a.red = sm; sm += 2 * (m + 1) + 2;
+    a.red = sm; sm += 2 * (m + 1);
     a.part = sm; sm += npart;
+    a.nrm = sm; sm += Gu;
+    a.tick = reinterpret_cast<int *>(sm); sm += ntick;
     a.sc = reinterpret_cast<GmScal *>(sm);
     sm += nscal;
     if ((size_t)(sm - ws) != nvec * vs + small) {
@@ -519,6 +582,7 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
     }
     a.x = x; a.b = b; a.dinv = A->diag_inv; a.wcl = A->wcl; a.use_wcl = A->ntgv > 0;
     FFGPU_CUDA(cudaMemsetAsync(a.sc, 0, sizeof(GmScal), s));
+    FFGPU_CUDA(cudaMemsetAsync(a.tick, 0, sizeof(int) * ngrp, s));
     FFGPU_CUDA(cudaFuncSetAttribute((const void *)gm_dots, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem));
     FFGPU_CUDA(cudaFuncSetAttribute((const void *)gm_back, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
     int rc = FFGPU_OK;
@@ -621,7 +685,7 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
                 if (hs.stop) break;
                 gm_prep<<<Gv, kGmThreads, 0, s>>>(a);
                 if ((rc = spmv(A, a.vpc, a.w, trans, s))) break;
-                gm_dots<<<Gd, kGmThreads, dsmem, s>>>(a);
+                gm_dots<<<Gd, kGmThreads, dsmem, s>>>(a);   // may say stop: the two kernels below then return
                 gm_coef<<<Gc, kGmThreads, 0, s>>>(a);
                 gm_update<<<Gu, kGmThreads, 0, s>>>(a);
                 ctx->launches += 4;
@@ -641,7 +705,7 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
             break;
         }
         ++cycles;
-        if (!host_loop) ctx->launches += 4 + 5 * (hs.steps - steps_seen);
+        if (!host_loop) ctx->launches += 4 + 5 * (hs.steps - steps_seen + 1);   // the step that stops the cycle too
         steps_seen = hs.steps;
         if (hs.conv) break;
         if (hs.iter > itmax) break;

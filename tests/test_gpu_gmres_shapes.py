@@ -56,3 +56,17 @@ def test_long_column():
     S = sp.csr_matrix((vl, cl, rp), (A.n, A.n))
     free = S.diagonal() < 1e20
     assert np.linalg.norm((b - S @ u)[free]) <= 1e-9 * np.linalg.norm(b)
+
+
+def test_one_vector_cycles():
+    """Restarts after every step: the cycle's only step is finished by the step that is not taken."""
+    Th = square(2, 3)
+    Vh = FESpace(Th, "P1")
+    b = np.empty(Vh.ndof)
+    A = ffgpu.matrix(ffgpu.varf_diffusion(f=1.0, on=(1, 2, 3, 4)), Vh, solver="GMRES", eps=1e-10, dim_krylov=1,
+                     itmax=40000, rhs_out=b)
+    u = A.solve(b)
+    rp, cl, vl = A.csr()
+    S = sp.csr_matrix((vl, cl, rp), (A.n, A.n))
+    free = S.diagonal() < 1e20
+    assert np.linalg.norm((b - S @ u)[free]) <= 1e-9 * np.linalg.norm(b)
