@@ -21,6 +21,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "ffgpu_internal.cuh"
 #include "ffgpu_sell.cuh"
 
@@ -34,7 +36,7 @@ struct InnerScalars {
     float gcg, gcgp, eps2, rho, gamma, s_gh, s_hq, pad0;
     int iter, itmax, done, converged;
     unsigned int ticket;
-    int pad1;
+    int fail;   // a wait for staged entries ran out
 };
 
 __device__ __noinline__ void ir_graph_stop(cudaGraphConditionalHandle cond) { cudaGraphSetConditional(cond, 0); }
@@ -61,6 +63,170 @@ __global__ void __launch_bounds__(sell_threads(BS, ASSIGN)) ir_ka(SellArgs S, co
             }
         }
     });
+    float tot;
+    float p = block_sum_t(hq, sh);
+    if (last_block_sum(p, part, &ks->ticket, &tot, sh)) { ks->s_hq = tot; ks->rho = -ks->s_gh / tot; }
+}
+
+// K_a of scalar rows with the matrix staged through shared memory.  A chunk's columns and values are
+// contiguous; each warp keeps kRingStages stages of kRingSlots slots filled ahead of its lanes by
+// bulk copies (one mbarrier per stage, lane 0 issues), and the lanes read their entries from
+// there.  In the plain form each batch of slots waits for its columns, then for the gathers they give,
+// with the stream idle meanwhile (P1 on 120^3 cells: 173 MB from memory at 35 % of its rate, nine warps
+// per scheduler nearly all waiting for loads); here only the gathers, from L1 and L2, are waited for.
+// Same products in the same order as ir_ka.  P1 on 120^3 cells: 36.2 us for the stride with the deep
+// row loop, 29.6 us (26.6 us at the copy rate of memory); two stages of 16 slots and four blocks per
+// SM 32.6 us in the tuner, three and three 34.0, four and two 37.1, four of 8 slots 35.4; chunks
+// in ranges 35.0.
+constexpr int kRingSlots = 16, kRingStages = 2;
+constexpr unsigned long long kRingWaitNs = 1000000000ull;
+static inline size_t ring_bytes(bool c16) {
+    return (size_t)kMxWarps * kRingStages * kRingSlots * 32 * (sizeof(float) + (c16 ? 2 : 4));
+}
+
+__device__ __forceinline__ uint32_t ring_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ring_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar, uint64_t pol) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(dst),
+        "l"(src), "r"(bytes), "r"(bar), "l"(pol)
+        : "memory");
+}
+__device__ __forceinline__ uint32_t ring_try(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done;
+}
+// whole warp; false when the second allowed runs out
+__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
+    uint32_t ok = ring_try(bar, parity);
+    if (!__all_sync(0xffffffffu, ok)) {
+        unsigned long long t0, t;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+        do {
+            ok = ring_try(bar, parity);
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        } while (!__all_sync(0xffffffffu, ok) && __any_sync(0xffffffffu, t - t0 <= kRingWaitNs));
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+
+template <bool C16>
+__global__ void __launch_bounds__(kMxThreads) ir_ka_ring(SellArgs S, const float *__restrict__ val,
+                                                         const float *__restrict__ h, float *__restrict__ q,
+                                                         InnerScalars *ks, float *part) {
+    using Col = std::conditional_t<C16, int16_t, int32_t>;
+    constexpr int kRow = kRingSlots * 32;   // entries of a stage
+    extern __shared__ __align__(128) unsigned char ring[];
+    __shared__ unsigned long long bars[kMxWarps][kRingStages];
+    __shared__ float sh[32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float *vr = reinterpret_cast<const float *>(ring) + warp * kRingStages * kRow;
+    const Col *cr = reinterpret_cast<const Col *>(ring + kMxWarps * kRingStages * kRow * sizeof(float)) + warp * kRingStages * kRow;
+    const uint32_t bar = ring_u32(bars[warp]), vs = ring_u32(vr), cs = ring_u32(cr);
+    const Col *cg = C16 ? reinterpret_cast<const Col *>(S.col16) : reinterpret_cast<const Col *>(S.col);
+    // the warp's chunks chunk(0) .. chunk(K - 1): the rotated stride
+    const int w = blockIdx.x * kMxWarps + warp, nw = gridDim.x * kMxWarps;
+    const auto chunk = [&](int k) { return k * nw + (w + 5 * k) % nw; };
+    int K = S.nchunk / nw;
+    if (chunk(K) < S.nchunk) ++K;
+    // lengths and offsets of 32 chunks at a time, one per lane
+    int plen = 0, poff = 0, clen = 0;
+    const auto lengths = [&](int k) { return k + lane < K ? __ldg(S.len + chunk(k + lane)) : 0; };
+    const auto offsets = [&](int k) { return k + lane < K ? __ldg(S.off + chunk(k + lane)) : 0; };
+    uint64_t pol = 0;
+    int pk = 0, pj = 0, pst = 0;   // the next stage to fill: slots pj .. of chunk pk, into stage pst
+    const auto produce = [&]() {
+        if (pk >= K) return;
+        const int L = __shfl_sync(0xffffffffu, plen, pk & 31), o = __shfl_sync(0xffffffffu, poff, pk & 31);
+        if (lane == 0) {
+            const int m = min(kRingSlots, L - pj);
+            const int64_t e = ((int64_t)o + pj) * 32;
+            const uint32_t b = bar + 8 * pst, bv = m * 32 * (uint32_t)sizeof(float), bc = m * 32 * (uint32_t)sizeof(Col);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bv + bc) : "memory");
+            if (m > 0) {
+                ring_copy(vs + pst * kRow * (uint32_t)sizeof(float), val + e, bv, b, pol);
+                ring_copy(cs + pst * kRow * (uint32_t)sizeof(Col), cg + e, bc, b, pol);
+            }
+        }
+        pst = pst + 1 == kRingStages ? 0 : pst + 1;
+        pj += kRingSlots;
+        if (pj >= L) {
+            pj = 0;
+            ++pk;
+            if ((pk & 31) == 0) {
+                plen = lengths(pk);
+                poff = offsets(pk);
+            }
+        }
+    };
+    plen = clen = lengths(0);
+    poff = offsets(0);
+    int issued = 0;
+    if (lane == 0) {
+        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+        for (int k = 0; k < kRingStages; ++k)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar + 8 * k), "r"(1) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    // the matrix is no kernel's output in the loop: its first slots need not wait for h
+    for (; issued < kRingStages && pk < K; ++issued) produce();
+    griddep_wait();
+    if (ks->done) {             // nothing to do but to see the copies home
+        for (int k = 0; k < issued; ++k) ring_wait(bar + 8 * k, 0);
+        return;
+    }
+    float hq = 0;
+    bool ok = true;
+    if (K > 0) {
+        int a = __ldg(S.perm + (int64_t)chunk(0) * 32 + lane), st = 0;
+        uint32_t ph = 0;
+        for (int k = 0; k < K && ok; ++k) {
+            if (k > 0 && (k & 31) == 0) clen = lengths(k);
+            const int L = __shfl_sync(0xffffffffu, clen, k & 31);
+            const int an = k + 1 < K ? __ldg(S.perm + (int64_t)chunk(k + 1) * 32 + lane) : 0;
+            const int ar = a < 0 ? 0 : a;
+            const float hv = __ldg(h + ar);
+            float y = 0;
+            int j = 0;
+            do {
+                const int m = min(kRingSlots, L - j);
+                ok = ring_wait(bar + 8 * st, ph);
+                if (!ok) break;
+                const float *vt = vr + st * kRow + lane;
+                const Col *ct = cr + st * kRow + lane;
+                float av[kRingSlots], xv[kRingSlots];
+#pragma unroll
+                for (int u = 0; u < kRingSlots; ++u)
+                    if (u < m) {
+                        av[u] = vt[32 * u];
+                        xv[u] = __ldg(h + ((C16 ? ar : 0) + (int)ct[32 * u]));
+                    }
+#pragma unroll
+                for (int u = 0; u < kRingSlots; ++u)
+                    if (u < m) y = fmaf(av[u], xv[u], y);
+                __syncwarp();   // all lanes have read the stage: it takes the next slots
+                produce();
+                if (++st == kRingStages) { st = 0; ph ^= 1u; }
+                j += kRingSlots;
+            } while (j < L);
+            if (a >= 0 && ok) {
+                q[a] = y;
+                hq = fmaf(hv, y, hq);
+            }
+            a = an;
+        }
+        if (!ok) {
+            // give the copies under way the same time again, so that none outlives the block
+            for (int i = 0; i < issued; ++i, st = st + 1 == kRingStages ? 0 : st + 1, ph ^= st == 0) ring_wait(bar + 8 * st, ph);
+            if (lane == 0) ks->fail = 1;
+        }
+    }
     float tot;
     float p = block_sum_t(hq, sh);
     if (last_block_sum(p, part, &ks->ticket, &tot, sh)) { ks->s_hq = tot; ks->rho = -ks->s_gh / tot; }
@@ -216,7 +382,7 @@ __global__ void ir_inner_keep(InnerScalars *ks, const double *out3, float eps_in
     ks->gcg = gcg; ks->gcgp = gcg;
     ks->eps2 = eps_in * eps_in * gcg;
     ks->iter = 0; ks->itmax = itmax; ks->converged = 0; ks->done = gcg < 1e-30f ? 1 : 0;
-    ks->ticket = 0u;
+    ks->ticket = 0u; ks->fail = 0;
 }
 
 __global__ void ir_inner_init(InnerScalars *ks, const double *out3, float eps_in, int itmax) {
@@ -224,7 +390,7 @@ __global__ void ir_inner_init(InnerScalars *ks, const double *out3, float eps_in
     ks->gcg = gcg; ks->gcgp = gcg; ks->s_gh = (float)out3[2];
     ks->eps2 = eps_in * eps_in * gcg;
     ks->iter = 0; ks->itmax = itmax; ks->converged = 0; ks->done = gcg < 1e-30f ? 1 : 0;
-    ks->ticket = 0u;
+    ks->ticket = 0u; ks->fail = 0;
 }
 
 __global__ void ir_update_kernel(int n, double *__restrict__ x, const float *__restrict__ d) {
@@ -253,11 +419,19 @@ struct IRState {
 // layout codes shared with the FP64 tuner: 64 + chunk assignment + 2 * deep unroll
 constexpr int kSellCode = 64;
 
+// code 5 (stride, batch) of scalar rows: staged
+static bool ir_ring(int kind) { return kind == kSellCode + 5; }
+static size_t ir_ka_smem(const ffgpu_matrix *A, int kind) { return ir_ring(kind) ? ring_bytes(A->scol16) : 0; }
 static void *ir_ka_fn(const ffgpu_matrix *A, int kind) {
     const int code = kind >= kSellCode ? kind - kSellCode : 0;
+    if (ir_ring(kind)) {
+        void *f = A->scol16 ? (void *)ir_ka_ring<true> : (void *)ir_ka_ring<false>;
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring_bytes(A->scol16));
+        return f;
+    }
 #define FFGPU_IR_ROW(BS, C16, T)                                                                     \
-    {(void *)ir_ka<BS, C16, 0, false, T>, (void *)ir_ka<BS, C16, 1, false, T>, (void *)ir_ka<BS, C16, 0, true, T>, \
-     (void *)ir_ka<BS, C16, 1, true, T>}
+    {BS == 3 ? (void *)ir_ka<3, C16, 0, false, T> : nullptr, (void *)ir_ka<BS, C16, 1, false, T>,    \
+     (void *)ir_ka<BS, C16, 0, true, T>, (void *)ir_ka<BS, C16, 1, true, T>}
     static void *const t[4][4] = {FFGPU_IR_ROW(1, false, 1), FFGPU_IR_ROW(1, true, 1), FFGPU_IR_ROW(3, false, 1),
                                   FFGPU_IR_ROW(3, false, 4)};
 #undef FFGPU_IR_ROW
@@ -265,10 +439,10 @@ static void *ir_ka_fn(const ffgpu_matrix *A, int kind) {
 }
 // grids: the FP32 K_a by the chunks it has to take, the vector kernels by the n/4 float4 quads
 static int ir_ka_assign(int kind) { return kind >= kSellCode ? (kind - kSellCode) & 1 : kSellRanges; }
-static int ir_ka_grid(const ffgpu_matrix *A, const void *ka, int assign) {
+static int ir_ka_grid(const ffgpu_matrix *A, const void *ka, int assign, size_t smem) {
     return A->bs == 3 && assign == kSellStride
                ? sell_spread_grid(A->nchunk)
-               : sized_grid(ka, kMxWarps * 32, ((int64_t)A->nchunk + kMxWarps - 1) / kMxWarps);
+               : sized_grid(ka, kMxWarps * 32, ((int64_t)A->nchunk + kMxWarps - 1) / kMxWarps, smem);
 }
 static int ir_vec_grid(const void *k, int n) {
     return min(4096, sized_grid(k, kMxThreads, ((int64_t)n / 4 + kMxThreads - 1) / kMxThreads));
@@ -284,7 +458,8 @@ static int ir_body(ffgpu_matrix *A, IRState &S, int unroll, cudaGraphConditional
     SellArgs sa = sell_args(A);
     const float *sv = A->sval32;
     void *ka = ir_ka_fn(A, A->sell32_kind);
-    const int assign = ir_ka_assign(A->sell32_kind), gka = ir_ka_grid(A, ka, assign);
+    const size_t smem = ir_ka_smem(A, A->sell32_kind);
+    const int assign = ir_ka_assign(A->sell32_kind), gka = ir_ka_grid(A, ka, assign, smem);
     if (ir_ranges(A)) FFGPU_TRY(sell_partition(A, gka * kMxWarps, &sa.part));
     const int gkb = ir_vec_grid((const void *)ir_kb, A->n);
     const int gkc = ir_vec_grid((const void *)ir_kc, A->n);
@@ -294,7 +469,7 @@ static int ir_body(ffgpu_matrix *A, IRState &S, int unroll, cudaGraphConditional
         void *aa[] = {&sa, &sv, &S.h, &S.q, &S.ks, &part};
         void *ab[] = {&n, &S.d, &S.g, &S.h, &S.q, &S.dinv, &S.ks, &part, &cond, &in_graph};
         void *ac[] = {&n, &S.g, &S.h, &S.dinv, &S.ks, &part};
-        launch_ex(ka, gka, sell_threads(A->bs, assign), aa, 0, s, pdl);
+        launch_ex(ka, gka, sell_threads(A->bs, assign), aa, smem, s, pdl);
         launch_ex((const void *)ir_kb, gkb, kMxThreads, ab, 0, s, pdl);
         launch_ex((const void *)ir_kc, gkc, kMxThreads, ac, 0, s, pdl);
     }
@@ -305,6 +480,14 @@ static int ir_body(ffgpu_matrix *A, IRState &S, int unroll, cudaGraphConditional
 static int ir_tune(ffgpu_matrix *A, IRState &S) {
     if (A->sell32_kind) return FFGPU_OK;
     ffgpu_ctx *ctx = A->ctx;
+    // FFGPU_IR_LAYOUT: one of the candidates by its code, untimed
+    if (const char *e = getenv("FFGPU_IR_LAYOUT")) {
+        const int code = atoi(e), c = code - kSellCode;
+        if (A->bs == 1 ? c == 1 || c == 2 || c == 3 || c == 5 : c >= 0 && c < 4) {
+            A->sell32_kind = code;
+            return FFGPU_OK;
+        }
+    }
     if (const int known = tuned_layout(ctx, A, 2)) {
         A->sell32_kind = known;
         return FFGPU_OK;
@@ -316,19 +499,24 @@ static int ir_tune(ffgpu_matrix *A, IRState &S) {
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     float tms[4];
-    const int kinds[4] = {kSellCode, kSellCode + 1, kSellCode + 2, kSellCode + 3};
-    const char *names[4] = {"ranges", "stride", "ranges deep", "stride deep"};
+    // scalar rows: the staged form in place of plain ranges, which were never the fastest there
+    const int scalar[4] = {kSellCode + 1, kSellCode + 2, kSellCode + 3, kSellCode + 5};
+    const int blocks[4] = {kSellCode, kSellCode + 1, kSellCode + 2, kSellCode + 3};
+    const int *kinds = A->bs == 1 ? scalar : blocks;
+    const char *names[6] = {"ranges", "stride", "ranges deep", "stride deep", "", "stride staged"};
     for (int kk = 0; kk < 4; ++kk) {
+        const int assign = ir_ka_assign(kinds[kk]);
         SellArgs sa = sell_args(A);
         const float *sv = A->sval32;
         void *ka = ir_ka_fn(A, kinds[kk]);
-        const int g = ir_ka_grid(A, ka, kk & 1);
-        if ((kk & 1) == kSellRanges) FFGPU_TRY(sell_partition(A, g * kMxWarps, &sa.part));
+        const size_t smem = ir_ka_smem(A, kinds[kk]);
+        const int g = ir_ka_grid(A, ka, assign, smem);
+        if (assign == kSellRanges) FFGPU_TRY(sell_partition(A, g * kMxWarps, &sa.part));
         float *part = (float *)ctx->d_part;
         void *aa[] = {&sa, &sv, &S.h, &S.q, &S.ks, &part};
-        cudaLaunchKernel(ka, g, sell_threads(A->bs, kk & 1), aa, 0, s);
+        cudaLaunchKernel(ka, g, sell_threads(A->bs, assign), aa, smem, s);
         cudaEventRecord(e0, s);
-        for (int r = 0; r < 3; ++r) cudaLaunchKernel(ka, g, sell_threads(A->bs, kk & 1), aa, 0, s);
+        for (int r = 0; r < 3; ++r) cudaLaunchKernel(ka, g, sell_threads(A->bs, assign), aa, smem, s);
         cudaEventRecord(e1, s);
         FFGPU_CUDA(cudaEventSynchronize(e1));
         FFGPU_CUDA(cudaGetLastError());
@@ -336,7 +524,7 @@ static int ir_tune(ffgpu_matrix *A, IRState &S) {
         float ms = 0;
         cudaEventElapsedTime(&ms, e0, e1);
         if (getenv("FFGPU_VERBOSE"))
-            fprintf(stderr, "ffgpu: FP32 SpMV tuner (%d block rows): sell32 %s %.4f ms\n", A->nb, names[kk],
+            fprintf(stderr, "ffgpu: FP32 SpMV tuner (%d block rows): sell32 %s %.4f ms\n", A->nb, names[kinds[kk] - kSellCode],
                     ms / 3);
         tms[kk] = ms;
     }
@@ -362,7 +550,8 @@ int ir_time_ka(ffgpu_matrix *A, int nrep, float *ms) {
     SellArgs sa = sell_args(A);
     const float *sv = A->sval32;
     void *ka = ir_ka_fn(A, A->sell32_kind);
-    const int assign = ir_ka_assign(A->sell32_kind), g = ir_ka_grid(A, ka, assign);
+    const size_t smem = ir_ka_smem(A, A->sell32_kind);
+    const int assign = ir_ka_assign(A->sell32_kind), g = ir_ka_grid(A, ka, assign, smem);
     int rc = FFGPU_OK;
     if (ir_ranges(A)) rc = sell_partition(A, g * kMxWarps, &sa.part);
     float t = 0;
@@ -372,9 +561,9 @@ int ir_time_ka(ffgpu_matrix *A, int nrep, float *ms) {
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
-        cudaLaunchKernel(ka, g, sell_threads(A->bs, assign), aa, 0, s);
+        cudaLaunchKernel(ka, g, sell_threads(A->bs, assign), aa, smem, s);
         cudaEventRecord(e0, s);
-        for (int r = 0; r < nrep; ++r) cudaLaunchKernel(ka, g, sell_threads(A->bs, assign), aa, 0, s);
+        for (int r = 0; r < nrep; ++r) cudaLaunchKernel(ka, g, sell_threads(A->bs, assign), aa, smem, s);
         cudaEventRecord(e1, s);
         cudaError_t e = cudaEventSynchronize(e1);
         if (e == cudaSuccess) e = cudaEventElapsedTime(&t, e0, e1);
@@ -398,7 +587,8 @@ static int ir_build_graph(ffgpu_matrix *A, IRState &S, int unroll) {
     // the warp partition is built before the capture starts (no allocation inside a capture)
     if (ir_ranges(A)) {
         const int32_t *part = nullptr;
-        FFGPU_TRY(sell_partition(A, ir_ka_grid(A, ir_ka_fn(A, A->sell32_kind), kSellRanges) * kMxWarps, &part));
+        FFGPU_TRY(sell_partition(A, ir_ka_grid(A, ir_ka_fn(A, A->sell32_kind), kSellRanges,
+                                                ir_ka_smem(A, A->sell32_kind)) * kMxWarps, &part));
     }
     // with programmatic dependent launch between the body's kernels first, else the plain graph
     cudaError_t e = cudaErrorUnknown;
@@ -565,6 +755,9 @@ int ffgpu_solve_ir(ffgpu_matrix *A, const double *b, double *x, const ffgpu_ir_p
         InnerScalars hk;
         cudaMemcpyAsync(&hk, S.ks, sizeof(hk), cudaMemcpyDeviceToHost, s);
         cudaStreamSynchronize(s);
+        if (hk.fail) {
+            set_error("ffgpu_solve_ir: a copy of matrix entries did not arrive"); rc = FFGPU_ECUDA; break;
+        }
         inner_total += hk.iter;
         if (fresh && first_its < 0) first_its = hk.iter;
         if (!fresh && !hk.converged) {
