@@ -56,6 +56,7 @@ enum DevStatus : int {
 
 // Scalars of a running Krylov solve, kept in device memory so the iteration loop runs
 // inside one CUDA graph without host round trips.
+constexpr int kWaitRanOut = 2;   // KrylovScalars::done when a wait in a kernel ran out
 struct KrylovScalars {
     double gcg, gcgp, eps2, rho, gamma, s_gh, s_hq;
     double gcg0;

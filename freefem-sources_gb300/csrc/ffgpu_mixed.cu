@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "ffgpu_internal.cuh"
+#include "ffgpu_ring.cuh"
 #include "ffgpu_sell.cuh"
 
 namespace ffgpu {
@@ -79,40 +80,8 @@ __global__ void __launch_bounds__(sell_threads(BS, ASSIGN)) ir_ka(SellArgs S, co
 // SM 32.6 us in the tuner, three and three 34.0, four and two 37.1, four of 8 slots 35.4; chunks
 // in ranges 35.0.
 constexpr int kRingSlots = 16, kRingStages = 2;
-constexpr unsigned long long kRingWaitNs = 1000000000ull;
 static inline size_t ring_bytes(bool c16) {
     return (size_t)kMxWarps * kRingStages * kRingSlots * 32 * (sizeof(float) + (c16 ? 2 : 4));
-}
-
-__device__ __forceinline__ uint32_t ring_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void ring_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar, uint64_t pol) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(dst),
-        "l"(src), "r"(bytes), "r"(bar), "l"(pol)
-        : "memory");
-}
-__device__ __forceinline__ uint32_t ring_try(uint32_t bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return done;
-}
-// whole warp; false when the second allowed runs out
-__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok = ring_try(bar, parity);
-    if (!__all_sync(0xffffffffu, ok)) {
-        unsigned long long t0, t;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-        do {
-            ok = ring_try(bar, parity);
-            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-        } while (!__all_sync(0xffffffffu, ok) && __any_sync(0xffffffffu, t - t0 <= kRingWaitNs));
-    }
-    return __all_sync(0xffffffffu, ok);
 }
 
 template <bool C16>
@@ -147,7 +116,7 @@ __global__ void __launch_bounds__(kMxThreads) ir_ka_ring(SellArgs S, const float
             const int m = min(kRingSlots, L - pj);
             const int64_t e = ((int64_t)o + pj) * 32;
             const uint32_t b = bar + 8 * pst, bv = m * 32 * (uint32_t)sizeof(float), bc = m * 32 * (uint32_t)sizeof(Col);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bv + bc) : "memory");
+            ring_expect(b, bv + bc);
             if (m > 0) {
                 ring_copy(vs + pst * kRow * (uint32_t)sizeof(float), val + e, bv, b, pol);
                 ring_copy(cs + pst * kRow * (uint32_t)sizeof(Col), cg + e, bc, b, pol);
@@ -168,10 +137,8 @@ __global__ void __launch_bounds__(kMxThreads) ir_ka_ring(SellArgs S, const float
     poff = offsets(0);
     int issued = 0;
     if (lane == 0) {
-        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-        for (int k = 0; k < kRingStages; ++k)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar + 8 * k), "r"(1) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        pol = ring_policy();
+        ring_init(bar, kRingStages);
     }
     __syncwarp();
     // the matrix is no kernel's output in the loop: its first slots need not wait for h

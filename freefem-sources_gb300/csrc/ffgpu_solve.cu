@@ -19,9 +19,11 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <type_traits>
 #include <vector>
 
 #include "ffgpu_internal.cuh"
+#include "ffgpu_ring.cuh"
 #include "ffgpu_sell.cuh"
 
 namespace ffgpu {
@@ -606,6 +608,128 @@ __global__ void __launch_bounds__(sell_threads(BS, ASSIGN)) cg_kax_sell(SellArgs
     }
 }
 
+// K_a of 3x3 blocks with the matrix staged through shared memory (FP64: V = double, x = h; double-float:
+// V = float2, x = the split h): one block of 16 warps per SM, five stages of one slot (32 blocks of
+// 72 bytes and their columns) per warp; the gathers of a slot are issued before the products of the
+// one before it.  The chunks and the order of a row's products are those of cg_ka_sell and cg_kax_sell
+// with the stride assignment.  Where a matrix is past the L2 the streams' latency shows in the plain form:
+// double-float [P2]^3 on 24^3 cells 72.6 -> 57.6 us, FP64 on 37^3 cells 219 -> 209 us (bound by its
+// products, 170 us); below, one block of 16 warps per SM has too few chunks each (17^3 cells:
+// 35.7 us, block CSR 32.7).  The tuner decides.
+constexpr int kStWarps = 16, kStStages = 5;
+constexpr int kStSlot = 32 * 9 * 8;   // bytes of a slot's values
+constexpr size_t kStBytes = (size_t)kStWarps * kStStages * (kStSlot + 32 * sizeof(int));
+template <typename V, int T>
+__global__ void __launch_bounds__(kStWarps * 32) cg_ka_staged(SellArgs S, const V *__restrict__ val, const V *__restrict__ x,
+                                                              const double *__restrict__ h, double *__restrict__ q,
+                                                              KrylovScalars *ks, double *part) {
+    static_assert(sizeof(V) == 8, "values of 8 bytes");
+    extern __shared__ __align__(128) unsigned char ring[];
+    __shared__ unsigned long long bars[kStWarps][kStStages];
+    __shared__ double sh[32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char *vb = ring + warp * kStStages * kStSlot;
+    const int *cb = reinterpret_cast<const int *>(ring + kStWarps * kStStages * kStSlot) + warp * kStStages * 32;
+    const uint32_t bar = ring_u32(bars[warp]), vs = ring_u32(vb), cs = ring_u32(cb);
+    uint64_t pol = 0;
+    if (lane == 0) {
+        pol = ring_policy();
+        ring_init(bar, kStStages);
+    }
+    __syncwarp();
+    // the producer's walk over the warp's chunks: slot pj of chunk w.c goes into stage pst next
+    ChunkWalk<kSellStride, 3> w(S);
+    int pL = 0, po = 0, nL = 0, no = 0, nc = w.c, pj = 0, pst = 0, made = 0, used = 0;
+    const auto chunk = [&](int c, int &L, int &o) {
+        L = c < w.ce ? __ldg(S.len + c) : 0;
+        o = c < w.ce ? __ldg(S.off + c) : 0;
+    };
+    const auto advance = [&]() {   // to the next chunk with slots, its successor's length under way
+        do {
+            if (nc != w.c) w.advance(nc);
+            pL = nL; po = no; pj = 0;
+            if (w.c >= w.ce) return;
+            nc = w.next();
+            chunk(nc, nL, no);
+        } while (pL == 0);
+    };
+    const auto produce = [&]() {
+        if (w.c >= w.ce) return;
+        if (lane == 0) {
+            const int64_t e = ((int64_t)po + pj) * 32;
+            const uint32_t b = bar + 8 * pst;
+            ring_expect(b, kStSlot + 128);
+            ring_copy(vs + pst * kStSlot, val + e * 9, kStSlot, b, pol);
+            ring_copy(cs + pst * 128, S.col + e, 128, b, pol);
+        }
+        pst = pst + 1 == kStStages ? 0 : pst + 1;
+        ++made;
+        if (++pj == pL) advance();
+    };
+    chunk(nc, nL, no);
+    advance();
+    // the matrix is no kernel's output in the loop: its first slots need not wait for h
+    for (int k = 0; k < kStStages; ++k) produce();
+    griddep_wait();
+    if (ks->done) {   // nothing to do but to see the copies home
+        for (int k = 0; k < made; ++k) ring_wait(bar + 8 * k, 0);
+        return;
+    }
+    double hq = 0;
+    bool ok = true;
+    int st = 0;
+    uint32_t ph = 0;
+    sell_for_chunks<kSellStride, 3>(S, [&](int c, int a, int L, int64_t sr) {
+        std::conditional_t<std::is_same_v<V, double>, AccF64, AccDF> acc[3];
+        V xv[3];
+        const auto gather = [&](V *d) {
+            const int64_t col = 3 * (int64_t)cb[st * 32 + lane];
+#pragma unroll
+            for (int m = 0; m < 3; ++m) d[m] = __ldg(x + col + m);
+        };
+        if (L > 0 && ok && (ok = ring_wait(bar + 8 * st, ph))) gather(xv);
+        for (int j = 0; j < L && ok; ++j) {
+            const V *v = reinterpret_cast<const V *>(vb + st * kStSlot) + lane;
+            if (++st == kStStages) { st = 0; ph ^= 1u; }
+            V xn[3];
+            if (j + 1 < L) {
+                if (!(ok = ring_wait(bar + 8 * st, ph))) break;
+                gather(xn);
+            }
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int m = 0; m < 3; ++m) acc[r].fma_(v[32 * (3 * r + m)], xv[m]);
+            __syncwarp();   // all lanes have read the stage: it takes the next slot
+            ++used;
+            produce();
+#pragma unroll
+            for (int m = 0; m < 3; ++m) xv[m] = xn[m];
+        }
+        double y[3];
+#pragma unroll
+        for (int m = 0; m < 3; ++m) y[m] = acc[m].get();
+        if (sell_reduce<3, T>(y, a, lane) && ok) {
+#pragma unroll
+            for (int m = 0; m < (T == 1 ? 3 : 1); ++m) {
+                const int64_t i = sell_dof<3, T>(a, lane) + m;
+                q[i] = y[m];
+                hq = fma(h[i], y[m], hq);
+            }
+        }
+    });
+    if (!ok) {   // give the copies under way the same time again, so that none outlives the block
+        for (int k = used; k < made; ++k) ring_wait(bar + 8 * (k % kStStages), (k / kStStages) & 1);
+        if (lane == 0) ks->done = kWaitRanOut;
+    }
+    double tot;
+    double p = block_sum(hq, sh);
+    if (last_block_total(p, part, &ks->ticket, &tot, sh)) {
+        ks->s_hq = tot;
+        ks->rho = -ks->s_gh / tot;
+    }
+}
+
 // y = A x (FP64)
 template <int BS, bool C16, int ASSIGN, int LOOP, int T = 1>
 __global__ void __launch_bounds__(sell_threads(BS, ASSIGN)) spmv_sell(SellArgs S, const double *__restrict__ val,
@@ -761,9 +885,13 @@ __global__ void transpose_kernel(int nb, int bs, const int32_t *brp, const int32
 constexpr int kSellCode = 64;
 // SELL codes: kSellCode + assign + 2 * loop; loop 0/1: unrolled row loop (plain, deep), 2/3
 // (FP64 kernels only): batched row loop (plain, deep)
+// 3x3 blocks: the stride assignment with the matrix staged through shared memory, FP64 and double-float
+// (in place of the batched and the deep row loop, which were the slowest or close to it there)
+constexpr int kStaged64 = kSellCode + 7, kStagedX = kSellCode + 3;
 static bool is_sell(int T) { return T >= kSellCode && T < kSellCode + 8; }
 static int sell_assign(int T) { return (T - kSellCode) & 1; }
-static const char *sell_name(int T) {
+static const char *sell_name(int T, bool staged) {
+    if (staged) return "sell32 stride staged";
     static const char *names[8] = {"sell32 ranges", "sell32 stride", "sell32 ranges deep", "sell32 stride deep",
                                    "sell32 ranges batch", "sell32 stride batch", "sell32 ranges batch deep",
                                    "sell32 stride batch deep"};
@@ -777,7 +905,7 @@ static int sell_format(const ffgpu_matrix *A) {
 }
 #define FFGPU_SELL_ROW(K, BS, C16, T)                                                                  \
     {(void *)K<BS, C16, 0, false, T>, (void *)K<BS, C16, 1, false, T>, (void *)K<BS, C16, 0, true, T>,  \
-     (void *)K<BS, C16, 1, true, T>}
+     BS == 3 ? nullptr : (void *)K<1, C16, 1, true, 1>}   /* 3x3 blocks: kStagedX */
 static void *cg_kax_sell_fn(const ffgpu_matrix *A, int code) {
     static void *const t[4][4] = {FFGPU_SELL_ROW(cg_kax_sell, 1, false, 1), FFGPU_SELL_ROW(cg_kax_sell, 1, true, 1),
                                   FFGPU_SELL_ROW(cg_kax_sell, 3, false, 1), FFGPU_SELL_ROW(cg_kax_sell, 3, false, 4)};
@@ -788,7 +916,7 @@ static void *cg_kax_sell_fn(const ffgpu_matrix *A, int code) {
 #define FFGPU_SELL64_ROW(K, BS, C16, T)                                                               \
     {(void *)K<BS, C16, 0, 0, T>, (void *)K<BS, C16, 1, 0, T>, (void *)K<BS, C16, 0, 1, T>,            \
      (void *)K<BS, C16, 1, 1, T>, (void *)K<BS, C16, 0, 2, T>, (void *)K<BS, C16, 1, 2, T>,            \
-     (void *)K<BS, C16, 0, 3, T>, (void *)K<BS, C16, 1, 3, T>}
+     (void *)K<BS, C16, 0, 3, T>, BS == 3 ? nullptr : (void *)K<1, C16, 1, 3, 1>}   /* 3x3 blocks: kStaged64 */
 #define FFGPU_SELL64_FN(K)                                                                            \
     static void *K##_fn(const ffgpu_matrix *A, int code) {                                            \
         static void *const t[4][8] = {FFGPU_SELL64_ROW(K, 1, false, 1), FFGPU_SELL64_ROW(K, 1, true, 1),   \
@@ -799,6 +927,15 @@ FFGPU_SELL64_FN(cg_ka_sell)
 FFGPU_SELL64_FN(spmv_sell)
 #undef FFGPU_SELL64_FN
 #undef FFGPU_SELL64_ROW
+
+// K_a staged through shared memory (3x3 blocks)
+static bool ka_staged(const ffgpu_matrix *A, int mode, int T) { return A->bs == 3 && T == (mode == 1 ? kStagedX : kStaged64); }
+template <typename V>
+static void *ka_staged_fn(const ffgpu_matrix *A) {
+    void *f = sell_lanes(A) == 4 ? (void *)cg_ka_staged<V, 4> : (void *)cg_ka_staged<V, 1>;
+    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStBytes);
+    return f;
+}
 
 // lanes per block row of the block-CSR kernels
 static int pick_lanes(const ffgpu_matrix *A) {
@@ -874,8 +1011,9 @@ struct KaCall {
     KrylovScalars *ks = nullptr;
     double *part = nullptr;
     void *args[7];
+    size_t smem = 0;
     cudaError_t launch(cudaStream_t s, bool pdl = false) {
-        return launch_ex(fn, grid, threads, args, 0, s, pdl);
+        return launch_ex(fn, grid, threads, args, smem, s, pdl);
     }
 };
 
@@ -898,14 +1036,23 @@ static int ka_setup(ffgpu_matrix *A, int mode, int trans, int T, const double *h
         k.sl = sell_args(A);
         if (mode == 1) {
             k.vx = trans ? A->svalx_t : A->svalx;
-            k.fn = cg_kax_sell_fn(A, T);
+            k.fn = ka_staged(A, 1, T) ? ka_staged_fn<float2>(A) : cg_kax_sell_fn(A, T);
             k.args[0] = &k.sl; k.args[1] = &k.vx; k.args[2] = &k.hx; k.args[3] = &k.h; k.args[4] = &k.q;
             k.args[5] = &k.ks; k.args[6] = &k.part;
         } else {
             k.v64 = trans ? A->sval_t : A->sval;
-            k.fn = cg_ka_sell_fn(A, T);
-            k.args[0] = &k.sl; k.args[1] = &k.v64; k.args[2] = &k.h; k.args[3] = &k.q; k.args[4] = &k.ks;
-            k.args[5] = &k.part;
+            const bool staged = ka_staged(A, 0, T);
+            k.fn = staged ? ka_staged_fn<double>(A) : cg_ka_sell_fn(A, T);
+            k.args[0] = &k.sl; k.args[1] = &k.v64; k.args[2] = &k.h;
+            void **r = k.args + 3;
+            if (staged) *r++ = &k.h;
+            r[0] = &k.q; r[1] = &k.ks; r[2] = &k.part;
+        }
+        if (ka_staged(A, mode, T)) {
+            k.smem = kStBytes;
+            k.threads = kStWarps * 32;
+            k.grid = sell_spread_grid(A->nchunk);
+            return FFGPU_OK;
         }
         return sell_launch_shape(A, k.fn, sell_assign(T), k.sl, &k.grid, &k.threads);
     }
@@ -998,7 +1145,7 @@ static int tune_lanes(ffgpu_matrix *A, int mode) {
             for (int c = 0; c < ncand; ++c)
                 fprintf(stderr, "ffgpu: SpMV tuner (mode %d, %d block rows, %lld blocks): %s%s %d %.4f ms\n", mode,
                         A->nb, (long long)A->nnzb, cands[c] == bestT ? "* " : "",
-                        is_sell(cands[c]) ? sell_name(cands[c]) : "bsr lanes", cands[c], tms[c]);
+                        is_sell(cands[c]) ? sell_name(cands[c], ka_staged(A, mode, cands[c])) : "bsr lanes", cands[c], tms[c]);
         FFGPU_CUDA(cudaMemsetAsync(ks, 0, sizeof(KrylovScalars), s));
         FFGPU_CUDA(cudaStreamSynchronize(s));
     }
@@ -1044,7 +1191,8 @@ int spmv(ffgpu_matrix *A, const double *x, double *y, int trans, cudaStream_t st
     const double *sv = trans ? A->sval_t : A->sval;
     if (sv) {
         SellArgs sl = sell_args(A);
-        const int code = is_sell(A->csr_lanes) ? A->csr_lanes : kSellCode;
+        int code = is_sell(A->csr_lanes) ? A->csr_lanes : kSellCode;
+        if (ka_staged(A, 0, code)) code = kSellCode + 1;   // the same chunks, plain
         void *fn = spmv_sell_fn(A, code);
         int grid = 0, threads = 0;
         FFGPU_TRY(sell_launch_shape(A, fn, sell_assign(code), sl, &grid, &threads));
@@ -1447,7 +1595,7 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     int bodies = bodies_host >= 0 ? bodies_host
                                   : (fused ? hk.iter / unroll + 1 : (hk.iter == 0 ? 1 : (hk.iter + unroll - 1) / unroll));
     if (use_graph) ctx->launches += (int64_t)bodies * A->cg_kernels_body;
-    FFGPU_CHECK(!loop || hk.done != 2, FFGPU_ECUDA, "CG loop: a wait between blocks ran out after %d iterations", hk.iter);
+    FFGPU_CHECK(hk.done != kWaitRanOut, FFGPU_ECUDA, "CG: a wait in a kernel ran out after %d iterations", hk.iter);
     if (st) {
         st->iterations = hk.iter;
         st->converged = hk.converged != 0;

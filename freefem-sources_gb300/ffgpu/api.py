@@ -536,8 +536,8 @@ class Matrix:
     def spmv_layout(self, mode=0):
         """The SpMV layout the tuner chose for mode 0 (FP64 CG), 1 (double-float CG) or 2 (FP32
         inner solve): 'sell32' (chunk ranges) or 'sell32-rot', with '-deep' for the deeper unroll and
-        '-batch' / '-batch-deep' for the batched row loop (mode 2: '-batch' is the form that stages the
-        entries through shared memory), 'bsr/T' (T lanes per block row) or None."""
+        '-batch' / '-batch-deep' for the batched row loop (staged through shared memory: 'sell32-rot-batch' in mode 2,
+        on 3x3 blocks 'sell32-rot-batch-deep' in mode 0 and 'sell32-rot-deep' in mode 1), 'bsr/T' (T lanes per block row) or None."""
         v = int(lib().ffgpu_matrix_spmv_layout(self.h, int(mode)))
         if v <= 0:
             return None
