@@ -1083,6 +1083,13 @@ static const int kCandsX[] = {kSellCode, kSellCode + 1, kSellCode + 2, kSellCode
 // K_a is launch-latency bound and the candidates' times differ by noise only
 constexpr int64_t kTuneMinEntries = 1 << 16;
 
+// 3x3 blocks, FP64: below this many block rows only block CSR is timed.  A SELL warp reads its chunk
+// range, then the chunk's rows, length and offset, then columns, before its first gather; between
+// the other kernels of an iteration that chain costs more than the tuner's repeated launches show.
+// Whole solves, block CSR and four-lane SELL (which the tuner prefers by 6 to 9 %): [P2]^3 on
+// 13 x 12 x 13 cells, 18 225 rows, 24.3 and 26.4 ms; 16^3, 35 937 rows, 42.3 and 41.7 ms.
+constexpr int kSellBlockRows = 24000;
+
 static bool layout_valid(int mode, int code) {
     const int *c = mode == 1 ? kCandsX : kCands64;
     const int n = mode == 1 ? 8 : 12;
@@ -1125,6 +1132,7 @@ static int tune_lanes(ffgpu_matrix *A, int mode) {
         for (int c = 0; c < ncand; ++c) tms[c] = 1e30f;
         for (int pass = 0; pass < 2; ++pass)
             for (int c = 0; c < ncand; ++c) {
+                if (mode == 0 && A->bs == 3 && A->nb < kSellBlockRows && is_sell(cands[c])) continue;
                 KaCall k;
                 FFGPU_TRY(ka_setup(A, mode, 0, cands[c], x, y, k));
                 k.launch(s);   // warm

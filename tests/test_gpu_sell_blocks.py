@@ -71,3 +71,12 @@ def test_one_lane_per_row_above_the_limit():
     z = A.mult(x)
     free = z.abs() < 1e20
     assert float((y - z)[free].abs().max()) <= 600 * 2.2e-16 * float(z[free].abs().max()) * 40
+
+
+@pytest.mark.parametrize("n", [(9, 10, 11), (14, 14, 13)])
+def test_small_block_matrices_take_block_csr(n):
+    """9 177 and 22 707 block rows: past the size that is tuned, below the one where SELL is timed."""
+    A, b, S = _elasticity(n)
+    u = A.solve(b)
+    assert A.layout_code() in (1, 2, 4, 8)
+    assert np.linalg.norm(S @ u - b) <= 1e-8 * np.linalg.norm(b)
