@@ -9,6 +9,7 @@
 // is two passes over the problem's rows and two CTA reductions: the SpMV forms the direction
 // h = gamma h_old - C g where it reads it (two direction buffers alternate), and the update
 // pass sums (g, Cg) and (g, h), from which (g, h_next) = gamma (g, h) - (g, Cg) follows.
+// Where the largest problem's vectors fit an SM they live in shared memory (batch_sm_kernel).
 // The launch sequence
 // (FP32 values, Jacobi, queue reset, persistent solve) is captured in a CUDA graph.  The CTA
 // size and lanes per SpMV row are picked by timing the candidates on the batch (autotune).

@@ -12,6 +12,8 @@
 // CG = C G is recomputed where it is used instead of being stored.  Small scalar systems (the
 // matrix in L2, an iteration bound by kernel boundaries) run two kernels per iteration: K_b
 // stores C G and the next K_a forms H = gamma H - C G at every column it gathers (cg_kca_sell).
+// By default scalar systems whose vectors fit the SMs run the whole loop in one cooperative kernel
+// instead (ffgpu_persist.cu), which needs no kernel boundaries at all.
 // The iteration loop is a CUDA graph `while` node whose condition K_b clears on convergence or
 // at itmax, so a whole solve is one graph launch with no host round trip.
 #include <math.h>
