@@ -1189,7 +1189,7 @@ static int pin_layout(ffgpu_matrix *A, int mode, int code) {
     *slot = code;
     if (A->cg_exec) { cudaGraphExecDestroy(A->cg_exec); A->cg_exec = nullptr; }
     if (!is_sell(code)) {
-        // spmv() takes the SELL copy whenever it exists: drop it so every SpMV uses the pin
+        // the losing copy is not kept
         ffgpu_ctx *ctx = A->ctx;
         if (mode == 1) { dfree(ctx, A->svalx); dfree(ctx, A->svalx_t); A->svalx = A->svalx_t = nullptr; }
         else { dfree(ctx, A->sval); dfree(ctx, A->sval_t); A->sval = A->sval_t = nullptr; }
@@ -1197,11 +1197,13 @@ static int pin_layout(ffgpu_matrix *A, int mode, int code) {
     return FFGPU_OK;
 }
 
+// y = A x in the matrix's own layout.  (A SELL copy that another kernel built beside a block-CSR layout is
+// not read: the summation order would depend on what ran before.)
 int spmv(ffgpu_matrix *A, const double *x, double *y, int trans, cudaStream_t st) {
     const double *sv = trans ? A->sval_t : A->sval;
-    if (sv) {
+    if (sv && is_sell(A->csr_lanes)) {
         SellArgs sl = sell_args(A);
-        int code = is_sell(A->csr_lanes) ? A->csr_lanes : kSellCode;
+        int code = A->csr_lanes;
         if (ka_staged(A, 0, code)) code = kSellCode + 1;   // the same chunks, plain
         void *fn = spmv_sell_fn(A, code);
         int grid = 0, threads = 0;
@@ -1513,6 +1515,9 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     const bool may_loop = mode == 0 && !cluster && !A->layout_pinned && in_kernel_loops();
     const bool band = may_loop && band_cg_fits(A);
     bool loop = band || (may_loop && loop_cg_fits(A));
+    // the initial residual is summed in the order of the matrix's layout, whatever ran before: the
+    // copy that cg_graph makes for the launches
+    if (loop && is_sell(A->csr_lanes)) FFGPU_TRY(sell_values(A, trans ? kSell64T : kSell64));
     if (!cluster && !loop) FFGPU_TRY(cg_graph(A, trans, unroll, mode, x, g, h, q, fused, h2, cgv));
     FFGPU_CUDA(cudaMemcpyAsync(x, xu, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     cudaEvent_t e0, e1;
