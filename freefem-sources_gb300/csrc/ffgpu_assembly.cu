@@ -314,11 +314,10 @@ __device__ __forceinline__ void store4(double *p, double a, double b, double c, 
 
 // Element matrices of int(c_stiff kappa grad u.grad v + c_mass u v) on P1, one thread each:
 //   grad phi_i = N_i / det with N_i the inward normals (cross products of edges), so
-//   K_ij = (kappa c_stiff / (DIM! det)) N_i.N_j, the pairs among the vertices 1..DIM as dot products
-//   and the others from the zero row sums (sum_i grad phi_i = 0).
+//   K_ij = (kappa c_stiff / (DIM! det)) N_i.N_j, one dot product per pair.
 // Row la of element e at out[(e * (DIM + 1) + la) * 4], four doubles wide (32-byte stores; the
-// row fill reads one sector).  FP64 issue bounds it (one warp instruction per 76 cycles and
-// sub-partition): about 75 FP64 operations per tetrahedron against about 60 for the gradients
+// row fill reads one sector).  FP64 issue bounds it (one warp instruction per 64 cycles and
+// sub-partition): about 90 FP64 operations per tetrahedron against about 60 for the gradients
 // alone, and none of the products is left to the row fill.
 template <int DIM>
 __global__ void __launch_bounds__(256) p1_elem_kernel(const double *__restrict__ X, const int32_t *__restrict__ elems, int nt,
@@ -339,14 +338,16 @@ __global__ void __launch_bounds__(256) p1_elem_kernel(const double *__restrict__
     const double w = (kappa ? kappa[e] : 1.0) * c_stiff / (DIM == 2 ? 2.0 * det : 6.0 * det);
     double K[NV][NV];
     if constexpr (DIM == 2) {
-        // edges opposite the vertices: e0 = V2 - V1, e1 = -V2, e2 = V1
-        const double x0 = V[1][0] - V[0][0], y0 = V[1][1] - V[0][1];
+        // edges opposite the vertices: e0 = P2 - P1, e1 = -V1, e2 = V0; every entry a product of its own (row
+        // sums would carry the rounding of the largest entry: 600 eps of an entry at aspect 1e4 instead of 3)
+        const double x0 = __ldg(X + 2 * (int64_t)v[2]) - __ldg(X + 2 * (int64_t)v[1]);
+        const double y0 = __ldg(X + 2 * (int64_t)v[2] + 1) - __ldg(X + 2 * (int64_t)v[1] + 1);
         K[0][1] = -w * fma(x0, V[1][0], y0 * V[1][1]);
         K[0][2] = w * fma(x0, V[0][0], y0 * V[0][1]);
         K[1][2] = -w * fma(V[1][0], V[0][0], V[1][1] * V[0][1]);
-        K[0][0] = -(K[0][1] + K[0][2]);
-        K[1][1] = -(K[0][1] + K[1][2]);
-        K[2][2] = -(K[0][2] + K[1][2]);
+        K[0][0] = w * fma(x0, x0, y0 * y0);
+        K[1][1] = w * fma(V[1][0], V[1][0], V[1][1] * V[1][1]);
+        K[2][2] = w * fma(V[0][0], V[0][0], V[0][1] * V[0][1]);
     } else {
         // N1 = V1 x V2 (c), N2 = V2 x V0, N3 = V0 x V1
         const double p0 = det2(V[2][1], V[2][2], V[0][1], V[0][2]), p1 = det2(V[2][2], V[2][0], V[0][2], V[0][0]),
@@ -359,10 +360,13 @@ __global__ void __launch_bounds__(256) p1_elem_kernel(const double *__restrict__
         K[1][2] = w * fma(c[2], p2, fma(c[1], p1, c[0] * p0));
         K[1][3] = w * fma(c[2], q2, fma(c[1], q1, c[0] * q0));
         K[2][3] = w * fma(p2, q2, fma(p1, q1, p0 * q0));
-        K[0][1] = -(K[1][1] + K[1][2] + K[1][3]);
-        K[0][2] = -(K[1][2] + K[2][2] + K[2][3]);
-        K[0][3] = -(K[1][3] + K[2][3] + K[3][3]);
-        K[0][0] = -(K[0][1] + K[0][2] + K[0][3]);
+        // N0 from the zero sum of the N_i; its products by themselves: as row sums they would carry the
+        // rounding of the largest entry (needles and flat elements: 3e4 eps of an entry instead of 70)
+        const double n0 = -(c[0] + p0 + q0), n1 = -(c[1] + p1 + q1), n2 = -(c[2] + p2 + q2);
+        K[0][0] = w * fma(n2, n2, fma(n1, n1, n0 * n0));
+        K[0][1] = w * fma(n2, c[2], fma(n1, c[1], n0 * c[0]));
+        K[0][2] = w * fma(n2, p2, fma(n1, p1, n0 * p0));
+        K[0][3] = w * fma(n2, q2, fma(n1, q1, n0 * q0));
     }
 #pragma unroll
     for (int i = 0; i < NV; ++i)
