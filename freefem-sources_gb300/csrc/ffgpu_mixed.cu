@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kMxThreads) ir_ka_ring(SellArgs S, const float
         if (!ok) {
             // give the copies under way the same time again, so that none outlives the block
             for (int i = 0; i < issued; ++i, st = st + 1 == kRingStages ? 0 : st + 1, ph ^= st == 0) ring_wait(bar + 8 * st, ph);
-            if (lane == 0) ks->fail = 1;
+            if (lane == 0) { ks->fail = 1; ks->done = 1; }   // the next K_b ends the loop
         }
     }
     float tot;
@@ -497,6 +497,10 @@ static int ir_tune(ffgpu_matrix *A, IRState &S) {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    int fail = 0;
+    FFGPU_CUDA(cudaMemcpyAsync(&fail, &S.ks->fail, sizeof(int), cudaMemcpyDeviceToHost, s));
+    FFGPU_CUDA(cudaStreamSynchronize(s));
+    FFGPU_CHECK(!fail, FFGPU_ECUDA, "FP32 SpMV tuner: a copy of matrix entries did not arrive");
     A->sell32_kind = kinds[tuned_pick(tms, 4)];
     tuned_store(ctx, A, 2, A->sell32_kind);
     return FFGPU_OK;

@@ -1156,8 +1156,11 @@ static int tune_lanes(ffgpu_matrix *A, int mode) {
                 fprintf(stderr, "ffgpu: SpMV tuner (mode %d, %d block rows, %lld blocks): %s%s %d %.4f ms\n", mode,
                         A->nb, (long long)A->nnzb, cands[c] == bestT ? "* " : "",
                         is_sell(cands[c]) ? sell_name(cands[c], ka_staged(A, mode, cands[c])) : "bsr lanes", cands[c], tms[c]);
+        int done = 0;
+        FFGPU_CUDA(cudaMemcpyAsync(&done, &ks->done, sizeof(int), cudaMemcpyDeviceToHost, s));
         FFGPU_CUDA(cudaMemsetAsync(ks, 0, sizeof(KrylovScalars), s));
         FFGPU_CUDA(cudaStreamSynchronize(s));
+        FFGPU_CHECK(done != kWaitRanOut, FFGPU_ECUDA, "SpMV tuner: a wait in a kernel ran out");
     }
     if (is_sell(bestT)) {
         if (mode == 1) { dfree(ctx, A->valx); A->valx = nullptr; }
@@ -1610,6 +1613,8 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     int bodies = bodies_host >= 0 ? bodies_host
                                   : (fused ? hk.iter / unroll + 1 : (hk.iter == 0 ? 1 : (hk.iter + unroll - 1) / unroll));
     if (use_graph) ctx->launches += (int64_t)bodies * A->cg_kernels_body;
+    // (blocks that saw the end skipped their sums: the ticket starts again)
+    if (hk.done == kWaitRanOut) FFGPU_CUDA(cudaMemsetAsync(A->ks, 0, sizeof(KrylovScalars), s));
     FFGPU_CHECK(hk.done != kWaitRanOut, FFGPU_ECUDA, "CG: a wait in a kernel ran out after %d iterations", hk.iter);
     if (st) {
         st->iterations = hk.iter;
