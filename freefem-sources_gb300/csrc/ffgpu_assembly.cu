@@ -439,6 +439,7 @@ __global__ void __launch_bounds__(128) pattern_kernel(int nnodes, const int32_t 
             if (v == a) { drank[a] = r; self = true; }
         }
         self = __any_sync(0xffffffffu, self);
+        __syncwarp();   // the ranks in tab are read by other lanes (a vote orders no memory)
         for (int p = lane; p < m; p += 32) rmap[(int64_t)b * NN + p] = (uint16_t)tab[sl[p]];
         if (lane == 0) {
             deg[a] = u;
