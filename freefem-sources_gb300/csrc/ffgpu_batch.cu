@@ -287,7 +287,8 @@ __global__ void __launch_bounds__(NT) batch_ir_kernel(BatchArgs B) {
 // gradient g and the correction d -- and q = A h in registers, so that an inner iteration moves only
 // the packed matrix, coalesced, from L2 (6 bytes per entry).  The inner system is scaled to a
 // unit diagonal, S A S with S = C^(1/2): conjugate gradients on it are the Jacobi-preconditioned
-// ones (g here is S g, d is S^-1 d) without 1/A_ii.  The values are rounded to FP32 once, as the unscaled.
+// ones (g here is S g, d is S^-1 d) without 1/A_ii.  The values, the gradient and the correction are rounded
+// to FP32 once, as the unscaled: the scale is applied in FP64.
 // The kernel above gathers three values per entry through L1 and reads CSR rows, two lanes each.
 // Per inner iteration of the largest problems (N = 128, 16 641 rows): 37 us there, 12.7 us here,
 // and a batch ends when its largest problem does.
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_sm_kernel(BatchArgs B) {
                 if (i < n) {
                     const double ri = B.b[r0 + i] - B.r[r0 + i];
                     s64 = fma(ri, B.dinv[r0 + i] * ri, s64);
-                    gi = -(float)ri * scale[i];
+                    gi = -(float)(ri * (double)scale[i]);
                     sa = fmaf(gi, gi, sa);
                 }
                 g[i] = gi;
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batch_sm_kernel(BatchArgs B) {
                 ++inner;
                 if (!(ig == ig)) break;
             }
-            for (int i = threadIdx.x; i < n; i += NT) B.x[r0 + i] += (double)(d[i] * scale[i]);
+            for (int i = threadIdx.x; i < n; i += NT) B.x[r0 + i] += (double)d[i] * (double)scale[i];
             __syncthreads();
         }
         if (threadIdx.x == 0) {
