@@ -1377,6 +1377,7 @@ int ffgpu_matrix_destroy(ffgpu_matrix *M) {
     direct_release(M);
     dfree(M->ctx, M->browptr); dfree(M->ctx, M->bcol); dfree(M->ctx, M->diagpos); dfree(M->ctx, M->rowperm); dfree(M->ctx, M->val);
     dfree(M->ctx, M->geo); dfree(M->ctx, M->bcmask); dfree(M->ctx, M->rmap);
+    dfree(M->ctx, M->band_perm);
     dfree(M->ctx, M->diag_inv); dfree(M->ctx, M->wcl); dfree(M->ctx, M->vec); dfree(M->ctx, M->val_t);
     dfree(M->ctx, M->val32); dfree(M->ctx, M->valx); dfree(M->ctx, M->valx_t); dfree(M->ctx, M->hx); dfree(M->ctx, M->ks);
     sell_release(M);

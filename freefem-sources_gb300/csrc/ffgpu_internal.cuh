@@ -145,7 +145,7 @@ struct ffgpu_matrix {
     int csr_lanes;        // lanes per block row of the FP64 SpMV (tuned)
     int csr_lanes_x;      // lanes per block row of the double-float SpMV (tuned)
     int layout_pinned;    // the caller fixed the SpMV layout of the current solve
-    int last_cluster;     // the last FP64 CG solve ran in one thread-block cluster
+    int cg_path;          // how the last CG solve ran (CgPath)
     void *direct;         // factorisation state of the direct solver (ffgpu_direct.cu), or NULL
     int direct_method;    // FFGPU_DIRECT_AUTO / _CHOLESKY / _QR
     // SELL-32 copy for the Krylov SpMVs: block rows sliced into chunks of 32 lanes (one row per
@@ -165,9 +165,10 @@ struct ffgpu_matrix {
     // per-grid partitions of the chunks over warps, balanced by slot count (nw+1 starts)
     int spart_nw[4];
     int32_t *spart[4];
-    // in-kernel CG loop (ffgpu_persist.cu): widest column range and most row-group slots of a
-    // block (0: not measured yet, -1: could not be)
-    int band_range, band_slots;
+    // in-kernel CG loop (ffgpu_persist.cu): its form, the widest column range and the most row-group slots
+    // of a block, and the blocks' rows by length (NULL: as numbered)
+    int band_kind, band_range, band_slots;
+    uint16_t *band_perm;
     int sell32_kind;      // chunk assignment of the FP32 SELL SpMV (tuned): 64 ranges, 65 stride
 };
 
@@ -349,8 +350,13 @@ bool cluster_cg_fits(ffgpu_matrix *A, int trans);
 // the CG loop of a scalar system with a narrow column range in one cooperative kernel
 // (ffgpu_persist.cu), under the same contract
 constexpr int kLoopRefused = 1;      // the launch was refused, nothing ran
+// how a CG solve runs: three or two launches per iteration, one cluster, or one cooperative kernel (cg_band
+// staged or wide, cg_loop)
+enum CgPath { kPathNone = 0, kPathThree = 1, kPathTwo = 2, kPathCluster = 3, kPathBand = 4, kPathWide = 5, kPathLoop = 6 };
+enum BandKind { kBandUnknown = 0, kBandStaged = 1, kBandWide = 2, kBandNone = 3 };
 bool band_cg_fits(ffgpu_matrix *A);
-int band_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, double *h2, double *cg, cudaStream_t s);
+int band_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, double *h2, double *cg, double *pair,
+                cudaStream_t s);
 // the same for larger scalar systems, which stream from L2 or HBM
 bool loop_cg_fits(const ffgpu_matrix *A);
 int loop_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, double *q, double *z, cudaStream_t s);

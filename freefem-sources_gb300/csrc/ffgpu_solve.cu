@@ -1363,7 +1363,9 @@ static bool in_kernel_loops() {
 static bool cg_fused_fits(const ffgpu_matrix *A, int mode) {
     const char *e = getenv("FFGPU_CG_FUSE");
     if (e && e[0] == '0') return false;
-    return mode == 0 && A->bs == 1 && A->nnz <= kFuseMaxEntries;
+    if (mode != 0 || A->bs != 1 || A->nnz > kFuseMaxEntries) return false;
+    // many lanes per row (a few long rows) can give a grid whose partials the reduction buffer does not hold
+    return is_sell(A->csr_lanes) || 2 * spmv_grid(A, pick_lanes(A)) + vec_grid_kb(A->n) <= 4 * kRedBlocks;
 }
 
 static int kca_setup(ffgpu_matrix *A, int trans, const double *hold, double *hnew, const double *cgv,
@@ -1511,16 +1513,20 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     // small scalar systems: the whole iteration loop in one thread-block cluster
     // (ffgpu_cluster.cu), unless a layout is fixed by the caller
     const bool cluster = mode == 0 && !A->layout_pinned && cluster_cg_fits(A, trans);
-    A->last_cluster = cluster;
     bool fused = !cluster && cg_fused_fits(A, mode);
     if (fused) unroll += unroll & 1;   // the H buffers alternate: an even number of iterations per body
     // the whole loop in one cooperative kernel where a block's rows and columns fit its SM
     const bool may_loop = mode == 0 && !cluster && !A->layout_pinned && in_kernel_loops();
     const bool band = may_loop && band_cg_fits(A);
-    bool loop = band || (may_loop && loop_cg_fits(A));
+    const bool sell = is_sell(A->csr_lanes);
     // the initial residual is summed in the order of the matrix's layout, whatever ran before: the
     // copy that cg_graph makes for the launches
-    if (loop && is_sell(A->csr_lanes)) FFGPU_TRY(sell_values(A, trans ? kSell64T : kSell64));
+    if (may_loop && sell) FFGPU_TRY(sell_values(A, trans ? kSell64T : kSell64));
+    bool loop = band || (may_loop && sell && loop_cg_fits(A));
+    A->cg_path = cluster ? kPathCluster
+                 : band  ? (A->band_kind == kBandWide ? kPathWide : kPathBand)
+                 : loop  ? kPathLoop
+                         : (fused ? kPathTwo : kPathThree);
     if (!cluster && !loop) FFGPU_TRY(cg_graph(A, trans, unroll, mode, x, g, h, q, fused, h2, cgv));
     FFGPU_CUDA(cudaMemcpyAsync(x, xu, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     cudaEvent_t e0, e1;
@@ -1547,12 +1553,13 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     int bodies_host = -1;
     bool use_graph = !cluster && !loop;
     if (loop) {
-        const int rc = band ? band_cg_run(A, trans, x, g, h, h2, cgv, s) : loop_cg_run(A, trans, x, g, h, q, cgv, s);
+        const int rc = band ? band_cg_run(A, trans, x, g, h, h2, cgv, A->vec + 5 * vs, s) : loop_cg_run(A, trans, x, g, h, q, cgv, s);
         if (rc == kLoopRefused) {
             // the launches per iteration from the same state
             FFGPU_TRY(cg_graph(A, trans, unroll, mode, x, g, h, q, false, h2, cgv));
             loop = fused = false;
             use_graph = true;
+            A->cg_path = kPathThree;
         } else {
             FFGPU_TRY(rc);
             bodies_host = 0;
@@ -1562,7 +1569,7 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
         const int rc = cluster_cg_run(A, trans, x, g, h, s);
         if (rc == kClusterRefused) {
             // the device refused this cluster shape: the regular path from the same state
-            A->last_cluster = 0;
+            A->cg_path = kPathThree;
             FFGPU_TRY(cg_graph(A, trans, unroll, mode, x, g, h, q, false, h2, cgv));
             use_graph = true;
         } else {
@@ -1687,7 +1694,8 @@ int ffgpu_solve_gmres(ffgpu_matrix *A, const double *b, double *x, int nrhs, int
 int ffgpu_matrix_spmv_layout(const ffgpu_matrix *A, int mode) {
     if (!A) return 0;
     if (mode == 3) return A->scol16 != nullptr;
-    if (mode == 5) return A->last_cluster;
+    if (mode == 5) return A->cg_path == kPathCluster;
+    if (mode == 6) return A->cg_path;
     if (mode == 4) return A->nslot > 0 && A->nslot * 32 <= INT32_MAX ? (int)(A->nslot * 32) : (A->nslot ? -1 : 0);
     return mode == 2 ? A->sell32_kind : (mode == 1 ? A->csr_lanes_x : A->csr_lanes);
 }

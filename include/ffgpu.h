@@ -329,6 +329,9 @@ int ffgpu_matrix_info(const ffgpu_matrix *A, int *n, int64_t *nnz, int *block_si
  * mode 5: 1 when the last FP64 CG solve ran its whole iteration loop in one thread-block
  * cluster (opt-in with FFGPU_CLUSTER_CG=1: scalar systems of up to 8 x 9216 rows; a fixed
  * layout selects the regular path).
+ * mode 6: how the last CG solve ran: 1 three launches per iteration, 2 two, 3 one cluster, or one
+ * cooperative kernel for the whole loop: 4 matrix and direction in shared memory, 5 matrix in shared
+ * memory and the direction gathered, 6 matrix streamed; 0 before the first.
  * No FreeFEM counterpart. */
 int ffgpu_matrix_spmv_layout(const ffgpu_matrix *A, int mode);
 /* Average device time in ms of `nrep` back-to-back launches of the solver's SpMV kernel (K_a,
