@@ -31,8 +31,10 @@
 //
 // No kernel ends with one block that works alone: gm_dots ends with one per vector group, the norm
 // is summed where it is read, and the rotation (a chain of square roots and divisions) runs beside
-// the next step's dot products, at the price of that step's first three kernels once per cycle,
-// when it says stop (9282 rows, 381 steps: 16.7 ms with last blocks in gm_dots and gm_update,
+// the next step's dot products, at the price of that step's first three kernels once per solve,
+// when it says stop.  The last step of a full cycle is finished by the back substitution's block, so that a
+// short restart pays for no step of its own (90 x 90 cells, 400 steps, dim_krylov 1: 29.5 -> 25.8 ms, with last
+// blocks 26.2; dim_krylov 3: 16.4 -> 15.0, 18.8).  (9282 rows, 381 steps: 16.7 ms with last blocks in gm_dots and gm_update,
 // 14.3 ms now; the FP64 products alone are 3.1 ms, the rest is latency inside the five kernels).
 // Sums of gm_dots' slabs by every block of gm_coef instead: 16.2 ms.
 // A rotation after the other (FreeFEM's loop) is a chain of 2 it dependent FP64 operations, 76
@@ -173,8 +175,8 @@ __global__ void __launch_bounds__(kGmThreads) gm_resid(GmArgs a) {
     }
 }
 
-// ||v_it||^2 before its scaling, in every thread of the block: the sum of gm_update's parts (at
-// most 4 * kNumSM of them)
+// ||v_it||^2 before its scaling, in every thread of the block (kGmThreads or more): the sum of gm_update's
+// parts (at most 4 * kNumSM of them)
 __device__ __forceinline__ double gm_norm2(const GmArgs &a) {
     __shared__ double sh[kGmWarps];
     static_assert(4 * kNumSM <= 3 * kGmThreads && kGmWarps == 8, "parts per thread");
@@ -182,10 +184,10 @@ __device__ __forceinline__ double gm_norm2(const GmArgs &a) {
 #pragma unroll
     for (int u = 0; u < 3; ++u) {
         const int b = threadIdx.x + u * kGmThreads;
-        v[u] = b < a.nupd ? __ldcg(a.nrm + b) : 0.0;
+        v[u] = b < a.nupd && threadIdx.x < kGmThreads ? __ldcg(a.nrm + b) : 0.0;
     }
     double t = warp_sum((v[0] + v[1]) + v[2]);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+    if ((threadIdx.x & 31) == 0 && threadIdx.x < kGmThreads) sh[threadIdx.x >> 5] = t;
     __syncthreads();
     t = sh[threadIdx.x & 7];
 #pragma unroll
@@ -196,7 +198,6 @@ __device__ __forceinline__ double gm_norm2(const GmArgs &a) {
 // v_it *= 1/||.|| (FreeFEM: Vi[it] = (1./aux)*wi), vp = C v_it into Vp[it] and the SpMV input
 __global__ void __launch_bounds__(kGmThreads) gm_prep(GmArgs a) {
     const int it = a.sc->next;
-    if (it >= a.m) return;   // the cycle is full: gm_dots finishes its last step
     double *v = a.V + it * a.vs, *vp = a.Vp + it * a.vs;
     const double inv = it == 0 ? 1. / a.g[0] : 1. / sqrt(gm_norm2(a));
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n; k += (int64_t)gridDim.x * blockDim.x) {
@@ -208,45 +209,49 @@ __global__ void __launch_bounds__(kGmThreads) gm_prep(GmArgs a) {
     }
 }
 
-// the end of step it: the new rotation, the triangle's column, Q, the stopping tests (one block)
-__device__ void gm_finish(const GmArgs &a, int it) {
+// the end of step it: the new rotation, the triangle's column, Q, the stopping tests (one block; in_loop: of
+// a kernel inside the while node)
+__device__ void gm_finish(const GmArgs &a, int it, bool in_loop) {
     __shared__ double rot[2];
     const int ld = a.m + 1;
     GmScal *c = a.sc;
+    // what the chain below reads is under way during the norm's sum
+    const double hd = a.u[it], g0 = a.g[it], normb = c->normb, eps = c->eps;
+    const int itmax = c->itmax, iter = c->iter, steps = c->steps;
     const double aux = sqrt(gm_norm2(a));
     if (threadIdx.x == 0) {
-        const double hd = a.u[it], hs1 = aux;
+        const double hs1 = aux;
         const double sq = sqrt(hd * hd + hs1 * hs1);
         const double c0 = hd / sq, s0 = hs1 / sq;
         rot[0] = c0;
         rot[1] = s0;
         a.R[(int64_t)it * ld + it] = c0 * hd + s0 * hs1;
-        const double g0 = a.g[it];
         a.g[it + 1] = -s0 * g0;
         a.g[it] = c0 * g0;
         const double relres = fabs(-s0 * g0);
         c->relres = relres;
-        c->steps += 1;
+        c->steps = steps + 1;
         c->itf = it;
         bool stop = false;
-        if (relres / c->normb < fabs(c->eps)) {
+        if (relres / normb < fabs(eps)) {
             c->conv = 1;
             stop = true;
-        } else if (it > c->itmax) {
+        } else if (it > itmax) {
             stop = true;                       // FreeFEM: `if (it > nbitermx) break;`
         } else {
             c->it = it + 1;                    // the loop increment it++, iter++
-            c->iter += 1;
+            c->iter = iter + 1;
             if (it + 1 >= a.m) { stop = true; c->itf = a.m - 1; }
         }
         c->stop = stop;
-        if (stop && a.in_graph) gm_set_cond(a.cond, 0);
+        if (stop && a.in_graph && in_loop) gm_set_cond(a.cond, 0);
     }
     __syncthreads();
     // the column of the triangle, and Q with the new rotation of its rows it and it + 1
     double *q0 = a.Q + (int64_t)it * (ld + 1), *q1 = q0 + ld + 1;
     for (int i = threadIdx.x; i <= it + 1; i += blockDim.x) {
         if (i < it) a.R[(int64_t)it * ld + i] = a.u[i];
+        if (!in_loop) continue;   // no step comes after
         const double q = i <= it ? q0[i] : 0.0;
         q0[i] = i <= it ? rot[0] * q : rot[1];
         q1[i] = i <= it ? -rot[1] * q : rot[0];
@@ -266,10 +271,9 @@ __global__ void __launch_bounds__(kGmThreads) gm_dots(GmArgs a) {
     double *wsh = smd, *vsh = smd + kGmSub, *acc = smd + 2 * kGmSub;
     const int it = a.sc->next;
     if (blockIdx.x == 0) {
-        if (it > 0) gm_finish(a, it - 1);
+        if (it > 0) gm_finish(a, it - 1, true);
         return;
     }
-    if (it >= a.m) return;
     const int ni = it + 1, K = 2 * ni;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int blk = blockIdx.x - 1;
@@ -411,6 +415,8 @@ __global__ void __launch_bounds__(kGmThreads) gm_update(GmArgs a) {
     if (a.sc->stop) return;
     const int it = a.sc->it;
     const int ni = it + 1, ld = a.m + 1;
+    // the cycle is full: no step comes after this one (gm_back finishes it)
+    if (ni == a.m && a.in_graph && blockIdx.x == 0 && threadIdx.x == 0) gm_set_cond(a.cond, 0);
     const double *hh = a.h;
     if (ni <= kGmHs) {
         for (int i = threadIdx.x; i < ni; i += blockDim.x) hs[i] = a.h[i];
@@ -454,6 +460,10 @@ __global__ void __launch_bounds__(kGmThreads) gm_update(GmArgs a) {
 // 750 us for 381 rows; the whole solve: 31.2 -> 16.7 ms)
 __global__ void __launch_bounds__(kGmBack) gm_back(GmArgs a) {
     extern __shared__ __align__(16) double smb[];
+    if (!a.sc->stop) {           // a full cycle
+        gm_finish(a, a.m - 1, false);
+        __syncthreads();
+    }
     const int it = a.sc->itf;
     if (it < 0) return;
     const int ld = a.m + 1, t = threadIdx.x;
@@ -682,7 +692,7 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
                 if ((rc = launch_check(ctx, "gmres resid"))) break;
                 FFGPU_CUDA(cudaMemcpyAsync(&hs, a.sc, sizeof(hs), cudaMemcpyDeviceToHost, s));
                 FFGPU_CUDA(cudaStreamSynchronize(s));
-                if (hs.stop) break;
+                if (hs.stop || hs.next >= m) break;
                 gm_prep<<<Gv, kGmThreads, 0, s>>>(a);
                 if ((rc = spmv(A, a.vpc, a.w, trans, s))) break;
                 gm_dots<<<Gd, kGmThreads, dsmem, s>>>(a);   // may say stop: the two kernels below then return
@@ -705,7 +715,9 @@ int gmres_one(ffgpu_matrix *A, const double *b, double *x, int trans, const ffgp
             break;
         }
         ++cycles;
-        if (!host_loop) ctx->launches += 4 + 5 * (hs.steps - steps_seen + 1);   // the step that stops the cycle too
+        // a stop inside the cycle is found in the step after it
+        const int64_t steps = hs.steps - steps_seen;
+        if (!host_loop) ctx->launches += 4 + 5 * (steps >= m || hs.itf < 0 ? steps : steps + 1);
         steps_seen = hs.steps;
         if (hs.conv) break;
         if (hs.iter > itmax) break;
