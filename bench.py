@@ -444,7 +444,12 @@ def run_gpu(args, cfgname, steps, warmup, rank, world, variants=(), cpu=True):
         traffic = tr.get(cfgname, {}).get("spmv_bytes_per_launch")
     except Exception:
         pass
-    cluster = bool(ffgpu.lib().ffgpu_matrix_spmv_layout(A.h, 5))
+    # the CG loops that are one kernel for the whole solve (ffgpu_matrix_spmv_layout mode 6)
+    path = int(ffgpu.lib().ffgpu_matrix_spmv_layout(A.h, 6))
+    loop = {3: ("cg_cluster", "one cluster of thread blocks"),
+            4: ("cg_band", "one cooperative kernel, matrix and direction in shared memory"),
+            5: ("cg_band", "one cooperative kernel, matrix in shared memory, direction gathered"),
+            6: ("cg_loop", "one cooperative kernel, matrix streamed")}.get(path)
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "traffic": traffic,
             "kernel": f"FP64 SpMV of the CG (K_a), layout {layout}, block size {bs}",
@@ -452,17 +457,17 @@ def run_gpu(args, cfgname, steps, warmup, rank, world, variants=(), cpu=True):
             "stored_bytes_per_launch": stored,
             "frac_of_stored_bytes": stored / (spmv_avg * 1e-3) / 1e9 / peak,
             "peak_source": peak_src}
-    if cluster:
-        # the whole CG loop is one kernel (one thread-block cluster): its time per iteration
-        # against the algorithmic bytes of one fused PCG iteration, B_spmv + 56 n; the matrix
-        # (below L2) streams from L2, so HBM is not what bounds it
+    if loop:
+        # the whole CG loop is one kernel: its time per iteration against the algorithmic bytes of one
+        # fused PCG iteration, B_spmv + 56 n; the matrix stays on chip or in L2 on the small systems, so HBM
+        # is not what bounds it
         its_c = max(1, iters[-1])
         it_ms = statistics.median(phase["solve"][-steps:]) / its_c
         b_it = spmv_bytes + 56 * n
         ach = b_it / (it_ms * 1e-3) / 1e9
-        roof = {"bound": "latency / L2 (whole CG loop in one cluster of thread blocks)", "achieved": ach,
+        roof = {"bound": f"latency / L2 (whole CG loop in {loop[1]})", "achieved": ach,
                 "peak": peak, "unit": "GB/s", "frac": ach / peak, "traffic": None,
-                "kernel": "cg_cluster (one launch per solve, %d iterations)" % its_c,
+                "kernel": "%s (one launch per solve, %d iterations)" % (loop[0], its_c),
                 "bytes_per_iteration": b_it, "ms_per_iteration": it_ms, "peak_source": peak_src,
                 "regular_path_spmv": {"kernel": f"K_a, layout {layout}", "ms_per_launch": spmv_avg,
                                       "frac": achieved / peak}}
@@ -625,8 +630,9 @@ def run_gpu(args, cfgname, steps, warmup, rank, world, variants=(), cpu=True):
                    "solve_ms": solve_fp64,
                    "ms_per_cg_iteration": solve_fp64 / max(1, iters[-1]),
                    "spmv_layout": layout,
-                   "cg_path": ("one thread-block cluster (whole iteration loop in one kernel)"
-                               if cluster else "CUDA graph of K_a, K_b, K_c per iteration"),
+                   "cg_path": (f"{loop[0]}: whole iteration loop in {loop[1]}" if loop else
+                               "CUDA graph of two kernels per iteration" if path == 2 else
+                               "CUDA graph of K_a, K_b, K_c per iteration"),
                    "rel_residual": rel_res,
                    "element_matrices": elem},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
