@@ -316,9 +316,9 @@ __device__ __forceinline__ void store4(double *p, double a, double b, double c, 
 //   grad phi_i = N_i / det with N_i the inward normals (cross products of edges), so
 //   K_ij = (kappa c_stiff / (DIM! det)) N_i.N_j, one dot product per pair.
 // Row la of element e at out[(e * (DIM + 1) + la) * 4], four doubles wide (32-byte stores; the
-// row fill reads one sector).  FP64 issue bounds it (one warp instruction per 64 cycles and
+// row fill reads one sector).  FP64 issue bounds it (one warp instruction per 76 cycles and
 // sub-partition): about 90 FP64 operations per tetrahedron against about 60 for the gradients
-// alone, and none of the products is left to the row fill.
+// alone, and none of the products is left to the row fill (5.3 M tetrahedra: 0.84 ms).
 template <int DIM>
 __global__ void __launch_bounds__(256) p1_elem_kernel(const double *__restrict__ X, const int32_t *__restrict__ elems, int nt,
                                                       const double *__restrict__ kappa, double c_stiff, double c_mass,
@@ -505,7 +505,7 @@ static int neg_tgv_bits(double tgv) {
 // The form this replaces gave the row one copy per concurrent element and summed the copies:
 // 21 warp adds per P1 row in 3D instead of 3.  PLAIN: the element matrices are complete (kloc or
 // eloc and nothing to add); the general form keeps its tests out of that loop.  On 96^3 cells (912 673 rows, 13.4 M entries), the
-// products moved to p1_elem_kernel (0.76 ms): 3.27 -> 0.30 ms.  (With the tests on tgv and c_mass
+// products moved to p1_elem_kernel (0.84 ms): 3.27 -> 0.30 ms.  (With the tests on tgv and c_mass
 // as FP64 compares in the loops it took 1.6 ms: a compare costs as much as an add.)
 template <int DIM, int FE, bool PLAIN>
 __global__ void __launch_bounds__(256) fill_kernel(FillArgs A) {

@@ -315,8 +315,10 @@ inline int sell_unit(int nchunk) { return nchunk >= 4 * 8 * kNumSM ? 8 : 1; }
 inline int sell_spread_grid(int nchunk) { return nchunk < kNumSM ? (nchunk > 0 ? nchunk : 1) : kNumSM; }
 // Lanes per block row: four for 3x3 blocks below kSellWideRows block rows.  A chunk is then 8 rows, a
 // quarter as long, which 608 FP64 pipes can share evenly, against 5 % of padding (rows end at
-// multiples of four) and three adds a row.  K_a, best of the candidates: 117 649 block rows 82 us with one lane (and with block
-// CSR), 74 us with four; 388 725 rows 196 and 198 us (double-float 145 and 159 us).
+// multiples of four) and three adds a row.  K_a with one lane and with four, best of the candidates, us: FP64 94.4 and 86.2 at
+// 148 877 block rows, 131.1 and 119.3 at 226 981, 154.4 and 150.5 at 291 785, 187.3 and 193.0 at 357 911, 282 and 301
+// at 614 125; double-float 77.0 and 67.3, 98.9 and 96.6, 115.9 and 116.5, 140.3 and 143.3, 211 and 236; FP32 47.1 and 42.6,
+// 65.9 and 60.6, 72.9 and 76.9, 86.9 and 84.2, 136 and 138.
 constexpr int kSellWideRows = 300000;
 inline int sell_lanes(const ffgpu_matrix *A) { return A->bs == 3 && A->nb < kSellWideRows ? 4 : 1; }
 int sell_prepare(ffgpu_matrix *A);               // structure (once per pattern)

@@ -13,8 +13,8 @@
 // Every lane of a warp runs the same trip count, every load is a full 128/256-byte line, and
 // no lane-group reductions are needed with one lane per row.  How the chunks go to the warps:
 // ffgpu_sell.cuh.
-// Within a row the entries keep their column order, so the row sums are formed in the same
-// order as the block-CSR kernels form them.
+// Within a row the entries keep their column order, so with one lane per row the sums are formed in the
+// order of block CSR with one lane; four lanes sum every fourth entry each.
 // For bs == 1 the column is stored as the 16-bit difference column - row whenever the
 // matrix bandwidth allows (2 instead of 4 bytes per entry).
 #include <string.h>

@@ -12,8 +12,9 @@
 // CG = C G is recomputed where it is used instead of being stored.  Small scalar systems (the
 // matrix in L2, an iteration bound by kernel boundaries) run two kernels per iteration: K_b
 // stores C G and the next K_a forms H = gamma H - C G at every column it gathers (cg_kca_sell).
-// By default scalar systems whose vectors fit the SMs run the whole loop in one cooperative kernel
-// instead (ffgpu_persist.cu), which needs no kernel boundaries at all.
+// By default scalar systems whose matrix fits the SMs, and larger ones with a local numbering whose vectors
+// do, run the whole loop in one cooperative kernel instead (ffgpu_persist.cu), which needs no kernel
+// boundaries at all.
 // The iteration loop is a CUDA graph `while` node whose condition K_b clears on convergence or
 // at itmax, so a whole solve is one graph launch with no host round trip.
 #include <math.h>
@@ -1088,8 +1089,8 @@ constexpr int64_t kTuneMinEntries = 1 << 16;
 // 3x3 blocks, FP64: below this many block rows only block CSR is timed.  A SELL warp reads its chunk
 // range, then the chunk's rows, length and offset, then columns, before its first gather; between
 // the other kernels of an iteration that chain costs more than the tuner's repeated launches show.
-// Whole solves, block CSR and four-lane SELL (which the tuner prefers by 6 to 9 %): [P2]^3 on
-// 13 x 12 x 13 cells, 18 225 rows, 24.3 and 26.4 ms; 16^3, 35 937 rows, 42.3 and 41.7 ms.
+// Whole solves of [P2]^3, best block CSR and best four-lane SELL (which the tuner prefers by 6 to 9 %): 18 225 rows
+// 21.5 and 22.4 ms, 24 389 rows 27.3 and 28.0, 29 791 rows 33.3 and 32.0, 35 937 rows 35.9 and 35.9.
 constexpr int kSellBlockRows = 24000;
 
 static bool layout_valid(int mode, int code) {
@@ -1353,8 +1354,8 @@ struct KcaCall {
     }
 };
 
-// The loops that stay inside one kernel (ffgpu_persist.cu) are the default; FFGPU_CG_FUSE=0 or
-// FFGPU_CLUSTER_CG=0 selects launches per iteration.
+// The loops that stay inside one kernel (ffgpu_persist.cu) are the default.  FFGPU_CLUSTER_CG=0 (no loop in one
+// kernel, cluster or cooperative) selects launches per iteration, FFGPU_CG_FUSE=0 three of them.
 static bool in_kernel_loops() {
     const char *f = getenv("FFGPU_CG_FUSE"), *c = getenv("FFGPU_CLUSTER_CG");
     return !(f && f[0] == '0') && !(c && c[0] == '0');
