@@ -146,6 +146,7 @@ struct ffgpu_matrix {
     int csr_lanes_x;      // lanes per block row of the double-float SpMV (tuned)
     int layout_pinned;    // the caller fixed the SpMV layout of the current solve
     int cg_path;          // how the last CG solve ran (CgPath)
+    int sell_due;         // bit trans: the SELL copy of A or A' is made at the next product outside the CG (spmv)
     void *direct;         // factorisation state of the direct solver (ffgpu_direct.cu), or NULL
     int direct_method;    // FFGPU_DIRECT_AUTO / _CHOLESKY / _QR
     // SELL-32 copy for the Krylov SpMVs: block rows sliced into chunks of 32 lanes (one row per

@@ -267,6 +267,7 @@ void sell_release_values(ffgpu_matrix *A) {
     A->sval = A->sval_t = nullptr;
     A->svalx = A->svalx_t = nullptr;
     A->sval32 = nullptr;
+    A->sell_due = 0;
 }
 
 }  // namespace ffgpu

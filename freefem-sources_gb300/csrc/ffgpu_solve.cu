@@ -1201,9 +1201,21 @@ static int pin_layout(ffgpu_matrix *A, int mode, int code) {
     return FFGPU_OK;
 }
 
+// y = A x from block CSR
+static int spmv_csr(ffgpu_matrix *A, const double *x, double *y, int trans, cudaStream_t st) {
+    if (trans) FFGPU_TRY(matrix_prepare_transpose(A));
+    int T = pick_lanes(A);
+    SpmvArgs s = spmv_args(A, trans);
+    void *fn = A->bs == 3 ? spmv_fn<3>(T) : spmv_fn<1>(T);
+    void *args[] = {&s, &x, &y};
+    FFGPU_CUDA(cudaLaunchKernel(fn, spmv_grid(A, T), kSpmvWarps * 32, args, 0, st));
+    return launch_check(A->ctx, "spmv");
+}
+
 // y = A x in the matrix's own layout.  (A SELL copy that another kernel built beside a block-CSR layout is
 // not read: the summation order would depend on what ran before.)
 int spmv(ffgpu_matrix *A, const double *x, double *y, int trans, cudaStream_t st) {
+    if ((A->sell_due >> (trans != 0) & 1) && is_sell(A->csr_lanes)) FFGPU_TRY(sell_values(A, trans ? kSell64T : kSell64));
     const double *sv = trans ? A->sval_t : A->sval;
     if (sv && is_sell(A->csr_lanes)) {
         SellArgs sl = sell_args(A);
@@ -1216,13 +1228,7 @@ int spmv(ffgpu_matrix *A, const double *x, double *y, int trans, cudaStream_t st
         FFGPU_CUDA(cudaLaunchKernel(fn, grid, threads, args, 0, st));
         return launch_check(A->ctx, "spmv");
     }
-    if (trans) FFGPU_TRY(matrix_prepare_transpose(A));
-    int T = pick_lanes(A);
-    SpmvArgs s = spmv_args(A, trans);
-    void *fn = A->bs == 3 ? spmv_fn<3>(T) : spmv_fn<1>(T);
-    void *args[] = {&s, &x, &y};
-    FFGPU_CUDA(cudaLaunchKernel(fn, spmv_grid(A, T), kSpmvWarps * 32, args, 0, st));
-    return launch_check(A->ctx, "spmv");
+    return spmv_csr(A, x, y, trans, st);
 }
 
 int matrix_prepare_split(ffgpu_matrix *A, int trans) {
@@ -1520,9 +1526,11 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     const bool may_loop = mode == 0 && !cluster && !A->layout_pinned && in_kernel_loops();
     const bool band = may_loop && band_cg_fits(A);
     const bool sell = is_sell(A->csr_lanes);
-    // the initial residual is summed in the order of the matrix's layout, whatever ran before: the
-    // copy that cg_graph makes for the launches
-    if (may_loop && sell) FFGPU_TRY(sell_values(A, trans ? kSell64T : kSell64));
+    // The initial residual is summed in one order, whatever ran before: from block CSR where cg_band
+    // runs, which reads no SELL copy (a new matrix's copy is 90 us, of 640 for a small script), else from the
+    // layout's copy.  The other users of spmv() find the copy after any CG solve: cg_band leaves it due.
+    if (band) A->sell_due |= 1 << (trans != 0);
+    else if (may_loop && sell) FFGPU_TRY(sell_values(A, trans ? kSell64T : kSell64));
     bool loop = band || (may_loop && sell && loop_cg_fits(A));
     A->cg_path = cluster ? kPathCluster
                  : band  ? (A->band_kind == kBandWide ? kPathWide : kPathBand)
@@ -1538,7 +1546,7 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
         cg_x0_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, x, b, A->wcl, tgv);
         FFGPU_TRY(launch_check(ctx, "cg_x0"));
     }
-    FFGPU_TRY(spmv(A, x, g, trans, s));
+    FFGPU_TRY(band ? spmv_csr(A, x, g, trans, s) : spmv(A, x, g, trans, s));
     cg_init<<<kVecBlocks, kVecThreads, 0, s>>>(n, g, b, h, A->diag_inv, A->ks, prm->eps, itmax, ctx->d_part);
     FFGPU_TRY(launch_check(ctx, "cg_init"));
     if (mode == 1) {
