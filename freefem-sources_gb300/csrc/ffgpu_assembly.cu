@@ -316,8 +316,8 @@ __device__ __forceinline__ void store4(double *p, double a, double b, double c, 
 //   grad phi_i = N_i / det with N_i the inward normals (cross products of edges), so
 //   K_ij = (kappa c_stiff / (DIM! det)) N_i.N_j, one dot product per pair.
 // Row la of element e at out[(e * (DIM + 1) + la) * 4], four doubles wide (32-byte stores; the
-// row fill reads one sector).  FP64 issue bounds it (one warp instruction per 76 cycles and
-// sub-partition): about 90 FP64 operations per tetrahedron against about 60 for the gradients
+// row fill reads one sector).  FP64 issue bounds it (a warp's fused multiply-add
+// takes 64 cycles of its sub-partition, an add or multiply 76): about 90 FP64 operations per tetrahedron against about 60 for the gradients
 // alone, and none of the products is left to the row fill (5.3 M tetrahedra: 0.84 ms).
 template <int DIM>
 __global__ void __launch_bounds__(256) p1_elem_kernel(const double *__restrict__ X, const int32_t *__restrict__ elems, int nt,
@@ -500,7 +500,7 @@ static int neg_tgv_bits(double tgv) {
 // of one incident element after the other to the row in shared memory; a [P2]^3 group has a lane
 // per (lb, component) and adds three values.  The nodes of one element are distinct, so the lanes
 // of a step never meet on an entry, and every FP64 add is issued by all the rows of the warp at
-// once: FP64 issue (76 cycles per warp instruction and sub-partition, however many lanes are
+// once: FP64 issue (76 cycles per warp add and sub-partition, however many lanes are
 // active) bounds the fill, and a step per incident element is the fewest adds there are.
 // The form this replaces gave the row one copy per concurrent element and summed the copies:
 // 21 warp adds per P1 row in 3D instead of 3.  PLAIN: the element matrices are complete (kloc or

@@ -29,7 +29,7 @@
 // 128 threads take tiles from a counter; thread 0 issues the five MMAs and commits them to an
 // mbarrier; every wait is bounded in time and a timeout is reported through the status word.
 // The epilogue's conversions and scalings bound it (about 30 FP64 instructions per warp and
-// elasticity element, one per 76 cycles and sub-partition), and a warp may read only its own
+// elasticity element, one per 64 to 76 cycles and sub-partition), and a warp may read only its own
 // quarter of the TMEM lanes: with one copy of the pairs two of the four sub-partitions did all of
 // it.  The copies give every warp pairs of its own to finish, for different elements (63 888
 // elasticity elements: 552 -> 508 us).

@@ -35,10 +35,10 @@
 // when it says stop.  The last step of a full cycle is finished by the back substitution's block, so that a
 // short restart pays for no step of its own (90 x 90 cells, 400 steps, dim_krylov 1: 29.5 -> 25.8 ms, with last
 // blocks 26.2; dim_krylov 3: 16.4 -> 15.0, 18.8).  (9282 rows, 381 steps: 16.7 ms with last blocks in gm_dots and gm_update,
-// 14.3 ms now; the FP64 products alone are 3.1 ms, the rest is latency inside the five kernels).
+// 14.3 ms now; the FP64 products alone are 3.4 ms, the rest is latency inside the five kernels).
 // Sums of gm_dots' slabs by every block of gm_coef instead: 16.2 ms.
-// A rotation after the other (FreeFEM's loop) is a chain of 2 it dependent FP64 operations, 76
-// cycles each on GB300: 14 us at it = 190.  The product Q costs it^2 multiplications over all SMs.
+// A rotation after the other (FreeFEM's loop) is a chain of 2 it dependent FP64 operations, 64 to
+// 76 cycles each on GB300: 14 us at it = 190.  The product Q costs it^2 multiplications over all SMs.
 #include <math.h>
 #include <string.h>
 

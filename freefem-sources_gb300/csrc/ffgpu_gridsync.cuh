@@ -14,8 +14,8 @@
 // use, four exchanges on, lies a publishing one of the reader's that the sender has seen.
 // Every wait is bounded: after kGsPolls reads of a slot the sum reports failure to the whole block,
 // which leaves its loop, and so do the others when their own waits run out.
-// FP64 on GB300 issues one warp instruction per 76 cycles and SM sub-partition whatever lanes are
-// active, so the sums are arranged for few instructions: pairs of sums share a warp (lanes
+// FP64 on GB300 issues one warp instruction per 64 cycles (fused multiply-add) or 76 (add, multiply) and SM
+// sub-partition, whatever lanes are active, so the sums are arranged for few instructions: pairs of sums share a warp (lanes
 // 0-15 one, 16-31 the other), and four warps, one per sub-partition, read the slots.
 #pragma once
 #include "ffgpu_internal.cuh"

@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256) band_sort_kernel(int n, int rows, const i
 }
 
 // RPT rows per thread, NT threads.  Row u * NT + t of the block's order belongs to thread t.
-// FP64 instructions set the floor (one per 76 cycles and sub-partition): about 16 per group of
+// FP64 instructions set the floor (one per 64 to 76 cycles and sub-partition): about 16 per group of
 // 32 rows and iteration on a 2D P1 mesh.
 template <int NT, int RPT, bool WIDE>
 __global__ void __launch_bounds__(NT, 1) cg_band(BandArgs A) {
