@@ -361,7 +361,7 @@ bool band_cg_fits(ffgpu_matrix *A);
 int band_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, double *h2, double *cg, double *pair,
                 cudaStream_t s);
 // the same for larger scalar systems, which stream from L2 or HBM
-bool loop_cg_fits(const ffgpu_matrix *A);
+bool loop_cg_fits(ffgpu_matrix *A, bool sell);
 int loop_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, double *q, double *z, cudaStream_t s);
 constexpr int kClusterRefused = 1;   // cluster_cg_run: the launch was refused, nothing ran
 int cluster_cg_run(ffgpu_matrix *A, int trans, double *x, const double *g, const double *h, cudaStream_t s);

@@ -512,14 +512,21 @@ int band_cg_run(ffgpu_matrix *A, int trans, double *x, double *g, double *h, dou
 
 constexpr size_t kLoopSmem = 190 * 1024;   // the rest of the SM's 256 KB is the L1 the gathers go through
 static int loop_piece(int n) { return ((n + kNumSM - 1) / kNumSM + 1) & ~1; }
-// Whether the streaming loop takes a system whose tuned layout is SELL: a rule on sizes, the numbering (16-bit column
-// differences) and the device.  Per iteration, loop and launches: P1 along the grid, 60^3 cells 30.2 and 32.5 us,
-// 118^3 94 and 105, 1300^2 69.6 and 73.3; numbered at random 38.7 and 35.6, 191 and 148, 103 and 90.6: one block
-// per SM has fewer gathers in flight.  P2 on 20^3 and 28^3 cells, where the tuner takes block CSR: 32.2 and 26.5,
-// 42.7 and 40.6; one row of 1000 entries in 80^3, likewise: 237 and 149.
-bool loop_cg_fits(const ffgpu_matrix *A) {
-    return A->ctx->coop && A->ctx->d_sync && A->bs == 1 && A->scol16 &&
-           2 * sizeof(double) * (size_t)loop_piece(A->n) <= kLoopSmem;
+// Whether the streaming loop takes the system (sell: its tuned layout is SELL): a rule on sizes, the numbering (16-bit
+// column differences) and the device.  Per iteration, loop and launches: P1 along the grid, 60^3 cells 30.2 and
+// 32.5 us, 118^3 94 and 105, 1300^2 69.6 and 73.3; numbered at random 38.7 and 35.6, 191 and 148, 103 and 90.6: one
+// block per SM has fewer gathers in flight.
+// Where the tuner took block CSR, rows are long or of unequal length, and the loop's warps have to have chunks of
+// 32 rows alike: it runs where their passes are 0.65 full or more (P2 on 28^3 cells, 0.60: 44.0 and 43.5; 29^3, 0.66:
+// 44.4 and 45.4; 30^3, 0.73: 45.1 and 49.0; 32^3, 0.88: 46.1 and 58.3), the longest row is no more than its warp
+// can walk beside the others (one of 120 entries in 80^3 58.4 and 71.6, of 250 83.3 and 73.3) and little is padding.
+constexpr int kLoopDeg = 128;
+bool loop_cg_fits(ffgpu_matrix *A, bool sell) {
+    if (!A->ctx->coop || !A->ctx->d_sync || A->bs != 1 || 2 * sizeof(double) * (size_t)loop_piece(A->n) > kLoopSmem) return false;
+    if (sell) return A->scol16;
+    const int64_t chunks = (A->n + 31) / 32, warps = 32 * kNumSM, passes = (chunks + warps - 1) / warps;
+    if (A->max_deg > kLoopDeg || 20 * chunks < 13 * warps * passes) return false;
+    return sell_prepare(A) == FFGPU_OK && A->scol16 && 4 * A->nslot * 32 <= 5 * A->nnz;
 }
 
 // The loop from the state cg_init leaves; z: a work vector.

@@ -1212,23 +1212,26 @@ static int spmv_csr(ffgpu_matrix *A, const double *x, double *y, int trans, cuda
     return launch_check(A->ctx, "spmv");
 }
 
+// y = A x from the SELL copy
+static int spmv_sell_copy(ffgpu_matrix *A, const double *x, double *y, int trans, cudaStream_t st) {
+    FFGPU_TRY(sell_values(A, trans ? kSell64T : kSell64));
+    const double *sv = trans ? A->sval_t : A->sval;
+    SellArgs sl = sell_args(A);
+    int code = is_sell(A->csr_lanes) ? A->csr_lanes : kSellCode;
+    if (ka_staged(A, 0, code)) code = kSellCode + 1;   // the same chunks, plain
+    void *fn = spmv_sell_fn(A, code);
+    int grid = 0, threads = 0;
+    FFGPU_TRY(sell_launch_shape(A, fn, sell_assign(code), sl, &grid, &threads));
+    void *args[] = {&sl, &sv, &x, &y};
+    FFGPU_CUDA(cudaLaunchKernel(fn, grid, threads, args, 0, st));
+    return launch_check(A->ctx, "spmv");
+}
+
 // y = A x in the matrix's own layout.  (A SELL copy that another kernel built beside a block-CSR layout is
 // not read: the summation order would depend on what ran before.)
 int spmv(ffgpu_matrix *A, const double *x, double *y, int trans, cudaStream_t st) {
-    if ((A->sell_due >> (trans != 0) & 1) && is_sell(A->csr_lanes)) FFGPU_TRY(sell_values(A, trans ? kSell64T : kSell64));
-    const double *sv = trans ? A->sval_t : A->sval;
-    if (sv && is_sell(A->csr_lanes)) {
-        SellArgs sl = sell_args(A);
-        int code = A->csr_lanes;
-        if (ka_staged(A, 0, code)) code = kSellCode + 1;   // the same chunks, plain
-        void *fn = spmv_sell_fn(A, code);
-        int grid = 0, threads = 0;
-        FFGPU_TRY(sell_launch_shape(A, fn, sell_assign(code), sl, &grid, &threads));
-        void *args[] = {&sl, &sv, &x, &y};
-        FFGPU_CUDA(cudaLaunchKernel(fn, grid, threads, args, 0, st));
-        return launch_check(A->ctx, "spmv");
-    }
-    return spmv_csr(A, x, y, trans, st);
+    const bool have = (trans ? A->sval_t : A->sval) || (A->sell_due >> (trans != 0) & 1);
+    return have && is_sell(A->csr_lanes) ? spmv_sell_copy(A, x, y, trans, st) : spmv_csr(A, x, y, trans, st);
 }
 
 int matrix_prepare_split(ffgpu_matrix *A, int trans) {
@@ -1527,11 +1530,13 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
     const bool band = may_loop && band_cg_fits(A);
     const bool sell = is_sell(A->csr_lanes);
     // The initial residual is summed in one order, whatever ran before: from block CSR where cg_band
-    // runs, which reads no SELL copy (a new matrix's copy is 90 us, of 640 for a small script), else from the
-    // layout's copy.  The other users of spmv() find the copy after any CG solve: cg_band leaves it due.
+    // runs, which reads no SELL copy (a new matrix's copy is 90 us, of 640 for a small script), from the copy
+    // where cg_loop runs (block CSR would leave the L2 full of it: P2 on 29^3 cells 45.7 us per iteration,
+    // 44.0), else in the layout's order.  The other users of spmv() find the copy of a SELL layout after any
+    // CG solve: cg_band leaves it due.
     if (band) A->sell_due |= 1 << (trans != 0);
     else if (may_loop && sell) FFGPU_TRY(sell_values(A, trans ? kSell64T : kSell64));
-    bool loop = band || (may_loop && sell && loop_cg_fits(A));
+    bool loop = band || (may_loop && loop_cg_fits(A, sell));
     A->cg_path = cluster ? kPathCluster
                  : band  ? (A->band_kind == kBandWide ? kPathWide : kPathBand)
                  : loop  ? kPathLoop
@@ -1546,7 +1551,7 @@ static int cg_one(ffgpu_matrix *A, const double *b, double *x, int trans, const 
         cg_x0_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, x, b, A->wcl, tgv);
         FFGPU_TRY(launch_check(ctx, "cg_x0"));
     }
-    FFGPU_TRY(band ? spmv_csr(A, x, g, trans, s) : spmv(A, x, g, trans, s));
+    FFGPU_TRY(band ? spmv_csr(A, x, g, trans, s) : loop ? spmv_sell_copy(A, x, g, trans, s) : spmv(A, x, g, trans, s));
     cg_init<<<kVecBlocks, kVecThreads, 0, s>>>(n, g, b, h, A->diag_inv, A->ks, prm->eps, itmax, ctx->d_part);
     FFGPU_TRY(launch_check(ctx, "cg_init"));
     if (mode == 1) {

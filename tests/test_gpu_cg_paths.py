@@ -73,3 +73,20 @@ def test_past_the_last_size_the_matrix_is_streamed():
     A.solve(b)
     # (block CSR, should the layout tuner take it, runs with launches)
     assert A.layout_code(6) == (LOOP if A.layout_code() >= 64 else THREE)
+
+
+@pytest.mark.parametrize("n,full", [(28, False), (32, True)])
+def test_p2_is_streamed_where_the_passes_are_full(n, full, monkeypatch):
+    """P2 past the SMs' shared memory: 5 788 chunks of 32 rows over 4 864 warps (0.60 of two passes), 8 583 (0.88)."""
+    import torch
+    S = ffgpu.device_space("P2", 3, n, n, n)
+    b = torch.zeros(S.Vh.ndof, dtype=torch.float64, device="cuda")
+    A = ffgpu.matrix(ffgpu.varf_diffusion(f=1.0, on=(1, 2), c_mass=0.5), S, rhs_out=b, eps=1e-9)
+    u = A.solve(b)
+    it = A.stats.iterations
+    assert A.layout_code(6) == (LOOP if full or A.layout_code() >= 64 else THREE)
+    assert torch.equal(A.solve(b), u)
+    monkeypatch.setenv("FFGPU_CLUSTER_CG", "0")
+    v = A.solve(b)
+    assert A.layout_code(6) == THREE and abs(A.stats.iterations - it) <= 2
+    assert float((u - v).norm() / v.norm()) <= 1e-8
